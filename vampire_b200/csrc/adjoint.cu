@@ -229,7 +229,7 @@ __global__ void adj_reciprocal_kernel(const LLGArgs<R> a, int* bad) {
 
 template <typename R, int FMT>
 __global__ void __launch_bounds__(256) adj_k1(const LLGArgs<R> a, AdjBufs<R> b) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl
+   pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= b.n) return;
    const int st = b.stride;
@@ -281,7 +281,7 @@ __device__ __forceinline__ double ku_grad(const MatParams<R>& m, const R hb[3], 
 
 template <typename R, int FMT>
 __global__ void __launch_bounds__(256) adj_k2(const LLGArgs<R> a, AdjBufs<R> b) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl
+   pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    const int st = b.stride;
    double gv[5] = {0, 0, 0, 0, 0};
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) adj_k2(const LLGArgs<R> a, AdjBufs<R> b) 
 
 template <typename R, int FMT>
 __global__ void __launch_bounds__(256) adj_k3(const LLGArgs<R> a, AdjBufs<R> b) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl
+   pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    const int st = b.stride;
    double gv[5] = {0, 0, 0, 0, 0};
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(256) adj_k3(const LLGArgs<R> a, AdjBufs<R> b) 
 
 template <typename R, int FMT>
 __global__ void __launch_bounds__(256) adj_k4(const LLGArgs<R> a, AdjBufs<R> b, int64_t t) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl
+   pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= b.n) return;
    const int st = b.stride;
@@ -405,7 +405,7 @@ __global__ void adj_lambda_init(const LLGArgs<R> a, AdjBufs<R> b, int64_t N) {
 template <typename R>
 __global__ void mz_kernel(int n, const R* __restrict__ sz, const int* __restrict__ mat,
                           const MatParams<R>* __restrict__ mp, double* out) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl
+   pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    double v = 0.0;
    if (i < n) v = (double)sz[i] * (double)mp[mat ? mat[i] : 0].mu_s_muB;

@@ -143,7 +143,7 @@ template <typename R, int FMT, int MODE, int VAR>
 __global__ void __launch_bounds__(256) llg_pass_kernel(const LLGArgs<R> a) {
    // launched with programmatic stream serialisation (launch_pdl): the
    // previous kernel of the stream has completed and its writes are visible
-   asm volatile("griddepcontrol.wait;" ::: "memory");
+   pdl_begin();
    const int i = (MODE == PASS_FIELD ? 0 : 32 * a.slice_first) + blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= (MODE == PASS_FIELD ? a.n : a.n_upd)) return;
    if (MODE == PASS_PREDICTOR) {

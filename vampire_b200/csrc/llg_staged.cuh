@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * SL, 24 / SL) llg_staged_kernel(const LLGA
    __shared__ __align__(8) uint64_t mbar[2];
    // launched with programmatic stream serialisation: the previous kernel of
    // the stream has completed and its writes are visible after this
-   asm volatile("griddepcontrol.wait;" ::: "memory");
+   pdl_begin();
    const int tid = threadIdx.x;
    const int stride = buf_bytes + kStageOwnArrays * TS * 4;
    float4* sdict = reinterpret_cast<float4*>(stage_smem + NBUF * stride);
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(128, 6) llg_warp_kernel(const LLGArgs<float> a
                                                           int buf_bytes, int dict_bytes, int mp_bytes) {
    extern __shared__ __align__(128) unsigned char stage_smem[];
    __shared__ __align__(8) uint64_t wbar[2 * 4];
-   asm volatile("griddepcontrol.wait;" ::: "memory");
+   pdl_begin();
    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
    const int wpb = blockDim.x >> 5;
    float4* sdict = reinterpret_cast<float4*>(stage_smem);

@@ -33,6 +33,17 @@
 
 namespace vgpu {
 
+// thread-block clusters: this block's rank, and the barrier of all threads of
+// the cluster (release / acquire)
+__device__ __forceinline__ unsigned cluster_rank() {
+   unsigned r;
+   asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+   return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 struct MCState {
    int ncolours = 0;
    std::vector<int> colour_host;      // [n]
@@ -109,7 +120,7 @@ __device__ __forceinline__ R site_energy_delta(const LLGArgs<R>& a, int i, int m
 #endif
 template <typename R, int FMT>
 __global__ void __launch_bounds__(256, VGPU_MC_MIN_BLOCKS) mc_colour_kernel(const MCArgs<R> p) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched by launch_pdl: the previous colour is done
+   pdl_begin();  // launched by launch_pdl: the previous colour is done
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    bool rejected = false;
    if (t < p.count) {
@@ -503,13 +514,14 @@ extern "C" int vgpu_mc_counters(vgpu_handle h, double* moves, double* rejects) {
 // no atom of any pair interacts with an atom of another pair, and
 //
 //   propose  (one thread per pair)  the move, the compensating spin, both
-//            energy changes, exp(-dE) and the Jacobian factor, and the moment
-//            terms mu s of both spins before and after;
-//   accept   (one warp)  the pairs in order with the running total moment,
-//            exactly the reference's rule: a pair's energy change does not
-//            depend on the other pairs of the phase, so the sequence of
-//            decisions is that of the sequential chain for this order of
-//            pairs; lanes then write the accepted spins.
+//            energy changes, exp(-dE) times the Jacobian factor, the
+//            acceptance uniform, and the pair's change of the moment;
+//   accept   (one cluster)  the decisions of the pairs taken in order with the
+//            running total moment, exactly the reference's rule: a pair's
+//            energy change does not depend on the other pairs of the phase,
+//            so the decisions are those of the sequential chain for this
+//            order of pairs, found in parallel (cmc_accept_kernel); the
+//            accepted spins are then written.
 //
 // Every pair move keeps the target distribution (the reference's
 // Metropolis-Hastings step with its constraint Jacobian), so the phases
@@ -524,10 +536,10 @@ struct CMCState {
    int maxK = 0;
    int* pairs = nullptr;      // [2 maxK]
    void* prop = nullptr;      // [6 maxK] proposed spins s1', s2' (x|y|z of each, R)
-   double* ef = nullptr;      // [maxK] exp(-dE) (negative: sphere rejection)
-   double* jac = nullptr;     // [maxK] |s2z / s2z'| in the constraint frame
-   double* mom = nullptr;     // [12 maxK] mu1 s1', mu2 s2', mu1 s1, mu2 s2 (x|y|z blocks of maxK each)
-   double* u = nullptr;       // [maxK] acceptance uniforms (replay) or nullptr
+   double* fac = nullptr;     // [maxK] exp(-dE) |s2z / s2z'| (constraint frame; negative: sphere rejection)
+   double* u = nullptr;       // [maxK] acceptance uniforms
+   double* dz = nullptr;      // [maxK] change of the moment along the constraint
+   double* dm = nullptr;      // [3 maxK] change of the moment (x|y|z blocks of maxK each)
    double* rnd = nullptr;     // [4 maxK] replayed Gaussians and uniforms
    double* M = nullptr;       // [3] running total moment (mu_B)
    unsigned long long* cnt = nullptr;  // [4] accepted, energy rejections, sphere rejections,
@@ -551,7 +563,7 @@ static CMCState* cmc_of(vgpu_ctx* h) { return (CMCState*)h->extras[5]; }
 void cmc_destroy(vgpu_ctx* h) {
    CMCState* c = cmc_of(h);
    if (!c) return;
-   cudaFree(c->pairs); cudaFree(c->prop); cudaFree(c->ef); cudaFree(c->jac); cudaFree(c->mom);
+   cudaFree(c->pairs); cudaFree(c->prop); cudaFree(c->fac); cudaFree(c->u); cudaFree(c->dz); cudaFree(c->dm);
    cudaFree(c->rnd); cudaFree(c->M); cudaFree(c->cnt); cudaFree(c->Mm); cudaFree(c->lists); cudaFree(c->list_entries);
    delete c;
    h->extras[5] = nullptr;
@@ -569,7 +581,7 @@ struct CMCArgs {
    const double* rnd;   // replayed numbers [4K] or nullptr
    uint64_t sweep; uint32_t phase;
    double P[9];
-   int* pairs; R* prop; double* ef; double* jac; double* mom; int maxK;
+   int* pairs; R* prop; double* fac; double* u; double* dz; double* dm; int maxK;
 };
 
 template <typename R, int FMT>
@@ -588,6 +600,7 @@ __device__ __forceinline__ R cmc_delta(const LLGArgs<R>& a, int i, int mi, const
 
 template <typename R, int FMT>
 __global__ void __launch_bounds__(128) cmc_propose_kernel(const CMCArgs<R> p) {
+   pdl_begin();
    const int k = blockIdx.x * blockDim.x + threadIdx.x;
    if (k >= p.K) return;
    const LLGArgs<R>& a = p.a;
@@ -636,7 +649,7 @@ __global__ void __launch_bounds__(128) cmc_propose_kernel(const CMCArgs<R> p) {
    s2fm[1] = mr * (s1im[1] - s1fm[1]) + s2im[1];
    const int st = p.maxK;
    if (!((s2fm[0] * s2fm[0] + s2fm[1] * s2fm[1]) < 1.0) || i1 == i2) {
-      p.ef[k] = -1.0;  // off the unit sphere: rejected
+      p.fac[k] = -1.0;  // off the unit sphere: rejected
       return;
    }
    s2fm[2] = (s2im[2] >= 0.0 ? 1.0 : -1.0) * sqrt(1.0 - s2fm[0] * s2fm[0] - s2fm[1] * s2fm[1]);
@@ -647,85 +660,166 @@ __global__ void __launch_bounds__(128) cmc_propose_kernel(const CMCArgs<R> p) {
    const R de1 = cmc_delta<R, FMT>(a, i1, m1, mp1, S1, T1, (R)mu1);
    const R de2 = cmc_delta<R, FMT>(a, i2, m2, mp2, S2, T2, (R)mu2);
    const double de21 = (double)de1 * (double)__ldg(p.beta + m1) + (double)de2 * (double)__ldg(p.beta + m2);
-   p.ef[k] = exp(-de21);
-   p.jac[k] = fabs(s2im[2] / s2fm[2]);
+   p.fac[k] = exp(-de21) * fabs(s2im[2] / s2fm[2]);
+   if (p.rnd) {
+      p.u[k] = p.rnd[3 * (size_t)p.K + k];
+   } else {
+      const u32x4 c = {(uint32_t)k, (uint32_t)p.sweep, (uint32_t)(p.sweep >> 32) ^ (p.phase << 20), RNG_CMC_ACCEPT};
+      p.u[k] = u01d(philox4x32_10(c, a.seed_lo, a.seed_hi).x);
+   }
+   double dm[3];
    for (int q = 0; q < 3; ++q) {
       p.prop[q * st + k] = T1[q];
       p.prop[(3 + q) * st + k] = T2[q];
-      p.mom[q * st + k] = mu1 * (double)T1[q];
-      p.mom[(3 + q) * st + k] = mu2 * (double)T2[q];
-      p.mom[(6 + q) * st + k] = mu1 * (double)S1[q];
-      p.mom[(9 + q) * st + k] = mu2 * (double)S2[q];
+      dm[q] = mu1 * (double)T1[q] + mu2 * (double)T2[q] - mu1 * (double)S1[q] - mu2 * (double)S2[q];
+      p.dm[q * st + k] = dm[q];
    }
+   p.dz[k] = P[6] * dm[0] + P[7] * dm[1] + P[8] * dm[2];
 }
 
-// One warp: the pairs in order with the running total moment M (the
-// reference's acceptance, cmc.cpp:459-490); each lane holds a chunk's pair,
-// every lane follows the same decisions, lane l writes pair l's spins.
+// Acceptance of a phase (cmc.cpp:459-490): pair k is accepted when
+// f_k (z'/z)^2 >= u_k and z' > 0, z the running moment along the constraint
+// after the pairs before it and z' = z + dz_k.  The decisions form a serial
+// chain only through z, and z changes little over a few thousand pairs, so the
+// chain is solved by iteration: every thread takes kCmcItems consecutive pairs
+// of a chunk, a block-wide prefix sum of the accepted dz gives each thread its
+// z, the thread decides its pairs in order, and this repeats until no decision
+// changed.  After round r the first r threads hold the chain's decisions
+// whatever they held before, so the loop ends after at most kCmcThreads + 1
+// rounds with the one solution there is, the sequential one; two to four
+// rounds are usual.  (A one-warp walk of the chain, 32 pairs' data passed
+// through shuffles, was bound by its latency: 742 us for 3,456 pairs.  A step
+// of 13,824 spins at 400 K, four phases each, took 2.68 ms with it and takes
+// 0.10 ms now.)
+//
+// The phase runs on one cluster of kCmcCluster blocks.  Each block solves the
+// whole chain (the same instructions on the same numbers, so the same
+// decisions) and the blocks share the scattered spin writes, which one SM
+// alone would take longer over than the decisions.  The moment is written
+// after the cluster barrier, when every block has read it.
+constexpr int kCmcThreads = 1024;
+constexpr int kCmcItems = 4;
+constexpr int kCmcCluster = 8;
+
+// exclusive prefix sum of v over the block's threads (a function of the lower
+// threads' values alone) and its total; sh: 32 doubles
+__device__ __forceinline__ double block_exclusive(double v, double* sh, double& total) {
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   double x = v;
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+   }
+   if (lane == 31) sh[warp] = x;
+   __syncthreads();
+   double w = sh[lane];
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+   }
+   total = __shfl_sync(0xffffffffu, w, 31);
+   const double before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+   const double below = __shfl_up_sync(0xffffffffu, x, 1);  // lower lanes only: v itself plays no part
+   return (warp ? before : 0.0) + (lane ? below : 0.0);
+}
+
 template <typename R>
-__global__ void __launch_bounds__(32) cmc_accept_kernel(LLGArgs<R> a, int K, int st, const int* __restrict__ pairs,
-                                                        const R* __restrict__ prop, const double* __restrict__ ef,
-                                                        const double* __restrict__ jac,
-                                                        const double* __restrict__ mom, const double* __restrict__ urep,
-                                                        uint64_t sweep, uint32_t phase, const double* pvp, double* M,
-                                                        unsigned long long* cnt) {
-   const int lane = threadIdx.x;
-   const unsigned full = 0xffffffffu;
-   const double pv[3] = {pvp[0], pvp[1], pvp[2]};
-   double Mx = M[0], My = M[1], Mz = M[2];
-   unsigned long long nacc = 0, nrej = 0, nsph = 0;
-   for (int base = 0; base < K; base += 32) {
-      const int k = base + lane;
-      const bool on = k < K;
-      double e = -1.0, jk = 0.0, u = 0.0, mm[12];
-      for (int q = 0; q < 12; ++q) mm[q] = 0.0;
-      if (on) {
-         e = ef[k];
-         if (e >= 0.0) {
-            jk = jac[k];
-            for (int q = 0; q < 12; ++q) mm[q] = mom[q * st + k];
-         }
-         if (urep) {
-            u = urep[k];
-         } else {
-            const u32x4 c = {(uint32_t)k, (uint32_t)sweep, (uint32_t)(sweep >> 32) ^ (phase << 20), RNG_CMC_ACCEPT};
-            u = u01d(philox4x32_10(c, a.seed_lo, a.seed_hi).x);
-         }
+__global__ void __launch_bounds__(kCmcThreads) __cluster_dims__(kCmcCluster)
+    cmc_accept_kernel(LLGArgs<R> a, int K, int st, const int* __restrict__ pairs, const R* __restrict__ prop,
+                      const double* __restrict__ fac, const double* __restrict__ u, const double* __restrict__ dz,
+                      const double* __restrict__ dm, double* M, unsigned long long* cnt) {
+   static_assert(kCmcItems == 4 && kCmcThreads == 32 * 32, "two double2 loads per array, 32 warps");
+   pdl_begin();
+   __shared__ double sh[2][32];
+   __shared__ double red[3][32];
+   __shared__ unsigned long long scnt[3];
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   const int rank = (int)cluster_rank();
+   if (tid < 3) scnt[tid] = 0;
+   const double M0[3] = {M[0], M[1], M[2]};
+   double z0 = M0[0] * M[3] + M0[1] * M[4] + M0[2] * M[5];  // M[3..5]: the constraint direction
+   double sum[3] = {0.0, 0.0, 0.0};                          // this thread's accepted change of the moment
+   unsigned nacc = 0, nrej = 0, nsph = 0;
+   for (int base = 0; base < K; base += kCmcThreads * kCmcItems) {
+      const int k0 = base + kCmcItems * tid;
+      double f[kCmcItems] = {-1.0, -1.0, -1.0, -1.0}, uu[kCmcItems] = {0, 0, 0, 0}, d[kCmcItems] = {0, 0, 0, 0};
+      if (k0 < K) {  // the arrays are allocated to a multiple of kCmcItems
+         const double2 *pf = reinterpret_cast<const double2*>(fac + k0), *pu = reinterpret_cast<const double2*>(u + k0),
+                       *pd = reinterpret_cast<const double2*>(dz + k0);
+         const double2 f0 = pf[0], f1 = pf[1], u0 = pu[0], u1 = pu[1], d0 = pd[0], d1 = pd[1];
+         f[0] = f0.x; f[1] = f0.y; f[2] = f1.x; f[3] = f1.y;
+         uu[0] = u0.x; uu[1] = u0.y; uu[2] = u1.x; uu[3] = u1.y;
+         d[0] = d0.x; d[1] = d0.y; d[2] = d1.x; d[3] = d1.y;
       }
-      bool mine = false;
-      const int nl = min(32, K - base);
-      for (int l = 0; l < nl; ++l) {
-         const double el = __shfl_sync(full, e, l);
-         if (el < 0.0) {
-            ++nsph;
-            continue;
+      unsigned on = 0, acc = 0;  // bit q: pair k0 + q proposes a move / is accepted
+#pragma unroll
+      for (int q = 0; q < kCmcItems; ++q)
+         if (k0 + q < K && !(f[q] < 0.0)) on |= 1u << q;
+      double mine = 0.0, total = 0.0;
+      for (int round = 0; round <= kCmcThreads; ++round) {
+         double z = z0 + block_exclusive(mine, sh[round & 1], total);
+         unsigned now = 0;
+         mine = 0.0;
+#pragma unroll
+         for (int q = 0; q < kCmcItems; ++q) {
+            if ((on >> q) & 1u) {
+               const double zn = z + d[q], r = zn / z;
+               if (f[q] * (r * r) >= uu[q] && zn > 0.0) {
+                  now |= 1u << q;
+                  mine += d[q];
+                  z = zn;
+               }
+            }
          }
-         double ml[12];
-         for (int q = 0; q < 12; ++q) ml[q] = __shfl_sync(full, mm[q], l);
-         const double jl = __shfl_sync(full, jk, l), ul = __shfl_sync(full, u, l);
-         const double mzo = Mx * pv[0] + My * pv[1] + Mz * pv[2];
-         const double nx = Mx + ml[0] + ml[3] - ml[6] - ml[9];
-         const double ny = My + ml[1] + ml[4] - ml[7] - ml[10];
-         const double nz = Mz + ml[2] + ml[5] - ml[8] - ml[11];
-         const double mzn = nx * pv[0] + ny * pv[1] + nz * pv[2];
-         const double prob = el * ((mzn / mzo) * (mzn / mzo)) * jl;
-         if (prob >= ul && mzn > 0.0) {
-            Mx = nx; My = ny; Mz = nz;
-            ++nacc;
-            if (lane == l) mine = true;
-         } else {
-            ++nrej;
-         }
+         const bool changed = now != acc;
+         acc = now;
+         if (!__syncthreads_or(changed)) break;  // total is the sum of these decisions
       }
-      if (mine) {
-         const int i1 = pairs[2 * k], i2 = pairs[2 * k + 1];
-         a.ax[i1] = prop[k]; a.ay[i1] = prop[st + k]; a.az[i1] = prop[2 * st + k];
-         a.ax[i2] = prop[3 * st + k]; a.ay[i2] = prop[4 * st + k]; a.az[i2] = prop[5 * st + k];
+      z0 += total;
+      if (rank == 0) {
+#pragma unroll
+         for (int q = 0; q < kCmcItems; ++q)
+            if ((acc >> q) & 1u)
+               for (int c = 0; c < 3; ++c) sum[c] += dm[(size_t)c * st + k0 + q];
+         nacc += __popc(acc);
+         nrej += __popc(on & ~acc);
+         nsph += (k0 < K ? min(kCmcItems, K - k0) : 0) - __popc(on);
+      }
+      if ((warp & (kCmcCluster - 1)) == rank) {
+#pragma unroll
+         for (int q = 0; q < kCmcItems; ++q) {
+            if ((acc >> q) & 1u) {
+               const int k = k0 + q, i1 = pairs[2 * k], i2 = pairs[2 * k + 1];
+               a.ax[i1] = prop[k]; a.ay[i1] = prop[st + k]; a.az[i1] = prop[2 * st + k];
+               a.ax[i2] = prop[3 * st + k]; a.ay[i2] = prop[4 * st + k]; a.az[i2] = prop[5 * st + k];
+            }
+         }
       }
    }
-   if (lane == 0) {
-      M[0] = Mx; M[1] = My; M[2] = Mz;
-      cnt[0] += nacc; cnt[1] += nrej; cnt[2] += nsph;
+   if (rank == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+         for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+         if (lane == 0) red[c][warp] = sum[c];
+      }
+      nacc = __reduce_add_sync(0xffffffffu, nacc);
+      nrej = __reduce_add_sync(0xffffffffu, nrej);
+      nsph = __reduce_add_sync(0xffffffffu, nsph);
+      if (lane == 0) {
+         atomicAdd(&scnt[0], (unsigned long long)nacc);
+         atomicAdd(&scnt[1], (unsigned long long)nrej);
+         atomicAdd(&scnt[2], (unsigned long long)nsph);
+      }
+      __syncthreads();
+   }
+   cluster_barrier();  // every block has read M
+   if (rank == 0 && tid < 3) {
+      double s = 0.0;
+      for (int w = 0; w < 32; ++w) s += red[tid][w];
+      M[tid] = M0[tid] + s;
+      cnt[tid] += scnt[tid];
    }
 }
 
@@ -749,8 +843,7 @@ __global__ void cmc_moment_kernel(const LLGArgs<R> a, const R* __restrict__ mu_r
 template <typename R, int FMT>
 static cudaError_t launch_cmc_propose(const CMCArgs<R>& p, cudaStream_t st) {
    if (p.K <= 0) return cudaSuccess;
-   cmc_propose_kernel<R, FMT><<<(p.K + 127) / 128, 128, 0, st>>>(p);
-   return cudaGetLastError();
+   return launch_pdl(cmc_propose_kernel<R, FMT>, dim3((p.K + 127) / 128), dim3(128), 0, st, p);
 }
 
 template <typename R>
@@ -797,7 +890,7 @@ int cmc_phase(vgpu_handle h, const R* tab, const int* list, int count, const int
    p.sigma = tab; p.beta = tab + h->sys.M; p.mu_ratio = tab + 2 * h->sys.M;
    p.sweep = c->sweep; p.phase = phase;
    for (int q = 0; q < 9; ++q) p.P[q] = P[q];
-   p.pairs = c->pairs; p.prop = (R*)c->prop; p.ef = c->ef; p.jac = c->jac; p.mom = c->mom; p.maxK = c->maxK;
+   p.pairs = c->pairs; p.prop = (R*)c->prop; p.fac = c->fac; p.u = c->u; p.dz = c->dz; p.dm = c->dm; p.maxK = c->maxK;
    p.K = K;
    p.given = given;
    p.rnd = rnd;
@@ -814,10 +907,9 @@ int cmc_phase(vgpu_handle h, const R* tab, const int* list, int count, const int
    h->prof_begin(PROF_MC);
    cudaError_t e = cmc_propose_dispatch<R>(p, h->sys.fmt, h->stream);
    if (e == cudaSuccess && K > 0) {
-      cmc_accept_kernel<R><<<1, 32, 0, h->stream>>>(p.a, K, c->maxK, c->pairs, (const R*)c->prop, c->ef, c->jac,
-                                                    c->mom, rnd ? rnd + 3 * (size_t)K : nullptr, c->sweep, phase,
-                                                    Mdev + 3, Mdev, c->cnt);
-      e = cudaGetLastError();
+      e = launch_pdl(cmc_accept_kernel<R>, dim3(kCmcCluster), dim3(kCmcThreads), 0, h->stream, p.a, K, c->maxK,
+                     (const int*)c->pairs, (const R*)c->prop, (const double*)c->fac, (const double*)c->u,
+                     (const double*)c->dz, (const double*)c->dm, Mdev, c->cnt);
    }
    h->prof_end(PROF_MC);
    if (e != cudaSuccess) return cuda_err(h, e, "cmc launch");
@@ -949,12 +1041,14 @@ CMCState* cmc_new(vgpu_handle h) {
    int maxK = 1;
    for (int col = 0; col < s->ncolours; ++col) maxK = std::max(maxK, (s->colour_off[col + 1] - s->colour_off[col]) / 2);
    maxK = std::max(maxK, h->sys.n / 2);
+   maxK = (maxK + kCmcItems - 1) / kCmcItems * kCmcItems;  // whole vector loads in cmc_accept_kernel
    c->maxK = maxK;
    const size_t rs = h->prec == VGPU_PREC_FP64 ? sizeof(double) : sizeof(float);
    cudaError_t e;
    if ((e = cudaMalloc(&c->pairs, sizeof(int) * 2 * maxK)) || (e = cudaMalloc(&c->prop, rs * 6 * maxK)) ||
-       (e = cudaMalloc(&c->ef, sizeof(double) * maxK)) || (e = cudaMalloc(&c->jac, sizeof(double) * maxK)) ||
-       (e = cudaMalloc(&c->mom, sizeof(double) * 12 * maxK)) || (e = cudaMalloc(&c->rnd, sizeof(double) * 4 * maxK)) ||
+       (e = cudaMalloc(&c->fac, sizeof(double) * maxK)) || (e = cudaMalloc(&c->u, sizeof(double) * maxK)) ||
+       (e = cudaMalloc(&c->dz, sizeof(double) * maxK)) || (e = cudaMalloc(&c->dm, sizeof(double) * 3 * maxK)) ||
+       (e = cudaMalloc(&c->rnd, sizeof(double) * 4 * maxK)) ||
        (e = cudaMalloc(&c->M, sizeof(double) * 6)) || (e = cudaMalloc(&c->cnt, sizeof(unsigned long long) * 4))) {
       cmc_destroy(h);
       cuda_err(h, e, "cmc buffers");

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) stats_mag_small_kernel(const LLGArgs<R> a
    __shared__ double smu[kStatsMuShared];
    // launched with programmatic stream serialisation (launch_pdl): the
    // previous kernel of the stream (the corrector) has completed after this
-   asm volatile("griddepcontrol.wait;" ::: "memory");
+   pdl_begin();
    const bool mu_shared = a.M <= kStatsMuShared;
    for (int k = threadIdx.x; k < NB * ST_NQ; k += blockDim.x) acc[k] = 0.0;
    if (mu_shared)
@@ -398,7 +398,7 @@ static cudaError_t stats_dispatch(const LLGArgs<R>& a, int fmt, StatsMask& m, in
 
 // the rows of one mask into device-addressable host memory (vgpu_stats_copy_rows)
 __global__ void stats_rows_copy_kernel(const double* __restrict__ src, double* __restrict__ dst, int n) {
-   asm volatile("griddepcontrol.wait;" ::: "memory");
+   pdl_begin();
    for (int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = src[k];
 }
 

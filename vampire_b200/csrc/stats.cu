@@ -108,49 +108,43 @@ __device__ void stats_finalize_bin(const double* __restrict__ partial, int nbloc
       }
    }
    __syncthreads();
-   if (threadIdx.x != 0) return;
+   // one thread per output component (0-3 magnetisation, 4-8 energies), so
+   // the running sums' read-modify-writes are in flight together
+   const int k = threadIdx.x;
+   if (k >= ST_W) return;
    const double* v = vq;
    double* o = cur + (size_t)bin * ST_W;
    double* mn = mean + (size_t)bin * ST_W;
-   if (do_mag) {
+   double* dv = derived + (size_t)bin * ST_DV;
+   if (k < 4 && do_mag) {
       const double msat = v[ST_MU];
       const double magm = sqrt(v[ST_MX] * v[ST_MX] + v[ST_MY] * v[ST_MY] + v[ST_MZ] * v[ST_MZ]);
-      if (msat == 0.0) {
-         o[0] = o[1] = o[2] = o[3] = 0.0;
-      } else {
-         o[0] = v[ST_MX] / magm;
-         o[1] = v[ST_MY] / magm;
-         o[2] = v[ST_MZ] / magm;
-         o[3] = magm / msat;
-      }
-      for (int k = 0; k < 4; ++k) mn[k] += o[k];
-      double* dv = derived + (size_t)bin * ST_DV;
-      const double mm = o[3];
-      for (int k = 0; k < 3; ++k) {
-         dv[DV_SUS + k] += o[k] * mm;
-         dv[DV_SUS2 + k] += o[k] * o[k] * mm * mm;
-         dv[DV_ASUS + k] += fabs(o[k] * mm);
-         dv[DV_ASUS2 + k] += fabs(o[k] * o[k] * mm * mm);
-      }
-      dv[DV_SUS + 3] += mm;
-      dv[DV_SUS2 + 3] += mm * mm;
-      dv[DV_ASUS + 3] += mm;
-      dv[DV_ASUS2 + 3] += mm * mm;
-      for (int k = 0; k < 4; ++k) {  // Welford update, mag_count includes this update
-         const double r1 = o[k] - dv[DV_MEAN + k];
-         dv[DV_MEAN + k] += r1 / mag_count;
-         const double r2 = o[k] - dv[DV_MEAN + k];
-         dv[DV_RES + k] += r1 * r2;
-      }
+      const double mm = msat == 0.0 ? 0.0 : magm / msat;
+      const double m = msat == 0.0 ? 0.0 : k < 3 ? v[ST_MX + k] / magm : mm;
+      o[k] = m;
+      mn[k] += m;
+      // component products m_k |m|; |m| itself for k = 3
+      const double p1 = k < 3 ? m * mm : mm, p2 = k < 3 ? m * m * mm * mm : mm * mm;
+      dv[DV_SUS + k] += p1;
+      dv[DV_SUS2 + k] += p2;
+      dv[DV_ASUS + k] += k < 3 ? fabs(p1) : p1;
+      dv[DV_ASUS2 + k] += k < 3 ? fabs(p2) : p2;
+      // Welford update, mag_count includes this update
+      const double r1 = m - dv[DV_MEAN + k];
+      const double mean1 = dv[DV_MEAN + k] + r1 / mag_count;
+      dv[DV_MEAN + k] = mean1;
+      dv[DV_RES + k] += r1 * (m - mean1);
    }
-   if (do_energy) {
+   if (k >= 4 && do_energy) {
       const double ex = 0.5 * v[ST_EEX], an = v[ST_EAN], ap = v[ST_EAP], ms = 0.5 * v[ST_EMS];
-      o[4] = ex + an + ap + ms;
-      o[5] = ex; o[6] = an; o[7] = ap; o[8] = ms;
-      for (int k = 4; k < 9; ++k) mn[k] += o[k];
-      double* dv = derived + (size_t)bin * ST_DV;
-      dv[DV_E] += o[4];
-      dv[DV_E2] += o[4] * o[4];
+      const double tot = ex + an + ap + ms;
+      const double e = k == 4 ? tot : k == 5 ? ex : k == 6 ? an : k == 7 ? ap : ms;
+      o[k] = e;
+      mn[k] += e;
+      if (k == 4) {
+         dv[DV_E] += tot;
+         dv[DV_E2] += tot * tot;
+      }
    }
 }
 
@@ -162,6 +156,7 @@ __device__ void stats_finalize_bin(const double* __restrict__ partial, int nbloc
 // x, y, z, material and mask ids), the moments per material come from shared
 // memory (no dependent global load per atom).  Writes the same block partial
 // rows as stats_partial_kernel (energy quantities zero).
+constexpr int kStatsAtoms = 2;      // atoms per thread the energy and many-bin passes aim at
 constexpr int kStatsMuShared = 64;  // materials whose moments the kernel keeps in shared memory
 
 // The last block to finish (atomic ticket after a fence) merges every block's
@@ -253,15 +248,71 @@ __global__ void __launch_bounds__(256) stats_mag_small_kernel(const LLGArgs<R> a
    if (threadIdx.x == 0) *so.ticket = 0;
 }
 
-template <typename R, int FMT>
-__global__ void stats_partial_kernel(const LLGArgs<R> a, const int* __restrict__ mask, int size, int do_energy,
-                                     const R* __restrict__ hm, double* __restrict__ partial) {
-   extern __shared__ double acc[];
-   const int nq = ST_NQ;
-   const int nq_used = do_energy ? ST_NQ : ST_MU + 1;
+// Sums of ST_NQ values (NQ = 8) or of the first four (NQ = 4) over a warp by
+// halving: at each step a lane keeps half of its values and hands the other
+// half over, so NQ values take NQ + 1 (NQ = 4: 6) shuffles of a double instead
+// of 5 NQ.  The total of value q ends in lane first_lane<NQ>(q).
+template <int NQ>
+__device__ __forceinline__ double warp_sum_all(const double v[NQ]) {
    const int lane = threadIdx.x & 31;
-   for (int k = threadIdx.x; k < size * nq; k += blockDim.x) acc[k] = 0.0;
+   double w[NQ];
+#pragma unroll
+   for (int k = 0; k < NQ; ++k) w[k] = v[k];
+   int o = 16;
+#pragma unroll
+   for (int h = NQ / 2; h >= 1; h >>= 1, o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < h; ++k) {
+         const double keep = up ? w[k + h] : w[k], give = up ? w[k] : w[k + h];
+         w[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+   }
+#pragma unroll
+   for (; o >= 1; o >>= 1) w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+   return w[0];
+}
+
+// the quantity whose warp total warp_sum_all<NQ> leaves in this lane, or -1
+template <int NQ>
+__device__ __forceinline__ int warp_sum_owner() {
+   const int lane = threadIdx.x & 31;
+   if (NQ == 8) return (lane & 3) ? -1 : ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+   return (lane & 7) ? -1 : ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+}
+
+// Block partial rows of one mask.  EN: with the energies (NQ = 8 quantities,
+// else the four of the magnetisation).  Bound by the exchange gather with
+// energies and by the state's bytes without, as long as the sums stay in
+// registers, so they do:
+//
+//   NB = 2  (masks of at most two bins, such as the materials of an alloy) per
+//           thread and bin, reduced once at the end;
+//   NB = 0  per thread for the bin its warp is in -- replicas and regions are
+//           runs of atoms, so a warp rarely changes bin -- and added to the
+//           block's shared sums when the bin changes; a warp whose lanes hold
+//           several bins reduces per bin, one round each.
+template <typename R, int FMT, int NB, bool EN>
+__global__ void __launch_bounds__(256) stats_partial_kernel(const LLGArgs<R> a, const int* __restrict__ mask, int size,
+                                                            const R* __restrict__ hm, double* __restrict__ partial) {
+   extern __shared__ double acc[];
+   constexpr int NQ = EN ? ST_NQ : 4;
+   static_assert(ST_NQ == 8 && ST_MU == 3, "quantity order");
+   const int lane = threadIdx.x & 31;
+   for (int k = threadIdx.x; k < size * ST_NQ; k += blockDim.x) acc[k] = 0.0;
+   pdl_begin();
    __syncthreads();
+   double s[NB ? NB : 1][NQ];
+#pragma unroll
+   for (int b = 0; b < (NB ? NB : 1); ++b)
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) s[b][k] = 0.0;
+   const int owned_q = warp_sum_owner<NQ>();
+   auto add_shared = [&](int bin, const double v[NQ]) {
+      const double w = warp_sum_all<NQ>(v);
+      if (owned_q >= 0) atomicAdd(acc + (size_t)bin * ST_NQ + owned_q, w);
+   };
+   int cur = -1;  // NB = 0: the bin of the sums in s[0]
    const int per = (a.n_upd + gridDim.x - 1) / gridDim.x;  // owned atoms only
    const int begin = blockIdx.x * per;
    const int end = min(a.n_upd, begin + per);
@@ -269,13 +320,13 @@ __global__ void stats_partial_kernel(const LLGArgs<R> a, const int* __restrict__
    for (int base = begin; base < end; base += blockDim.x) {
       const int i = base + threadIdx.x;
       const bool on = i < end;
-      double q[ST_NQ];
+      double q[NQ];
 #pragma unroll
-      for (int k = 0; k < ST_NQ; ++k) q[k] = 0.0;
+      for (int k = 0; k < NQ; ++k) q[k] = 0.0;
       int bin = -1;
       if (on) {
          const int mi = a.mat ? __ldg(a.mat + i) : 0;
-         const MatParams<R> m = a.mp[mi];
+         const MatParams<R>& m = a.mp[mi];
          const double mu = (double)m.mu_s_muB;
          const R S[3] = {a.ax[i], a.ay[i], a.az[i]};
          bin = __ldg(mask + i);
@@ -283,9 +334,9 @@ __global__ void stats_partial_kernel(const LLGArgs<R> a, const int* __restrict__
          q[ST_MY] = (double)S[1] * mu;
          q[ST_MZ] = (double)S[2] * mu;
          q[ST_MU] = mu;
-         if (do_energy) {
+         if constexpr (EN) {
             R hx = 0, hy = 0, hz = 0;
-            exchange_gather<R, FMT>(a, i, mi, a.ax, a.ay, a.az, hx, hy, hz);
+            exchange_field<R, FMT, 0>(a, i, mi, a.ax, a.ay, a.az, hx, hy, hz);
             double eex = -((double)S[0] * hx + (double)S[1] * hy + (double)S[2] * hz);
             if (a.bq_off) {
                const double Sb[3] = {(double)S[0], (double)S[1], (double)S[2]};
@@ -308,36 +359,56 @@ __global__ void stats_partial_kernel(const LLGArgs<R> a, const int* __restrict__
             q[ST_EMS] = ems * mu;
          }
       }
-      // warp aggregation: one shuffle reduction per distinct bin in the warp
-      // (masks are mostly uniform over 32 consecutive atoms), so the shared
-      // accumulators see one atomic per bin and quantity instead of 32; a warp
-      // holding more than 4 bins adds the rest lane by lane
-      unsigned left = __ballot_sync(0xffffffffu, on);
-      for (int round = 0; left; ++round) {
-         if (round == 4) {
-            if (on && ((left >> lane) & 1u)) {
+      if constexpr (NB > 0) {
 #pragma unroll
-               for (int k = 0; k < ST_NQ; ++k)
-                  if (k < nq_used) atomicAdd(acc + (size_t)bin * nq + k, q[k]);
+         for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) s[b][k] += bin == b ? q[k] : 0.0;
+      } else {
+         unsigned left = __ballot_sync(0xffffffffu, on);
+         if (!left) continue;
+         const int b0 = __shfl_sync(0xffffffffu, bin, __ffs(left) - 1);
+         if (__all_sync(0xffffffffu, !on || bin == b0)) {
+            if (b0 != cur) {
+               if (cur >= 0) add_shared(cur, s[0]);
+               cur = b0;
+#pragma unroll
+               for (int k = 0; k < NQ; ++k) s[0][k] = q[k];
+            } else {
+#pragma unroll
+               for (int k = 0; k < NQ; ++k) s[0][k] += q[k];
             }
-            break;
-         }
-         const int src = __ffs(left) - 1;
-         const int b = __shfl_sync(0xffffffffu, bin, src);
-         const bool mine = on && bin == b;
-         left &= ~__ballot_sync(0xffffffffu, mine);
+         } else {
+            // past four bins in one warp the remaining lanes add one by one
+            for (int round = 0; left; ++round) {
+               if (round == 4) {
+                  if (on && ((left >> lane) & 1u)) {
 #pragma unroll
-         for (int k = 0; k < ST_NQ; ++k) {
-            if (k < nq_used) {
-               const double v = warp_sum(mine ? q[k] : 0.0);
-               if (lane == src) atomicAdd(acc + (size_t)b * nq + k, v);
+                     for (int k = 0; k < NQ; ++k) atomicAdd(acc + (size_t)bin * ST_NQ + k, q[k]);
+                  }
+                  break;
+               }
+               const int b = __shfl_sync(0xffffffffu, bin, __ffs(left) - 1);
+               const bool mine = on && bin == b;
+               left &= ~__ballot_sync(0xffffffffu, mine);
+               double v[NQ];
+#pragma unroll
+               for (int k = 0; k < NQ; ++k) v[k] = mine ? q[k] : 0.0;
+               add_shared(b, v);
             }
          }
       }
    }
+   if constexpr (NB > 0) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+         if (b < size) add_shared(b, s[b]);
+   } else {
+      if (cur >= 0) add_shared(cur, s[0]);
+   }
    __syncthreads();
-   double* out = partial + (size_t)blockIdx.x * size * nq;
-   for (int k = threadIdx.x; k < size * nq; k += blockDim.x) out[k] = acc[k];
+   double* out = partial + (size_t)blockIdx.x * size * ST_NQ;
+   for (int k = threadIdx.x; k < size * ST_NQ; k += blockDim.x) out[k] = acc[k];
 }
 
 // Compensated sum of block partials, then reference normalisation.  One
@@ -351,18 +422,25 @@ __global__ void __launch_bounds__(32 * ST_NQ) stats_final_kernel(const double* _
                                                                   double* __restrict__ raw,
                                                                   double* __restrict__ derived, double mag_count) {
    __shared__ double vq[ST_NQ];
+   pdl_begin();
    stats_finalize_bin(partial, nblocks, size, blockIdx.x, do_mag, do_energy, cur, mean, raw, derived, mag_count, vq);
+}
+
+template <typename R, int FMT, int NB, bool EN>
+static cudaError_t launch_partial(const LLGArgs<R>& a, StatsMask& m, int nblocks, const R* hm, cudaStream_t st) {
+   const size_t smem = (size_t)m.size * ST_NQ * sizeof(double);
+   if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(stats_partial_kernel<R, FMT, NB, EN>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   return launch_pdl(stats_partial_kernel<R, FMT, NB, EN>, dim3(nblocks), dim3(256), (int)smem, st, a,
+                     (const int*)m.mask, m.size, hm, m.partial);
 }
 
 template <typename R, int FMT>
 static cudaError_t launch_stats(const LLGArgs<R>& a, StatsMask& m, int nblocks, int do_mag, int do_energy,
                                 const R* hm, cudaStream_t st) {
-   const size_t smem = (size_t)m.size * ST_NQ * sizeof(double);
-   if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(stats_partial_kernel<R, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
-      if (e != cudaSuccess) return e;
-   }
    if (do_mag && !do_energy && m.size <= 4) {
       nblocks = std::max(1, nblocks / 2);  // 4 blocks per SM: measured best for this streaming kernel
       // the per-step magnetisation of small masks: one launch, merged and
@@ -375,12 +453,16 @@ static cudaError_t launch_stats(const LLGArgs<R>& a, StatsMask& m, int nblocks, 
       if (m.size == 2) return launch_pdl(stats_mag_small_kernel<R, 2>, g, b, 0, st, a, mk, m.size, pt, so);
       return launch_pdl(stats_mag_small_kernel<R, 4>, g, b, 0, st, a, mk, m.size, pt, so);
    }
-   stats_partial_kernel<R, FMT><<<nblocks, 256, smem, st>>>(a, m.mask, m.size, do_energy, hm, m.partial);
-   cudaError_t e = cudaGetLastError();
+   // blocks of the partial pass: a few atoms per thread, so that the sums at
+   // the end of a block are a small part of it
+   const int nb = std::max(1, std::min(nblocks, (a.n_upd + 256 * kStatsAtoms - 1) / (256 * kStatsAtoms)));
+   cudaError_t e;
+   if (!do_energy) e = launch_partial<R, FMT_ISO_TAB, 0, false>(a, m, nb, hm, st);  // no exchange: one format for all
+   else if (m.size == 2) e = launch_partial<R, FMT, 2, true>(a, m, nb, hm, st);
+   else e = launch_partial<R, FMT, 0, true>(a, m, nb, hm, st);
    if (e != cudaSuccess) return e;
-   stats_final_kernel<<<m.size, 32 * ST_NQ, 0, st>>>(m.partial, nblocks, m.size, do_mag, do_energy, m.cur, m.mean,
-                                                     m.raw, m.derived, (double)(m.counter_mag + 1));
-   return cudaGetLastError();
+   return launch_pdl(stats_final_kernel, dim3(m.size), dim3(32 * ST_NQ), 0, st, (const double*)m.partial, nb, m.size,
+                     do_mag, do_energy, m.cur, m.mean, m.raw, m.derived, (double)(m.counter_mag + 1));
 }
 
 template <typename R>

@@ -8,8 +8,8 @@
 // six dense Nc x Nc FP64 matrices (src/dipole/memory.cpp:29-56), 750 GB at
 // 125,000 cells; its GPU version is disabled.  Here nothing dense is stored:
 //
-//   K5  one warp per cell sums mu_s s over the cell's atoms (cell-sorted atom
-//       list, FP64), giving the cell moments in J/T and in mu_B for K6;
+//   K5  a group of lanes per cell sums mu_s s over the cell's atoms (cell-sorted
+//       atom list, FP64), giving the cell moments in J/T and in mu_B for K6;
 //   K6  every target cell runs over all source cells in 256-cell shared-memory
 //       tiles and adds the bare point-dipole term (3 e e - 1)/r^3 m_j in FP32,
 //       folding each tile's sum into FP64;
@@ -45,6 +45,7 @@ struct DipoleState {
    int solver = 1;
    int update_rate = 100;
    double size = 0.0, cutoff = 2.0;
+   int glog = 0;                // log2 of the lanes per cell of K5
    int* cell_start = nullptr;   // [nc+1] offsets into cell_atoms
    int* cell_atoms = nullptr;   // atoms sorted by cell (magnetic atoms only)
    double* mag = nullptr;       // [3][nc] cell moment, J/T
@@ -73,36 +74,43 @@ struct DipoleState {
    bool pending = false;        // partial moments in `mag`, field not yet computed
 };
 
+constexpr int kFinishFewCells = 65536;
+
 static DipoleState* dip_of(vgpu_ctx* h) { return (DipoleState*)h->extras[2]; }
 
-// K5: cell moments (cells.cpp mag()), FP64.
+// K5: cell moments (cells.cpp mag()), FP64.  G lanes per cell, G the power of
+// two at or above the mean atoms of a cell (2x2x2 simple-cubic cells hold 8:
+// with a whole warp per cell three quarters of the lanes had no atom, 43 us at
+// 125,000 cells).
 template <typename R>
-__global__ void cell_moment_kernel(int nc, const int* __restrict__ start, const int* __restrict__ atoms,
-                                   const R* __restrict__ sx, const R* __restrict__ sy, const R* __restrict__ sz,
-                                   const int* __restrict__ mat, const MatParams<R>* __restrict__ mp,
-                                   const double* __restrict__ mus_SI, double* __restrict__ mag,
-                                   const float4* __restrict__ pos, float4* __restrict__ mom) {
-   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-   const int lane = threadIdx.x & 31;
-   if (warp >= nc) return;
+__global__ void __launch_bounds__(256)
+    cell_moment_kernel(int nc, int glog, const int* __restrict__ start, const int* __restrict__ atoms,
+                       const R* __restrict__ sx, const R* __restrict__ sy, const R* __restrict__ sz,
+                       const int* __restrict__ mat, const double* __restrict__ mus_SI, double* __restrict__ mag,
+                       float4* __restrict__ mom) {
+   pdl_begin();
+   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+   const int G = 1 << glog, c = t >> glog, lane = t & (G - 1);
    double mx = 0.0, my = 0.0, mz = 0.0;
-   for (int k = start[warp] + lane; k < start[warp + 1]; k += 32) {
-      const int i = atoms[k];
-      const double mu = mus_SI[mat ? mat[i] : 0];
-      mx += (double)sx[i] * mu;
-      my += (double)sy[i] * mu;
-      mz += (double)sz[i] * mu;
+   if (c < nc) {
+      const int e = start[c + 1];
+      for (int k = start[c] + lane; k < e; k += G) {
+         const int i = atoms[k];
+         const double mu = mus_SI[mat ? mat[i] : 0];
+         mx += (double)sx[i] * mu;
+         my += (double)sy[i] * mu;
+         mz += (double)sz[i] * mu;
+      }
    }
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) {
+   for (int o = G >> 1; o > 0; o >>= 1) {
       mx += __shfl_xor_sync(0xffffffffu, mx, o);
       my += __shfl_xor_sync(0xffffffffu, my, o);
       mz += __shfl_xor_sync(0xffffffffu, mz, o);
    }
-   if (lane == 0) {
-      mag[warp] = mx; mag[nc + warp] = my; mag[2 * nc + warp] = mz;
+   if (lane == 0 && c < nc) {
+      mag[c] = mx; mag[nc + c] = my; mag[2 * nc + c] = mz;
       const double imuB = 1.0 / 9.27400915e-24;
-      mom[warp] = make_float4((float)(mx * imuB), (float)(my * imuB), (float)(mz * imuB), 0.f);
+      mom[c] = make_float4((float)(mx * imuB), (float)(my * imuB), (float)(mz * imuB), 0.f);
    }
 }
 
@@ -150,8 +158,11 @@ __global__ void __launch_bounds__(kFieldTile) cell_field_kernel(int nc, const fl
       float fx[T], fy[T], fz[T];
 #pragma unroll
       for (int q = 0; q < T; ++q) fx[q] = fy[q] = fz[q] = 0.f;
+      // the tile's own sources: a share of few cells is not padded to a whole
+      // tile (1,331 cells in 64 shares of 21: 53 us with padding)
+      const int live = min(kFieldTile, src1 - base);
 #pragma unroll 4
-      for (int k = 0; k < kFieldTile; ++k) {
+      for (int k = 0; k < live; ++k) {
          const float4 pj = sp[k];
          const float4 mj = sm[k];
 #pragma unroll
@@ -193,33 +204,61 @@ __global__ void near_ell_kernel(int npairs, int nc, int maxp, const int* __restr
    for (int q = 0; q < 6; ++q) te[((size_t)q * maxp + k) * nc + i] = near_t[(size_t)q * npairs + p];
 }
 
-// near-field correction and final scaling (update.cpp:56-99)
-template <typename R>
-__global__ void cell_finish_kernel(int nc, const int* __restrict__ near_cnt, const int* __restrict__ near_je,
-                                   const double* __restrict__ near_te, int maxp, const double* __restrict__ mag,
-                                   const double* __restrict__ self, const float4* __restrict__ pos,
-                                   double* __restrict__ field, R* __restrict__ tb, R* __restrict__ thd) {
-   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Near-field correction and final scaling (update.cpp:56-99).  The pairs' FP64
+// tensors are the bytes of this kernel (52 B a pair, about 33 pairs a cell),
+// so what counts is how many loads are in flight.  L = 1: a thread per cell,
+// four pairs' loads issued together; L = 8: eight lanes per cell, for grids
+// with too few cells to fill the GPU with one thread each.
+template <typename R, int L>
+__global__ void __launch_bounds__(128)
+    cell_finish_kernel(int nc, const int* __restrict__ near_cnt, const int* __restrict__ near_je,
+                       const double* __restrict__ near_te, int maxp, const double* __restrict__ mag,
+                       const double* __restrict__ self, const float4* __restrict__ pos, double* __restrict__ field,
+                       R* __restrict__ tb, R* __restrict__ thd) {
+   pdl_begin();
+   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+   const int i = t / L, lane = t % L;
+   const double imuB = 1.0 / 9.27400915e-24;
+   double fx = 0.0, fy = 0.0, fz = 0.0;
+   if (i < nc && lane == 0) { fx = field[i]; fy = field[nc + i]; fz = field[2 * nc + i]; }
+   if (i < nc && near_cnt) {
+      const size_t qs = (size_t)maxp * nc;
+      const int cnt = near_cnt[i];
+      constexpr int U = 4;
+      for (int k0 = lane; k0 < cnt; k0 += U * L) {
+         int j[U];
+         double T[U][6];
+#pragma unroll
+         for (int u = 0; u < U; ++u) {
+            const size_t e = (size_t)(k0 + u * L) * nc + i;
+            const bool on = k0 + u * L < cnt;
+            j[u] = on ? near_je[e] : -1;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) T[u][q] = on ? near_te[q * qs + e] : 0.0;
+         }
+#pragma unroll
+         for (int u = 0; u < U; ++u) {
+            if (j[u] < 0) continue;
+            const double mx = mag[j[u]] * imuB, my = mag[nc + j[u]] * imuB, mz = mag[2 * nc + j[u]] * imuB;
+            fx += mx * T[u][0] + my * T[u][1] + mz * T[u][2];
+            fy += mx * T[u][1] + my * T[u][3] + mz * T[u][4];
+            fz += mx * T[u][2] + my * T[u][4] + mz * T[u][5];
+         }
+      }
+   }
+   if (L > 1) {
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) {
+         fx += __shfl_xor_sync(0xffffffffu, fx, o);
+         fy += __shfl_xor_sync(0xffffffffu, fy, o);
+         fz += __shfl_xor_sync(0xffffffffu, fz, o);
+      }
+      if (lane != 0) return;
+   }
    if (i > nc) return;
    if (i == nc) {  // zero row read by non-magnetic atoms
       for (int q = 0; q < 3; ++q) { tb[q * (nc + 1) + nc] = (R)0; thd[q * (nc + 1) + nc] = (R)0; }
       return;
-   }
-   const double imuB = 1.0 / 9.27400915e-24;
-   double fx = field[i], fy = field[nc + i], fz = field[2 * nc + i];
-   if (near_cnt) {
-      const size_t qs = (size_t)maxp * nc;
-      const int cnt = near_cnt[i];
-      for (int k = 0; k < cnt; ++k) {
-         const size_t e = (size_t)k * nc + i;
-         const int j = near_je[e];
-         const double mx = mag[j] * imuB, my = mag[nc + j] * imuB, mz = mag[2 * nc + j] * imuB;
-         const double txx = near_te[e], txy = near_te[qs + e], txz = near_te[2 * qs + e];
-         const double tyy = near_te[3 * qs + e], tyz = near_te[4 * qs + e], tzz = near_te[5 * qs + e];
-         fx += mx * txx + my * txy + mz * txz;
-         fy += mx * txy + my * tyy + mz * tyz;
-         fz += mx * txz + my * tyz + mz * tzz;
-      }
    }
    const double k = 9.27400915e-01;
    const bool has = pos[i].w != 0.f;
@@ -316,12 +355,14 @@ static int dipole_moments_typed(vgpu_ctx* h) {
    SysDev& S = h->sys;
    const int nc = d->nc;
    h->prof_begin(PROF_DIPOLE);
-   cell_moment_kernel<R><<<(nc * 32 + 255) / 256, 256, 0, h->stream>>>(
-       nc, d->cell_start, d->cell_atoms, (const R*)S.s[0], (const R*)S.s[1], (const R*)S.s[2], (const int*)S.mat,
-       (const MatParams<R>*)S.mp, S.mus_SI, d->mag, d->pos, d->mom);
+   const long long threads = (long long)nc << d->glog;
+   const cudaError_t e = launch_pdl(cell_moment_kernel<R>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
+                                    h->stream, nc, d->glog, (const int*)d->cell_start, (const int*)d->cell_atoms,
+                                    (const R*)S.s[0], (const R*)S.s[1], (const R*)S.s[2], (const int*)S.mat,
+                                    (const double*)S.mus_SI, d->mag, d->mom);
    h->prof_end(PROF_DIPOLE);
    h->kernel_launches += 1;
-   return cuda_err(h, cudaGetLastError(), "dipole cell moments");
+   return cuda_err(h, e, "dipole cell moments");
 }
 
 // K6 and the finish from the cell moments in d->mag; with_mom: first convert
@@ -352,12 +393,18 @@ static int dipole_field_typed(vgpu_ctx* h, bool with_mom) {
       cell_field_kernel<<<dim3(tblocks, splits), kFieldTile, 0, h->stream>>>(nc, d->pos, d->mom, d->field);
       launches += 1;
    }
-   cell_finish_kernel<R><<<(nc + 1 + 255) / 256, 256, 0, h->stream>>>(
-       nc, d->near_cnt, d->near_je, d->near_te, d->maxp, d->mag, d->self, d->pos, d->field, (R*)d->table_b,
-       (R*)d->table_hd);
+   // below two waves of one thread per cell, eight lanes per cell
+   const bool few = nc < kFinishFewCells;
+   const unsigned blocks = (unsigned)(((long long)(nc + 1) * (few ? 8 : 1) + 127) / 128);
+   cudaError_t e = cudaGetLastError();
+   if (e == cudaSuccess)
+      e = launch_pdl(few ? cell_finish_kernel<R, 8> : cell_finish_kernel<R, 1>, dim3(blocks), dim3(128), 0, h->stream,
+                     nc, (const int*)d->near_cnt, (const int*)d->near_je, (const double*)d->near_te, d->maxp,
+                     (const double*)d->mag, (const double*)d->self, (const float4*)d->pos, d->field, (R*)d->table_b,
+                     (R*)d->table_hd);
    h->prof_end(PROF_DIPOLE);
    h->kernel_launches += launches;
-   return cuda_err(h, cudaGetLastError(), "dipole field");
+   return cuda_err(h, e, "dipole field");
 }
 
 // whole system: moments and field; shard: partial moments, field pending
@@ -472,6 +519,7 @@ static int dipole_build(vgpu_ctx* h, const vgpu_dipole_desc* dd, int ng, const i
       const int c = dd->atom_cell[gid(i)];
       acell[i] = (dd->cell_natoms[c] > 0 && magnetic[S.type_host[i]]) ? c : nc;
    }
+   while (d->glog < 5 && ((int64_t)nc << d->glog) < (int64_t)atoms.size()) d->glog++;
    std::vector<float4> pos(nc);
    std::vector<double> self(nc);
    for (int c = 0; c < nc; ++c) {

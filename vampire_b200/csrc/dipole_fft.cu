@@ -1,4 +1,4 @@
-// Far-field macrocell dipole sum by FFT convolution (FP64).
+// Far-field macrocell dipole sum by FFT convolution.
 //
 // The far field of every cell is H_i = sum_{j != i} T(r_j - r_i) m_j with the
 // bare point-dipole tensor T(r) = (3 e e - 1)/|r|^3 (src/dipole/inter.cpp:66-80
@@ -9,32 +9,36 @@
 // grid with T.  It is evaluated as a circular convolution on a grid padded to
 // P >= 2G - 1 points per axis (G = occupied extent), with P a power of two:
 //
-//   scatter  m_j (mu_B) into the G-box of three complex grids (zero at empty
-//            cells of the box)
-//   FFT      each grid along x and y (radix-2, one shared-memory tile of lines
-//            per block; strided axes load W adjacent x columns per block so
-//            every global access is a W*16-byte segment)
-//   z        per z column: forward transform, H(k) = T(k) M(k) (T symmetric
-//            3x3, six spectra computed once), inverse transform, in one kernel
-//   iFFT     along y, x, and gather H at the occupied cells (1/P^3 scaling).
+//   x    forward transform of the real lines of the G-box, two lines as the
+//        real and imaginary parts of one; the moments (mu_B) are read straight
+//        from the cells, and the P/2 + 1 points that determine the spectrum of
+//        a real line are written
+//   y    forward transform in place, planes z < G
+//   z    per z column: forward transform, H(k) = T(k) M(k), inverse transform
+//        in one kernel, the spectra in registers
+//   y    inverse transform in place, points y < G kept
+//   x    inverse transform of line pairs, written to the cells' field
 //
-// The transforms skip the lines that carry only zeros or whose results are not
-// needed: the moments occupy the G-box, so the forward x pass runs only the
-// gy*gz lines of the box (points past gx read as zero), the y pass only the
-// planes z < gz (points past gy read as zero) and the z transform reads zero
-// past gz and keeps only z < gz; the inverse y pass runs and keeps only those
-// planes' y < gy, the inverse x pass only the box lines' x < gx.  At a 50^3
-// grid (P = 128) this is about half of the line transforms of full passes,
-// the spectra never leave shared memory, and the grid needs no clearing.
+// T is real and even under r -> -r, so its spectrum is real; each component is
+// even or odd in every single axis, so one octant of it (kx, ky, kz <= P/2,
+// the rest by sign) is all that is kept: 6 (P/2+1)^3 reals, 6.6 MB in FP32 at
+// P = 128, resident in L2, where the full complex spectra were 100 MB read on
+// every update.
+//
+// The line transforms keep 8 points per thread in registers and go through
+// shared memory once between radix-8 passes (radix 2 or 4 last), ceil(log2 P
+// / 3) passes in all.  Blocks are bound by latency and L2 traffic, not by
+// arithmetic: with lines of 128 points the grids are 3 x 3.3 MB.  At 125,000
+// cells (50^3, P = 128) the five launches measured take the place of radix-2
+// passes through shared memory over complex lines (two barriers and integer
+// divisions per point and stage): 376 us then; see fft_z_kernel for the split.
 //
 // Precision follows the handle: in the FP64 build every step is FP64, so the
 // result equals the direct FP64 sum to rounding (~1e-15 of the field); the
 // FP32 production handles transform FP32 grids (the tensor spectra computed
 // in FP64 once and rounded, twiddles rounded from FP64, moments and fields
-// FP64 at the ends), about 1e-6 of the field.  Cost O(P^3 log P) instead of
-// O(Nc^2): at 125,000 cells (a 50^3 grid, P = 128) a few hundred microseconds
-// instead of tens of milliseconds.  Twiddle factors are tabulated on the host
-// in double precision.
+// FP64 at the ends), a few 1e-7 of the field.  Cost O(P^3 log P) instead of
+// O(Nc^2).
 #include "dipole_fft.cuh"
 
 #include <cuda_runtime.h>
@@ -43,244 +47,335 @@
 #include <cmath>
 #include <vector>
 
+#include "vgpu_internal.cuh"
+
 namespace vgpu {
 
 struct FFTField {
    int nc = 0;
-   int p[3] = {0, 0, 0};       // padded points per axis (powers of two)
+   int p[3] = {0, 0, 0};       // padded points per axis (powers of two, at least 8)
    int logp[3] = {0, 0, 0};
    int g[3] = {0, 0, 0};       // occupied extent in cells
+   int hx = 0;                 // stored points of an x spectrum: p[0] / 2 + 1
    size_t np = 0;              // p[0] * p[1] * p[2]
-   double2* tspec = nullptr;   // [6][np] spectra of Txx, Txy, Txz, Tyy, Tyz, Tzz
-   double2* grid = nullptr;    // [3][np] moment grids, transformed in place
-   double2* tw[3] = {nullptr, nullptr, nullptr};  // [p/2] exp(-2 pi i k / p) per axis
-   bool fp32 = false;          // FP32 transforms (the buffers below) instead of the FP64 ones
-   float2* tspec32 = nullptr;  // [6][np] the spectra rounded to FP32
-   float2* grid32 = nullptr;   // [3][np]
-   float2* tw32[3] = {nullptr, nullptr, nullptr};
-   int* cell_lin = nullptr;    // [nc] linear grid index, or -1 (empty cell)
+   bool fp32 = false;          // precision of grid, tspec and tw
+   void* tspec = nullptr;      // [6][p[2]/2+1][p[1]/2+1][hx] real spectra of Txx, Txy, Txz, Tyy, Tyz, Tzz
+   void* grid = nullptr;       // [3][g[2]][p[1]][hx] complex, transformed in place
+   void* tw[3] = {nullptr, nullptr, nullptr};  // [p] exp(-2 pi i k / p) per axis
    int* box_cell = nullptr;    // [gx*gy*gz] cell at each box point (x fastest), or -1
 };
 
 namespace {
 
-constexpr int kFFTThreads = 256;
-constexpr int kFFTTile = 2048;  // complex points per block tile (32 KB of shared memory)
+template <typename C> struct RealOf;
+template <> struct RealOf<float2> { using type = float; };
+template <> struct RealOf<double2> { using type = double; };
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
+   return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
 }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// complex value of the transform's precision
-template <typename C> __device__ __forceinline__ C cval(double x, double y);
-template <> __device__ __forceinline__ double2 cval<double2>(double x, double y) { return make_double2(x, y); }
-template <> __device__ __forceinline__ float2 cval<float2>(double x, double y) {
-   return make_float2((float)x, (float)y);
+template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return {a.x + b.x, a.y + b.y}; }
+template <typename C> __device__ __forceinline__ C csub(C a, C b) { return {a.x - b.x, a.y - b.y}; }
+// times -i (forward) or +i (inverse)
+template <typename C, bool INV> __device__ __forceinline__ C crot(C a) {
+   if (INV) return {-a.y, a.x};
+   return {a.y, -a.x};
 }
 
-// radix-2 decimation-in-time butterflies over `nlines` lines of n points held
-// in shared memory in bit-reversed order (line-major); results in natural order
-template <typename C>
-__device__ void fft_smem(C* s, int n, int nlines, const C* __restrict__ tw, bool inverse) {
-   const int half = n >> 1;
-   for (int h = 1; h < n; h <<= 1) {
-      const int step = half / h;  // twiddle stride: exp(-2 pi i j / (2h)) = tw[j * n / (2h)]
-      for (int b = threadIdx.x; b < nlines * half; b += blockDim.x) {
-         const int line = b / half, k = b - line * half;
-         const int j = k % h, grp = k / h;
-         const int i0 = line * n + grp * 2 * h + j, i1 = i0 + h;
-         C w = tw[j * step];
-         if (inverse) w.y = -w.y;
-         const C u = s[i0];
-         const C v = cmul(w, s[i1]);
-         s[i0] = {u.x + v.x, u.y + v.y};
-         s[i1] = {u.x - v.x, u.y - v.y};
+// discrete Fourier transforms of 2, 4 and 8 points in registers, natural order
+template <typename C, bool INV> __device__ __forceinline__ void dft4(C& a, C& b, C& c, C& d) {
+   const C t0 = cadd(a, c), t1 = csub(a, c), t2 = cadd(b, d), t3 = crot<C, INV>(csub(b, d));
+   a = cadd(t0, t2); b = cadd(t1, t3); c = csub(t0, t2); d = csub(t1, t3);
+}
+template <typename C, bool INV, int R> __device__ __forceinline__ void dft(C u[R]) {
+   if constexpr (R == 2) {
+      const C t = u[0];
+      u[0] = cadd(t, u[1]);
+      u[1] = csub(t, u[1]);
+   } else if constexpr (R == 4) {
+      dft4<C, INV>(u[0], u[1], u[2], u[3]);
+   } else {
+      using R1 = typename RealOf<C>::type;
+      C e0 = u[0], e1 = u[2], e2 = u[4], e3 = u[6], o0 = u[1], o1 = u[3], o2 = u[5], o3 = u[7];
+      dft4<C, INV>(e0, e1, e2, e3);
+      dft4<C, INV>(o0, o1, o2, o3);
+      const R1 h = (R1)0.70710678118654752440;
+      const C r1 = crot<C, INV>(o1), r3 = crot<C, INV>(o3);
+      o1 = {h * (o1.x + r1.x), h * (o1.y + r1.y)};  // (1 -+ i)/sqrt 2 times
+      o2 = crot<C, INV>(o2);
+      o3 = {h * (r3.x - o3.x), h * (r3.y - o3.y)};  // (-1 -+ i)/sqrt 2 times
+      u[0] = cadd(e0, o0); u[4] = csub(e0, o0);
+      u[1] = cadd(e1, o1); u[5] = csub(e1, o1);
+      u[2] = cadd(e2, o2); u[6] = csub(e2, o2);
+      u[3] = cadd(e3, o3); u[7] = csub(e3, o3);
+   }
+}
+
+// Transforms of NC lines of N = 2^LOGN points, each held by the same N/8
+// threads: thread j has points j + i N/8 (i = 0..7) of line c in v[c], before
+// and after (natural order both times).  Passes of radix 8, the last one of
+// the radix that is left; between passes the points go through shared memory
+// at idx(c, point), the NC lines between the same two barriers.  Every thread
+// of the block takes part.  NSLOG: log2 of the points already combined.
+template <typename C, int LOGN, bool INV, int NSLOG, int NC, typename Idx>
+__device__ __forceinline__ void fft_lines(C (&v)[NC][8], int j, C* s, Idx idx, const C* __restrict__ tw) {
+   constexpr int RL = LOGN - NSLOG >= 3 ? 3 : LOGN - NSLOG;
+   constexpr int R = 1 << RL, NB = 8 / R, NS = 1 << NSLOG, T = (1 << LOGN) / 8;
+   constexpr bool LAST = NSLOG + RL == LOGN;
+#pragma unroll
+   for (int q = 0; q < NB; ++q) {
+      const int bb = j + q * T, k = bb & (NS - 1);
+      C w[R];
+      if (NSLOG > 0) {
+#pragma unroll
+         for (int r = 1; r < R; ++r) {
+            w[r] = __ldg(tw + ((k * r) << (LOGN - NSLOG - RL)));
+            if (INV) w[r].y = -w[r].y;
+         }
       }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+         C u[R];
+#pragma unroll
+         for (int r = 0; r < R; ++r) u[r] = v[c][q + r * NB];
+         if (NSLOG > 0) {
+#pragma unroll
+            for (int r = 1; r < R; ++r) u[r] = cmul(w[r], u[r]);
+         }
+         dft<C, INV, R>(u);
+         if (LAST) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[c][q + r * NB] = u[r];
+         } else {
+            const int o = ((bb >> NSLOG) << (NSLOG + RL)) + k;
+#pragma unroll
+            for (int r = 0; r < R; ++r) s[idx(c, o + r * NS)] = u[r];
+         }
+      }
+   }
+   if constexpr (!LAST) {
       __syncthreads();
-   }
-}
-
-// lines along x (contiguous): block = `lines` lines of one grid, line r of
-// the nrows transformed being the x line (y, z) = (r % rpp, r / rpp) at
-// (z * py + y) * n; points p >= ld read as zero, points p < st are stored
-template <typename C>
-__global__ void __launch_bounds__(kFFTThreads) fft_x_kernel(C* __restrict__ data, size_t np, int n, int logn,
-                                                            int lines, const C* __restrict__ tw, int inverse,
-                                                            int nrows, int rpp, int py, int ld, int st) {
-   __shared__ C s[kFFTTile];
-   C* grid = data + (size_t)blockIdx.y * np;
-   const int r0 = blockIdx.x * lines;
-   const int tot = lines * n;
-   auto row = [&](int r) { return ((size_t)(r / rpp) * py + (size_t)(r % rpp)) * n; };
-   for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      const int line = e / n, p = e - line * n;
-      const int r = r0 + line;
-      s[line * n + (int)(__brev((unsigned)p) >> (32 - logn))] =
-          r < nrows && p < ld ? grid[row(r) + p] : cval<C>(0.0, 0.0);
-   }
-   __syncthreads();
-   fft_smem(s, n, lines, tw, inverse != 0);
-   for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      const int line = e / n, p = e - line * n;
-      const int r = r0 + line;
-      if (r < nrows && p < st) grid[row(r) + p] = s[e];
-   }
-}
-
-// lines along y or z: block = W adjacent x columns of one (other) index;
-// point p of column w sits at base + p * stride + w; points p >= ld read as
-// zero, points p < st are stored
-template <typename C>
-__global__ void __launch_bounds__(kFFTThreads) fft_strided_kernel(C* __restrict__ data, size_t np, int n, int logn,
-                                                                  int W, size_t stride, size_t other_stride,
-                                                                  const C* __restrict__ tw, int inverse, int ld,
-                                                                  int st) {
-   __shared__ C s[kFFTTile];
-   C* base = data + (size_t)blockIdx.z * np + (size_t)blockIdx.y * other_stride + (size_t)blockIdx.x * W;
-   const int tot = W * n;
-   for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      const int p = e / W, w = e - p * W;
-      s[w * n + (int)(__brev((unsigned)p) >> (32 - logn))] =
-          p < ld ? base[(size_t)p * stride + w] : cval<C>(0.0, 0.0);
-   }
-   __syncthreads();
-   fft_smem(s, n, W, tw, inverse != 0);
-   for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      const int p = e / W, w = e - p * W;
-      if (p < st) base[(size_t)p * stride + w] = s[w * n + p];
-   }
-}
-
-// The middle of the convolution in one pass over z columns: for W adjacent x
-// columns at one y, the three moment components' forward z transforms (points
-// z >= gz read as zero), the product H(k) = T(k) M(k) at every k, and the
-// inverse z transforms, of which z < gz is stored.  The same butterflies and
-// products as separate z passes around multiply_kernel, without writing the
-// spectra to memory and reading them back.
-constexpr int kFuseTile = 3072;  // complex points per block: 3 components x W x pz (48 KB)
-
-template <typename C>
-__device__ __forceinline__ void tensor_times(const C* __restrict__ t, size_t np, size_t q, C mx, C my, C mz, C h[3]) {
-   const C xx = t[q], xy = t[np + q], xz = t[2 * np + q];
-   const C yy = t[3 * np + q], yz = t[4 * np + q], zz = t[5 * np + q];
-   C hx = cmul(xx, mx), hy = cmul(xy, mx), hz = cmul(xz, mx);
-   C a = cmul(xy, my), b = cmul(xz, mz);
-   hx.x += a.x + b.x; hx.y += a.y + b.y;
-   a = cmul(yy, my); b = cmul(yz, mz);
-   hy.x += a.x + b.x; hy.y += a.y + b.y;
-   a = cmul(yz, my); b = cmul(zz, mz);
-   hz.x += a.x + b.x; hz.y += a.y + b.y;
-   h[0] = hx; h[1] = hy; h[2] = hz;
-}
-
-template <typename C>
-__global__ void __launch_bounds__(kFFTThreads) fft_z_multiply_kernel(C* __restrict__ data, const C* __restrict__ t,
-                                                                     size_t np, int px, int py, int n, int logn, int W,
-                                                                     int gz, const C* __restrict__ tw) {
-   __shared__ C s[kFuseTile];
-   const size_t stride = (size_t)px * py;
-   const size_t col0 = (size_t)blockIdx.y * px + (size_t)blockIdx.x * W;  // (x0, y) in the z = 0 plane
-   const int tot = W * n;
-   for (int e = threadIdx.x; e < 3 * tot; e += blockDim.x) {
-      const int c = e / tot, r = e - c * tot;
-      const int p = r / W, w = r - p * W;
-      s[(c * W + w) * n + (int)(__brev((unsigned)p) >> (32 - logn))] =
-          p < gz ? data[(size_t)c * np + col0 + (size_t)p * stride + w] : cval<C>(0.0, 0.0);
-   }
-   __syncthreads();
-   fft_smem(s, n, 3 * W, tw, false);
-   // H = T M at every (w, k), all read before any is written back at its
-   // bit-reversed position for the inverse
-   constexpr int kMaxPer = kFuseTile / 3 / kFFTThreads;  // points per thread
-   C h[kMaxPer][3];
 #pragma unroll
-   for (int u = 0; u < kMaxPer; ++u) {
-      const int r = threadIdx.x + u * kFFTThreads;
-      if (r < tot) {
-         const int k = r / W, w = r - k * W;
-         tensor_times(t, np, col0 + (size_t)k * stride + w, s[w * n + k], s[(W + w) * n + k], s[(2 * W + w) * n + k],
-                      h[u]);
-      }
-   }
-   __syncthreads();
+      for (int c = 0; c < NC; ++c)
 #pragma unroll
-   for (int u = 0; u < kMaxPer; ++u) {
-      const int r = threadIdx.x + u * kFFTThreads;
-      if (r < tot) {
-         const int k = r / W, w = r - k * W;
-         const int kr = (int)(__brev((unsigned)k) >> (32 - logn));
-#pragma unroll
-         for (int c = 0; c < 3; ++c) s[(c * W + w) * n + kr] = h[u][c];
-      }
-   }
-   __syncthreads();
-   fft_smem(s, n, 3 * W, tw, true);
-   for (int e = threadIdx.x; e < 3 * tot; e += blockDim.x) {
-      const int c = e / tot, r = e - c * tot;
-      const int p = r / W, w = r - p * W;
-      if (p < gz) data[(size_t)c * np + col0 + (size_t)p * stride + w] = s[(c * W + w) * n + p];
+         for (int i = 0; i < 8; ++i) v[c][i] = s[idx(c, j + i * T)];
+      __syncthreads();  // s may be written again
+      fft_lines<C, LOGN, INV, NSLOG + RL>(v, j, s, idx, tw);
    }
 }
 
-// bare tensor on the padded grid: offset (dx, dy, dz) cells, zero at the
-// origin and beyond the occupied extent
-__global__ void tensor_grid_kernel(double2* __restrict__ t, size_t np, int px, int py, int pz, int gx, int gy, int gz,
-                                   double size) {
-   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < np; q += (size_t)gridDim.x * blockDim.x) {
-      const int x = (int)(q % px), y = (int)((q / px) % py), z = (int)(q / ((size_t)px * py));
+// lines per block of the strided transforms: 2,048 points (256 threads) and
+// at most 64 lines.  16 adjacent columns at 128 points: a 128-byte segment per
+// point in FP32.
+constexpr int lines_of(int logn) { return (2048 >> logn) < 64 ? (2048 >> logn) : 64; }
+constexpr int threads_of(int logn) { return lines_of(logn) << (logn - 3); }
+
+// lines along y or z, in place: line l starts at (l / inner) * outer + l %
+// inner, its points are `ps` apart; points p >= ld read as zero, points p < st
+// are stored.  blockIdx.y: component (cs apart).
+template <typename C, int LOGN, bool INV>
+__global__ void __launch_bounds__(threads_of(LOGN)) fft_strided_kernel(C* __restrict__ data, size_t cs, int nlines,
+                                                                       int inner, size_t outer, size_t ps,
+                                                                       const C* __restrict__ tw, int ld, int st) {
+   constexpr int W = lines_of(LOGN), T = (1 << LOGN) / 8;
+   __shared__ C s[W << LOGN];
+   pdl_begin();
+   const int w = threadIdx.x % W, j = threadIdx.x / W;
+   const int l = blockIdx.x * W + w;
+   const bool on = l < nlines;
+   C* base = data + (size_t)blockIdx.y * cs + (size_t)(l / inner) * outer + (size_t)(l % inner);
+   C v[1][8];
+#pragma unroll
+   for (int i = 0; i < 8; ++i) {
+      const int p = j + i * T;
+      v[0][i] = on && p < ld ? base[(size_t)p * ps] : C{0, 0};
+   }
+   fft_lines<C, LOGN, INV, 0>(v, j, s, [&](int, int p) { return p * W + w; }, tw);
+#pragma unroll
+   for (int i = 0; i < 8; ++i) {
+      const int p = j + i * T;
+      if (on && p < st) base[(size_t)p * ps] = v[0][i];
+   }
+}
+
+// sources of the real x lines: row r of component c, point x
+struct MomentRows {  // the G-box, x fastest; zero at its empty cells
+   const int* box_cell;
+   const double* mag;
+   int nc, gx;
+   __device__ double operator()(int c, int r, int x) const {
+      if (x >= gx) return 0.0;
+      const int cell = __ldg(box_cell + (size_t)r * gx + x);
+      return cell >= 0 ? __ldg(mag + (size_t)c * nc + cell) * (1.0 / 9.27400915e-24) : 0.0;
+   }
+};
+
+struct TensorRows {  // bare tensor on the padded grid, zero at the origin and beyond the occupied extent
+   int px, py, pz, gx, gy, gz;
+   double size;
+   __device__ double operator()(int c, int r, int x) const {
+      const int y = r % py, z = r / py;
       const int dx = x < px / 2 ? x : x - px, dy = y < py / 2 ? y : y - py, dz = z < pz / 2 ? z : z - pz;
-      double v[6] = {0, 0, 0, 0, 0, 0};
-      const bool in = abs(dx) < gx && abs(dy) < gy && abs(dz) < gz && (dx | dy | dz) != 0;
-      if (in) {
-         const double rx = dx * size, ry = dy * size, rz = dz * size;
-         const double rij = 1.0 / sqrt(rx * rx + ry * ry + rz * rz);
-         const double ex = rx * rij, ey = ry * rij, ez = rz * rij;
-         const double r3 = rij * rij * rij;
-         v[0] = (3.0 * ex * ex - 1.0) * r3;
-         v[1] = (3.0 * ex * ey) * r3;
-         v[2] = (3.0 * ex * ez) * r3;
-         v[3] = (3.0 * ey * ey - 1.0) * r3;
-         v[4] = (3.0 * ey * ez) * r3;
-         v[5] = (3.0 * ez * ez - 1.0) * r3;
-      }
+      if (!(abs(dx) < gx && abs(dy) < gy && abs(dz) < gz && (dx | dy | dz) != 0)) return 0.0;
+      const double rx = dx * size, ry = dy * size, rz = dz * size;
+      const double rij = 1.0 / sqrt(rx * rx + ry * ry + rz * rz);
+      const double e[3] = {rx * rij, ry * rij, rz * rij};
+      const double r3 = rij * rij * rij;
+      const int a = c < 3 ? 0 : c < 5 ? 1 : 2, b = c < 3 ? c : c < 5 ? c - 2 : 2;
+      return (3.0 * e[a] * e[b] - (a == b ? 1.0 : 0.0)) * r3;
+   }
+};
+
+// Row r of the box or grid starts at row_start(r): rows per plane `rpp`, the
+// planes hold `py` rows of hx points.
+__device__ __forceinline__ size_t row_start(int r, int rpp, int py, int hx) {
+   return ((size_t)(r / rpp) * py + (size_t)(r % rpp)) * hx;
+}
+
+// lines of a block of the x transforms: 1,024 points, at least one line
+constexpr int xlines_of(int logn) { return logn >= 10 ? 1 : 1024 >> logn; }
+
+// forward x: rows 2t and 2t + 1 as real and imaginary part of complex line t;
+// the spectra are taken apart by their symmetry (Z(N - k) from shared memory)
+template <typename C, int LOGN, typename Rows>
+__global__ void __launch_bounds__(128) fft_x_forward_kernel(const Rows rows, C* __restrict__ out, size_t cs, int nrows,
+                                                            int rpp, int py, const C* __restrict__ tw) {
+   constexpr int N = 1 << LOGN, T = N / 8, L = xlines_of(LOGN), NP = N + N / 8, HX = N / 2 + 1;
+   using R = typename RealOf<C>::type;
+   __shared__ C s[L * NP];
+   pdl_begin();
+   const int j = threadIdx.x % T, line = threadIdx.x / T;
+   const int ra = 2 * (blockIdx.x * L + line), rb = ra + 1;
+   const int c = blockIdx.y;
+   auto idx = [&](int, int p) { return line * NP + p + (p >> 3); };  // padded: points 8 apart in different banks
+   C v[1][8];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) t[k * np + q] = make_double2(v[k], 0.0);
+   for (int i = 0; i < 8; ++i) {
+      const int x = j + i * T;
+      v[0][i] = {(R)(ra < nrows ? rows(c, ra, x) : 0.0), (R)(rb < nrows ? rows(c, rb, x) : 0.0)};
+   }
+   fft_lines<C, LOGN, false, 0>(v, j, s, idx, tw);
+#pragma unroll
+   for (int i = 0; i < 8; ++i) s[idx(0, j + i * T)] = v[0][i];
+   __syncthreads();
+   C* oa = out + (size_t)c * cs + row_start(ra, rpp, py, HX);
+   C* ob = out + (size_t)c * cs + row_start(rb, rpp, py, HX);
+#pragma unroll
+   for (int i = 0; i < 8; ++i) {
+      const int k = j + i * T;
+      if (k <= N / 2) {
+         const C z = v[0][i], n = s[idx(0, (N - k) & (N - 1))];
+         const R h = (R)0.5;
+         if (ra < nrows) oa[k] = {h * (z.x + n.x), h * (z.y - n.y)};
+         if (rb < nrows) ob[k] = {h * (z.y + n.y), h * (n.x - z.x)};
+      }
    }
 }
 
-// the moments (mu_B) at every point of the G-box, zero at its empty cells
-template <typename C>
-__global__ void scatter_moments_kernel(int nc, const int* __restrict__ box_cell, int gx, int gy, int nbox,
-                                       const double* __restrict__ mag, C* __restrict__ grid, int px, int py,
-                                       size_t np) {
-   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-   if (b >= nbox) return;
-   const int c = box_cell[b];
-   const int x = b % gx, y = (b / gx) % gy, z = b / (gx * gy);
-   const size_t q = ((size_t)z * py + y) * px + x;
-   const double imuB = 1.0 / 9.27400915e-24;
-   grid[q] = cval<C>(c >= 0 ? mag[c] * imuB : 0.0, 0.0);
-   grid[np + q] = cval<C>(c >= 0 ? mag[nc + c] * imuB : 0.0, 0.0);
-   grid[2 * np + q] = cval<C>(c >= 0 ? mag[2 * nc + c] * imuB : 0.0, 0.0);
+// inverse x of the G-box rows, two at a time, written to the cells' field
+template <typename C, int LOGN>
+__global__ void __launch_bounds__(128) fft_x_inverse_kernel(const C* __restrict__ in, size_t cs, int nrows, int rpp,
+                                                            int py, const C* __restrict__ tw,
+                                                            const int* __restrict__ box_cell, int gx, int nc,
+                                                            double scale, double* __restrict__ field) {
+   constexpr int N = 1 << LOGN, T = N / 8, L = xlines_of(LOGN), NP = N + N / 8, HX = N / 2 + 1;
+   __shared__ C s[L * NP];
+   pdl_begin();
+   const int j = threadIdx.x % T, line = threadIdx.x / T;
+   const int ra = 2 * (blockIdx.x * L + line), rb = ra + 1;
+   const int c = blockIdx.y;
+   const C* ia = in + (size_t)c * cs + row_start(ra, rpp, py, HX);
+   const C* ib = in + (size_t)c * cs + row_start(rb, rpp, py, HX);
+   C v[1][8];
+#pragma unroll
+   for (int i = 0; i < 8; ++i) {
+      const int k = j + i * T, m = k <= N / 2 ? k : N - k;
+      C a = ra < nrows ? ia[m] : C{0, 0}, b = rb < nrows ? ib[m] : C{0, 0};
+      if (m == 0 || m == N / 2) a.y = b.y = 0;  // real by symmetry
+      if (k > N / 2) { a.y = -a.y; b.y = -b.y; }
+      v[0][i] = {a.x - b.y, a.y + b.x};
+   }
+   fft_lines<C, LOGN, true, 0>(v, j, s, [&](int, int p) { return line * NP + p + (p >> 3); }, tw);
+#pragma unroll
+   for (int i = 0; i < 8; ++i) {
+      const int x = j + i * T;
+      if (x < gx) {
+         const int a = ra < nrows ? __ldg(box_cell + (size_t)ra * gx + x) : -1;
+         const int b = rb < nrows ? __ldg(box_cell + (size_t)rb * gx + x) : -1;
+         if (a >= 0) field[(size_t)c * nc + a] = (double)v[0][i].x * scale;
+         if (b >= 0) field[(size_t)c * nc + b] = (double)v[0][i].y * scale;
+      }
+   }
 }
 
-template <typename C>
-__global__ void gather_field_kernel(int nc, const int* __restrict__ lin, const C* __restrict__ grid, size_t np,
-                                    double scale, double* __restrict__ field) {
-   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-   if (c >= nc) return;
-   const int q = lin[c];
-   field[c] = q < 0 ? 0.0 : (double)grid[q].x * scale;
-   field[nc + c] = q < 0 ? 0.0 : (double)grid[np + q].x * scale;
-   field[2 * nc + c] = q < 0 ? 0.0 : (double)grid[2 * np + q].x * scale;
+// The middle of the convolution: for W adjacent (y, x) columns the three
+// moment components' forward z transforms (points z >= gz are zero), H(k) =
+// T(k) M(k), and the inverse transforms, of which z < gz is stored.  The three
+// spectra stay in registers (24 complex points a thread) and share the
+// barriers of the exchanges.
+template <typename C, int LOGN>
+__global__ void __launch_bounds__(threads_of(LOGN)) fft_z_kernel(C* __restrict__ data, size_t cs,
+                                                                 const typename RealOf<C>::type* __restrict__ t, int hx,
+                                                                 int py, int gz, const C* __restrict__ tw) {
+   constexpr int N = 1 << LOGN, W = lines_of(LOGN), T = N / 8;
+   using R = typename RealOf<C>::type;
+   extern __shared__ __align__(16) unsigned char fft_smem[];
+   C* s = reinterpret_cast<C*>(fft_smem);
+   pdl_begin();
+   const int w = threadIdx.x % W, j = threadIdx.x / W;
+   const int nlines = hx * py;
+   const int l = blockIdx.x * W + w;
+   const bool on = l < nlines;
+   C v[3][8];
+#pragma unroll
+   for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+         const int p = j + i * T;
+         v[c][i] = on && p < gz ? data[(size_t)c * cs + (size_t)p * nlines + l] : C{0, 0};
+      }
+   auto idx = [&](int c, int p) { return c * (W << LOGN) + p * W + w; };
+   fft_lines<C, LOGN, false, 0>(v, j, s, idx, tw);
+   {
+      const int ky = on ? l / hx : 0, kx = on ? l % hx : 0;
+      const int hy = py / 2 + 1;
+      const bool fy = ky > py / 2;  // the mirrored half: odd components change sign
+      const size_t ts = (size_t)hx * hy * (N / 2 + 1);
+      const R* row = t + (size_t)(fy ? py - ky : ky) * hx + kx;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+         const int k = j + i * T;
+         const bool fz = k > N / 2;
+         const R* q = row + (size_t)(fz ? N - k : k) * hx * hy;
+         const R xx = __ldg(q), yy = __ldg(q + 3 * ts), zz = __ldg(q + 5 * ts);
+         R xy = __ldg(q + ts), xz = __ldg(q + 2 * ts), yz = __ldg(q + 4 * ts);
+         if (fy) { xy = -xy; yz = -yz; }
+         if (fz) { xz = -xz; yz = -yz; }
+         const C mx = v[0][i], my = v[1][i], mz = v[2][i];
+         v[0][i] = {xx * mx.x + xy * my.x + xz * mz.x, xx * mx.y + xy * my.y + xz * mz.y};
+         v[1][i] = {xy * mx.x + yy * my.x + yz * mz.x, xy * mx.y + yy * my.y + yz * mz.y};
+         v[2][i] = {xz * mx.x + yz * my.x + zz * mz.x, xz * mx.y + yz * my.y + zz * mz.y};
+      }
+   }
+   fft_lines<C, LOGN, true, 0>(v, j, s, idx, tw);
+#pragma unroll
+   for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+         const int p = j + i * T;
+         if (on && p < gz) data[(size_t)c * cs + (size_t)p * nlines + l] = v[c][i];
+      }
 }
 
-// the FP64 spectra or twiddles rounded to FP32
-__global__ void round_complex_kernel(const double2* __restrict__ in, float2* __restrict__ out, size_t n) {
-   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-      out[q] = make_float2((float)in[q].x, (float)in[q].y);
+// the octant of the (real) tensor spectra from the full transforms, rounded to R
+template <typename R>
+__global__ void spectrum_octant_kernel(const double2* __restrict__ full, size_t cs, int hx, int py, int hy, int hz,
+                                       R* __restrict__ out) {
+   const size_t n = (size_t)hx * hy * hz;
+   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+      const size_t x = q % hx, y = (q / hx) % hy, z = q / ((size_t)hx * hy);
+      out[(size_t)blockIdx.y * n + q] = (R)full[(size_t)blockIdx.y * cs + (z * py + y) * hx + x].x;
+   }
 }
 
 int ilog2(int v) {
@@ -289,79 +384,118 @@ int ilog2(int v) {
    return l;
 }
 
-int grid_blocks(size_t np) { return (int)std::min<size_t>((np + 255) / 256, 148 * 16); }
-
-// forward 3-D FFT of `ncomp` consecutive grids, all lines (the tensor spectra)
-cudaError_t fft3d(FFTField* f, double2* data, int ncomp, cudaStream_t st) {
-   const int px = f->p[0], py = f->p[1], pz = f->p[2];
-   {  // x: lines of px points, kFFTTile / px lines per block
-      const int nrows = py * pz;
-      const int lines = std::max(1, std::min(kFFTTile / px, nrows));
-      dim3 grid((unsigned)((nrows + lines - 1) / lines), (unsigned)ncomp);
-      fft_x_kernel<double2><<<grid, kFFTThreads, 0, st>>>(data, f->np, px, f->logp[0], lines, f->tw[0], 0, nrows,
-                                                          py, py, px, px);
+// CALL with the constant LN = logn, for logn = 3..10 (the planner's range)
+#define VGPU_FFT_DISPATCH(logn, CALL)                                       \
+   switch (logn) {                                                          \
+      case 3: { constexpr int LN = 3; CALL; } break;                        \
+      case 4: { constexpr int LN = 4; CALL; } break;                        \
+      case 5: { constexpr int LN = 5; CALL; } break;                        \
+      case 6: { constexpr int LN = 6; CALL; } break;                        \
+      case 7: { constexpr int LN = 7; CALL; } break;                        \
+      case 8: { constexpr int LN = 8; CALL; } break;                        \
+      case 9: { constexpr int LN = 9; CALL; } break;                        \
+      case 10: { constexpr int LN = 10; CALL; } break;                      \
+      default: e = cudaErrorInvalidValue;                                   \
    }
-   {  // y: stride px, W adjacent x columns, one block per (x chunk, z)
-      const int W = std::max(1, std::min(kFFTTile / py, px));
-      dim3 grid((unsigned)(px / W), (unsigned)pz, (unsigned)ncomp);
-      fft_strided_kernel<double2><<<grid, kFFTThreads, 0, st>>>(data, f->np, py, f->logp[1], W, (size_t)px,
-                                                                (size_t)px * py, f->tw[1], 0, py, py);
-   }
-   {  // z: stride px*py, one block per (x chunk, y)
-      const int W = std::max(1, std::min(kFFTTile / pz, px));
-      dim3 grid((unsigned)(px / W), (unsigned)py, (unsigned)ncomp);
-      fft_strided_kernel<double2><<<grid, kFFTThreads, 0, st>>>(data, f->np, pz, f->logp[2], W, (size_t)px * py,
-                                                                (size_t)px, f->tw[2], 0, pz, pz);
-   }
-   return cudaGetLastError();
-}
 
-// the x and y passes of the moment transform (forward: x then y; inverse: y
-// then x), pruned to the G-box; the z passes run in fft_z_multiply_kernel
-template <typename C>
-cudaError_t fft_box(FFTField* f, C* grid_data, C* const* tw, bool inverse, cudaStream_t st, int* launches) {
-   const int px = f->p[0], py = f->p[1];
-   const int gx = f->g[0], gy = f->g[1], gz = f->g[2];
-   auto xpass = [&]() {
-      const int nrows = gy * gz;
-      const int lines = std::max(1, std::min(kFFTTile / px, nrows));
-      dim3 grid((unsigned)((nrows + lines - 1) / lines), 3u);
-      fft_x_kernel<C><<<grid, kFFTThreads, 0, st>>>(grid_data, f->np, px, f->logp[0], lines, tw[0], inverse, nrows,
-                                                    gy, py, inverse ? px : gx, inverse ? gx : px);
-   };
-   auto ypass = [&]() {
-      const int W = std::max(1, std::min(kFFTTile / py, px));
-      dim3 grid((unsigned)(px / W), (unsigned)gz, 3u);
-      fft_strided_kernel<C><<<grid, kFFTThreads, 0, st>>>(grid_data, f->np, py, f->logp[1], W, (size_t)px,
-                                                          (size_t)px * py, tw[1], inverse, inverse ? py : gy,
-                                                          inverse ? gy : py);
-   };
-   if (inverse) { ypass(); xpass(); }
-   else { xpass(); ypass(); }
-   if (launches) *launches += 2;
-   return cudaGetLastError();
-}
-
-template <typename C>
-cudaError_t field_apply(FFTField* f, C* grid, const C* tspec, C* const* tw, const double* mag, double* field,
-                        cudaStream_t st, int* launches) {
+template <typename C, typename Rows>
+cudaError_t x_forward(const Rows& rows, C* out, size_t cs, int logn, int ncomp, int nrows, int rpp, int py, const C* tw,
+                      cudaStream_t st) {
    cudaError_t e = cudaSuccess;
-   const int nc = f->nc;
-   const int nbox = f->g[0] * f->g[1] * f->g[2];
-   scatter_moments_kernel<C><<<(nbox + 255) / 256, 256, 0, st>>>(nc, f->box_cell, f->g[0], f->g[1], nbox, mag, grid,
-                                                                 f->p[0], f->p[1], f->np);
-   if ((e = fft_box<C>(f, grid, tw, false, st, launches)) != cudaSuccess) return e;
-   {
-      const int pz = f->p[2];
-      const int W = std::max(1, std::min(kFuseTile / (3 * pz), f->p[0]));
-      dim3 g((unsigned)(f->p[0] / W), (unsigned)f->p[1]);
-      fft_z_multiply_kernel<C><<<g, kFFTThreads, 0, st>>>(grid, tspec, f->np, f->p[0], f->p[1], pz, f->logp[2], W,
-                                                          f->g[2], tw[2]);
+   VGPU_FFT_DISPATCH(logn, {
+      constexpr int L = xlines_of(LN);
+      const int npairs = (nrows + 1) / 2;
+      e = launch_pdl(fft_x_forward_kernel<C, LN, Rows>, dim3((npairs + L - 1) / L, ncomp), dim3(L << (LN - 3)), 0, st,
+                     rows, out, cs, nrows, rpp, py, tw);
+   })
+   return e;
+}
+
+template <typename C, bool INV>
+cudaError_t strided(C* data, size_t cs, int logn, int ncomp, int nlines, int inner, size_t outer, size_t ps,
+                    const C* tw, int ld, int stp, cudaStream_t st) {
+   cudaError_t e = cudaSuccess;
+   VGPU_FFT_DISPATCH(logn, {
+      constexpr int W = lines_of(LN);
+      e = launch_pdl(fft_strided_kernel<C, LN, INV>, dim3((nlines + W - 1) / W, ncomp), dim3(threads_of(LN)), 0, st,
+                     data, cs, nlines, inner, outer, ps, tw, ld, stp);
+   })
+   return e;
+}
+
+template <typename C> constexpr int z_smem(int logn) { return 3 * (int)sizeof(C) * (lines_of(logn) << logn); }
+
+// the z kernel's shared memory above the default limit (FP64): asked for once per field
+template <typename C>
+cudaError_t z_prepare(int logn) {
+   cudaError_t e = cudaSuccess;
+   VGPU_FFT_DISPATCH(logn, {
+      e = cudaFuncSetAttribute(fft_z_kernel<C, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, z_smem<C>(LN));
+   })
+   return e;
+}
+
+template <typename C>
+cudaError_t field_apply(FFTField* f, const double* mag, double* field, cudaStream_t st, int* launches) {
+   using R = typename RealOf<C>::type;
+   const int px = f->p[0], py = f->p[1];
+   const int gx = f->g[0], gy = f->g[1], gz = f->g[2], hx = f->hx;
+   C* grid = static_cast<C*>(f->grid);
+   const C* tw[3] = {static_cast<const C*>(f->tw[0]), static_cast<const C*>(f->tw[1]), static_cast<const C*>(f->tw[2])};
+   const size_t cs = (size_t)gz * py * hx;
+   const size_t plane = (size_t)py * hx;
+   (void)px;
+   cudaError_t e = x_forward<C>(MomentRows{f->box_cell, mag, f->nc, gx}, grid, cs, f->logp[0], 3, gy * gz, gy, py,
+                                tw[0], st);
+   if (e == cudaSuccess) e = strided<C, false>(grid, cs, f->logp[1], 3, gz * hx, hx, plane, hx, tw[1], gy, py, st);
+   if (e == cudaSuccess) {
+      VGPU_FFT_DISPATCH(f->logp[2], {
+         constexpr int W = lines_of(LN);
+         e = launch_pdl(fft_z_kernel<C, LN>, dim3((hx * py + W - 1) / W), dim3(threads_of(LN)), z_smem<C>(LN), st,
+                        grid, cs, static_cast<const R*>(f->tspec), hx, py, gz, tw[2]);
+      })
    }
-   if ((e = fft_box<C>(f, grid, tw, true, st, launches)) != cudaSuccess) return e;
-   gather_field_kernel<C><<<(nc + 255) / 256, 256, 0, st>>>(nc, f->cell_lin, grid, f->np, 1.0 / (double)f->np, field);
-   if (launches) *launches += 3;
-   return cudaGetLastError();
+   if (e == cudaSuccess) e = strided<C, true>(grid, cs, f->logp[1], 3, gz * hx, hx, plane, hx, tw[1], py, gy, st);
+   if (e == cudaSuccess) {
+      VGPU_FFT_DISPATCH(f->logp[0], {
+         constexpr int L = xlines_of(LN);
+         const int npairs = (gy * gz + 1) / 2;
+         e = launch_pdl(fft_x_inverse_kernel<C, LN>, dim3((npairs + L - 1) / L, 3), dim3(L << (LN - 3)), 0, st,
+                        (const C*)grid, cs, gy * gz, gy, py, tw[0], (const int*)f->box_cell, gx, f->nc,
+                        1.0 / (double)f->np, field);
+      })
+   }
+   if (launches) *launches += 5;
+   return e;
+}
+
+// the tensor spectra: FP64 transforms of the six components on the whole grid,
+// then their octant in the field's precision
+template <typename C>
+cudaError_t make_spectra(FFTField* f, double size, double2* const* tw, cudaStream_t st) {
+   using R = typename RealOf<C>::type;
+   const int px = f->p[0], py = f->p[1], pz = f->p[2], hx = f->hx, hy = py / 2 + 1, hz = pz / 2 + 1;
+   const size_t cs = (size_t)pz * py * hx;
+   double2* full = nullptr;
+   cudaError_t e = cudaMalloc(&full, sizeof(double2) * 6 * cs);
+   if (e != cudaSuccess) return e;
+   e = cudaMalloc(&f->tspec, sizeof(R) * 6 * (size_t)hx * hy * hz);
+   if (e == cudaSuccess)
+      e = x_forward<double2>(TensorRows{px, py, pz, f->g[0], f->g[1], f->g[2], size}, full, cs, f->logp[0], 6, py * pz,
+                             py, py, (const double2*)tw[0], st);
+   if (e == cudaSuccess)
+      e = strided<double2, false>(full, cs, f->logp[1], 6, pz * hx, hx, (size_t)py * hx, hx, tw[1], py, py, st);
+   if (e == cudaSuccess)
+      e = strided<double2, false>(full, cs, f->logp[2], 6, py * hx, py * hx, 0, (size_t)py * hx, tw[2], pz, pz, st);
+   if (e == cudaSuccess) {
+      const size_t n = (size_t)hx * hy * hz;
+      spectrum_octant_kernel<R><<<dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 8), 6), 256, 0, st>>>(
+          full, cs, hx, py, hy, hz, static_cast<R*>(f->tspec));
+      e = cudaGetLastError();
+   }
+   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+   cudaFree(full);
+   return e;
 }
 
 }  // namespace
@@ -398,7 +532,7 @@ FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double
    size_t np = 1;
    for (int a = 0; a < 3; ++a) {
       const long long G = hi[a] - lo[a] + 1;
-      int P = 2;
+      int P = 8;  // the line transforms hold 8 points per thread
       while (P < 2 * G - 1 && P <= 1024) P <<= 1;
       if (P > 1024) {
          *why = "cell grid too large for the FFT solver";
@@ -416,81 +550,55 @@ FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double
       return nullptr;
    }
    f->np = np;
-   // linear index of each occupied cell; two cells on one grid point are not a grid
-   std::vector<int> lin(nc, -1);
-   {
-      std::vector<char> used(np, 0);
-      for (int c = 0; c < nc; ++c) {
-         if (natoms[c] <= 0) continue;
-         const size_t x = (size_t)(gi[3 * (size_t)c] - lo[0]), y = (size_t)(gi[3 * (size_t)c + 1] - lo[1]),
-                      z = (size_t)(gi[3 * (size_t)c + 2] - lo[2]);
-         const size_t q = (z * f->p[1] + y) * f->p[0] + x;
-         if (used[q]) {
-            *why = "two cells share a grid point";
-            delete f;
-            return nullptr;
-         }
-         used[q] = 1;
-         lin[c] = (int)q;
-      }
-   }
-   cudaError_t e = cudaMalloc(&f->tspec, sizeof(double2) * 6 * np);
-   if (e == cudaSuccess) e = cudaMalloc(&f->grid, sizeof(double2) * 3 * np);
-   if (e == cudaSuccess) e = cudaMalloc(&f->cell_lin, sizeof(int) * std::max(nc, 1));
-   if (e == cudaSuccess) e = cudaMemcpyAsync(f->cell_lin, lin.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st);
-   // cell at each point of the G-box
+   f->hx = f->p[0] / 2 + 1;
+   f->fp32 = fp32;
+   // cell at each point of the G-box; two cells on one grid point are not a grid
    const size_t nbox = (size_t)f->g[0] * f->g[1] * f->g[2];
    std::vector<int> boxc(nbox, -1);
    for (int c = 0; c < nc; ++c) {
-      if (lin[c] < 0) continue;
-      const size_t q = (size_t)lin[c];
-      const size_t x = q % f->p[0], y = (q / f->p[0]) % f->p[1], z = q / ((size_t)f->p[0] * f->p[1]);
-      boxc[(z * f->g[1] + y) * f->g[0] + x] = c;
+      if (natoms[c] <= 0) continue;
+      const size_t x = (size_t)(gi[3 * (size_t)c] - lo[0]), y = (size_t)(gi[3 * (size_t)c + 1] - lo[1]),
+                   z = (size_t)(gi[3 * (size_t)c + 2] - lo[2]);
+      int& at = boxc[(z * f->g[1] + y) * f->g[0] + x];
+      if (at >= 0) {
+         *why = "two cells share a grid point";
+         delete f;
+         return nullptr;
+      }
+      at = c;
    }
+   const size_t cw = fp32 ? sizeof(float2) : sizeof(double2);
+   cudaError_t e = cudaMalloc(&f->grid, cw * 3 * (size_t)f->g[2] * f->p[1] * f->hx);
    if (e == cudaSuccess) e = cudaMalloc(&f->box_cell, sizeof(int) * nbox);
    if (e == cudaSuccess) e = cudaMemcpyAsync(f->box_cell, boxc.data(), sizeof(int) * nbox, cudaMemcpyHostToDevice, st);
+   // twiddles in FP64 for the spectra, and rounded to the field's precision
    std::vector<std::vector<double2>> tw(3);
+   std::vector<std::vector<float2>> twf(3);
+   double2* tw64[3] = {nullptr, nullptr, nullptr};
    for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
       const int P = f->p[a];
-      tw[a].resize(P / 2);
-      for (int k = 0; k < P / 2; ++k) {
+      tw[a].resize(P);
+      twf[a].resize(P);
+      for (int k = 0; k < P; ++k) {
          const double ang = -2.0 * M_PI * (double)k / (double)P;
          tw[a][k] = make_double2(std::cos(ang), std::sin(ang));
+         twf[a][k] = make_float2((float)tw[a][k].x, (float)tw[a][k].y);
       }
-      e = cudaMalloc(&f->tw[a], sizeof(double2) * (P / 2));
+      e = cudaMalloc(&tw64[a], sizeof(double2) * P);
       if (e == cudaSuccess)
-         e = cudaMemcpyAsync(f->tw[a], tw[a].data(), sizeof(double2) * (P / 2), cudaMemcpyHostToDevice, st);
-   }
-   if (e == cudaSuccess) {
-      tensor_grid_kernel<<<grid_blocks(np), 256, 0, st>>>(f->tspec, np, f->p[0], f->p[1], f->p[2], f->g[0], f->g[1],
-                                                          f->g[2], size);
-      e = cudaGetLastError();
-   }
-   if (e == cudaSuccess) e = fft3d(f, f->tspec, 6, st);
-   if (e == cudaSuccess && fp32) {
-      // FP32 transforms: the spectra and twiddles rounded once; the FP64
-      // moment grid is not needed
-      f->fp32 = true;
-      e = cudaMalloc(&f->tspec32, sizeof(float2) * 6 * np);
-      if (e == cudaSuccess) e = cudaMalloc(&f->grid32, sizeof(float2) * 3 * np);
-      if (e == cudaSuccess) {
-         round_complex_kernel<<<grid_blocks(6 * np), 256, 0, st>>>(f->tspec, f->tspec32, 6 * np);
-         e = cudaGetLastError();
-      }
-      for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
-         e = cudaMalloc(&f->tw32[a], sizeof(float2) * (f->p[a] / 2));
-         if (e == cudaSuccess) {
-            round_complex_kernel<<<1, 256, 0, st>>>(f->tw[a], f->tw32[a], (size_t)(f->p[a] / 2));
-            e = cudaGetLastError();
-         }
+         e = cudaMemcpyAsync(tw64[a], tw[a].data(), sizeof(double2) * P, cudaMemcpyHostToDevice, st);
+      if (e == cudaSuccess && fp32) {
+         e = cudaMalloc(&f->tw[a], sizeof(float2) * P);
+         if (e == cudaSuccess)
+            e = cudaMemcpyAsync(f->tw[a], twf[a].data(), sizeof(float2) * P, cudaMemcpyHostToDevice, st);
       }
    }
+   if (e == cudaSuccess) e = fp32 ? make_spectra<float2>(f, size, tw64, st) : make_spectra<double2>(f, size, tw64, st);
+   if (e == cudaSuccess) e = fp32 ? z_prepare<float2>(f->logp[2]) : z_prepare<double2>(f->logp[2]);
    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // host tables above leave scope
-   if (e == cudaSuccess && f->fp32) {
-      cudaFree(f->tspec);
-      cudaFree(f->grid);
-      f->tspec = nullptr;
-      f->grid = nullptr;
+   for (int a = 0; a < 3; ++a) {
+      if (e == cudaSuccess && !fp32) f->tw[a] = tw64[a];
+      else cudaFree(tw64[a]);
    }
    if (e != cudaSuccess) {
       *err = e;
@@ -501,22 +609,16 @@ FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double
 }
 
 cudaError_t fft_field_apply(FFTField* f, const double* mag, double* field, cudaStream_t st, int* launches) {
-   if (f->fp32) return field_apply<float2>(f, f->grid32, f->tspec32, f->tw32, mag, field, st, launches);
-   return field_apply<double2>(f, f->grid, f->tspec, f->tw, mag, field, st, launches);
+   if (f->fp32) return field_apply<float2>(f, mag, field, st, launches);
+   return field_apply<double2>(f, mag, field, st, launches);
 }
 
 void fft_field_destroy(FFTField* f) {
    if (!f) return;
    cudaFree(f->tspec);
    cudaFree(f->grid);
-   cudaFree(f->cell_lin);
    cudaFree(f->box_cell);
-   cudaFree(f->tspec32);
-   cudaFree(f->grid32);
-   for (int a = 0; a < 3; ++a) {
-      cudaFree(f->tw[a]);
-      cudaFree(f->tw32[a]);
-   }
+   for (int a = 0; a < 3; ++a) cudaFree(f->tw[a]);
    delete f;
 }
 

@@ -19,7 +19,7 @@ FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double
 
 // field[q * nc + c] = sum over occupied j != c of the bare point-dipole
 // tensor (3 e e - 1)/r^3 (r in Angstrom) times m_j in mu_B, for q = x, y, z;
-// mag is [3][nc] in J/T.  Empty cells get 0.
+// mag is [3][nc] in J/T.  Empty cells are left as they are.
 cudaError_t fft_field_apply(FFTField* f, const double* mag, double* field, cudaStream_t st, int* launches);
 
 void fft_field_destroy(FFTField* f);

@@ -81,6 +81,7 @@ __global__ void batch_persistent_kernel(LLGArgs<R> a, const int* __restrict__ gr
    const int q0 = grp_start[g], q1 = grp_start[g + 1];
    for (int s = 0; s < nsteps; ++s) {
       a.step = step0 + (uint64_t)s;
+      set_ramp(a);
       for (int q = q0; q < q1; ++q) {
          const int k = grp_sys[q];
          for (int i = off[k] + t; i < off[k + 1]; i += stride) llg_predict_atom<R, FMT, 1, VAR_HEUN>(a, i);

@@ -420,6 +420,13 @@ static int dipole_update_typed(vgpu_ctx* h) {
    return dipole_field_typed<R>(h, false);
 }
 
+uint64_t dipole_steps_left(vgpu_ctx* h) {
+   DipoleState* d = dip_of(h);
+   if (!d || d->update_rate <= 0) return UINT64_MAX;
+   const uint64_t rate = (uint64_t)d->update_rate;
+   return rate - h->step % rate;
+}
+
 int dipole_update(vgpu_ctx* h) {
    return h->prec == VGPU_PREC_FP64 ? dipole_update_typed<double>(h) : dipole_update_typed<float>(h);
 }

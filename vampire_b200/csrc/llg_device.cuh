@@ -13,6 +13,9 @@ template <typename R> __device__ __forceinline__ R rsqrt_(R x);
 template <> __device__ __forceinline__ float rsqrt_<float>(float x) { return rsqrtf(x); }
 template <> __device__ __forceinline__ double rsqrt_<double>(double x) { return 1.0 / sqrt(x); }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <typename R>
 __device__ __forceinline__ void thermal_xi(const LLGArgs<R>& a, int i, R& gx, R& gy, R& gz) {
    if (a.noise_mode == VGPU_NOISE_REPLAY) {
@@ -382,19 +385,14 @@ __device__ __forceinline__ void exchange_field(const LLGArgs<R>& a, int i, int m
    exchange_gather<R, FMT, LOAD>(a, i, mi, sx, sy, sz, hx, hy, hz);
 }
 
-// spin-dependent field of atom i at spin S: exchange + anisotropy
+// spin-dependent field of atom i at spin S given its bilinear exchange field
+// (hx, hy, hz): biquadratic exchange and anisotropy added
 // (calculate_spin_fields, src/simulate/fields.cpp:67-118)
 // EXT = false compiles the passes without the higher-order anisotropy terms
 // (register budget of the common case); launchers pick EXT from a.aniso_ext.
-template <typename R, int FMT, int LOAD = 0, bool STAGED = false, bool EXT = true, int REC = REC_ANY>
-__device__ __forceinline__ void spin_field(const LLGArgs<R>& a, int i, int mi, const MatParams<R>& m,
-                                           const R* sx, const R* sy, const R* sz, const R S[3], R H[3],
-                                           const int4* srec_tile = nullptr, int tile_off = 0,
-                                           const float4* sdict = nullptr, const float* swin = nullptr,
-                                           int wmax = 0) {
-   R hx = 0, hy = 0, hz = 0;
-   exchange_field<R, FMT, LOAD, STAGED, REC>(a, i, mi, sx, sy, sz, hx, hy, hz, srec_tile, tile_off, sdict, swin,
-                                             wmax);
+template <typename R, int LOAD, bool EXT>
+__device__ __forceinline__ void site_field(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R* sx, const R* sy,
+                                           const R* sz, const R S[3], R hx, R hy, R hz, R H[3]) {
    if (EXT && a.bq_off) {
       // biquadratic exchange (exchange/biquadratic_fields.cpp): its own sum,
       // added to the bilinear field as exchange::fields does
@@ -458,6 +456,19 @@ __device__ __forceinline__ void spin_field(const LLGArgs<R>& a, int i, int mi, c
       }
    }
    H[0] = hx; H[1] = hy; H[2] = hz;
+}
+
+// spin-dependent field of atom i at spin S: exchange + anisotropy
+template <typename R, int FMT, int LOAD = 0, bool STAGED = false, bool EXT = true, int REC = REC_ANY>
+__device__ __forceinline__ void spin_field(const LLGArgs<R>& a, int i, int mi, const MatParams<R>& m,
+                                           const R* sx, const R* sy, const R* sz, const R S[3], R H[3],
+                                           const int4* srec_tile = nullptr, int tile_off = 0,
+                                           const float4* sdict = nullptr, const float* swin = nullptr,
+                                           int wmax = 0) {
+   R hx = 0, hy = 0, hz = 0;
+   exchange_field<R, FMT, LOAD, STAGED, REC>(a, i, mi, sx, sy, sz, hx, hy, hz, srec_tile, tile_off, sdict, swin,
+                                             wmax);
+   site_field<R, LOAD, EXT>(a, i, m, sx, sy, sz, S, hx, hy, hz, H);
 }
 
 // anisotropy energy of atom i at spin S in the order of
@@ -531,9 +542,11 @@ template <typename R>
 __device__ __forceinline__ void external_field_g(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R g[3],
                                                  int cell_id, R E[3]) {
    R ex = 0, ey = 0, ez = 0;
-   if (a.thermal) { ex = g[0] * m.sigma; ey = g[1] * m.sigma; ez = g[2] * m.sigma; }
+   // products rounded by themselves, so that kernels compiled for a fixed set of
+   // terms give the generic kernels' fields (no fused add of the applied field)
+   if (a.thermal) { ex = mul_rn(g[0], m.sigma); ey = mul_rn(g[1], m.sigma); ez = mul_rn(g[2], m.sigma); }
    if (a.ramp_n) {
-      const R f = (R)(a.step < a.ramp_n ? a.step : a.ramp_n) / (R)a.ramp_n;
+      const R f = a.ramp_f;
       ex += a.hx + (m.hlx + m.dhx * f); ey += a.hy + (m.hly + m.dhy * f); ez += a.hz + (m.hlz + m.dhz * f);
    } else if (a.local_field) { ex += a.hx + m.hlx; ey += a.hy + m.hly; ez += a.hz + m.hlz; }
    else { ex += a.hx; ey += a.hy; ez += a.hz; }

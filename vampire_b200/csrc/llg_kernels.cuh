@@ -26,23 +26,32 @@
 namespace vgpu {
 
 // Predictor tail of atom i, given s0 and its total field H:
-// s' = n(s0 + dt f(s0, H)) (LLGHeun.cpp:195-222).
+// s' = n(s0 + dt f(s0, H)) (LLGHeun.cpp:195-222).  The step tails return the
+// state that they compute; llg_*_finish store it.
 template <typename R>
-__device__ __forceinline__ void llg_predict_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
-                                                   const R H[3]) {
+__device__ __forceinline__ void llg_predict(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                            const R H[3], R out[3]) {
    R d[3];
    llg_rhs<R>(m.A, m.B, S0, H, d);
    if (a.ex) { a.ex[i] = d[0]; a.ey[i] = d[1]; a.ez[i] = d[2]; }
    R Sn[3] = {S0[0] + d[0] * a.dt, S0[1] + d[1] * a.dt, S0[2] + d[2] * a.dt};
    const R r = rsqrt_<R>(Sn[0] * Sn[0] + Sn[1] * Sn[1] + Sn[2] * Sn[2]);
-   a.bx[i] = Sn[0] * r; a.by[i] = Sn[1] * r; a.bz[i] = Sn[2] * r;
+   out[0] = Sn[0] * r; out[1] = Sn[1] * r; out[2] = Sn[2] * r;
+}
+
+template <typename R>
+__device__ __forceinline__ void llg_predict_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                                   const R H[3]) {
+   R o[3];
+   llg_predict<R>(a, i, m, S0, H, o);
+   a.bx[i] = o[0]; a.by[i] = o[1]; a.bz[i] = o[2];
 }
 
 // Corrector tail of atom i, given s0, s' and the total field H' of s':
 // s1 = n(s0 + dt/2 (f0 + f(s', H'))) (LLGHeun.cpp:238-279), written over s0.
 template <typename R>
-__device__ __forceinline__ void llg_correct_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
-                                                   const R S1[3], const R H[3]) {
+__device__ __forceinline__ void llg_correct(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                            const R S1[3], const R H[3], R out[3]) {
    R d[3];
    llg_rhs<R>(m.A, m.B, S1, H, d);
    R Sn[3];
@@ -64,7 +73,15 @@ __device__ __forceinline__ void llg_correct_finish(const LLGArgs<R>& a, int i, c
    const R n2 = Sn[0] * Sn[0] + Sn[1] * Sn[1] + Sn[2] * Sn[2];
    const R r = rsqrt_<R>(n2);
    if (!(n2 > (R)0.25 && n2 < (R)4)) atomicOr(a.status, 1);  // non-finite or runaway
-   a.ax[i] = Sn[0] * r; a.ay[i] = Sn[1] * r; a.az[i] = Sn[2] * r;
+   out[0] = Sn[0] * r; out[1] = Sn[1] * r; out[2] = Sn[2] * r;
+}
+
+template <typename R>
+__device__ __forceinline__ void llg_correct_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                                   const R S1[3], const R H[3]) {
+   R o[3];
+   llg_correct<R>(a, i, m, S0, S1, H, o);
+   a.ax[i] = o[0]; a.ay[i] = o[1]; a.az[i] = o[2];
 }
 
 // Cayley-transform rotation of sim::LLG_Midpoint (src/simulate/LLGMidpoint.cpp:
@@ -87,24 +104,162 @@ __device__ __forceinline__ void midpoint_rotate(R alpha, R beta, const R M[3], c
 
 // midpoint first half: M = (S0 + R(S0; F(S0, H))) / 2, not renormalised
 template <typename R>
-__device__ __forceinline__ void mid_predict_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
-                                                   const R H[3]) {
+__device__ __forceinline__ void mid_predict(const MatParams<R>& m, const R S0[3], const R H[3], R out[3]) {
    R r[3];
    midpoint_rotate<R>(m.alpha, m.beta_mid, S0, S0, H, r);
-   a.bx[i] = (S0[0] + r[0]) * (R)0.5;
-   a.by[i] = (S0[1] + r[1]) * (R)0.5;
-   a.bz[i] = (S0[2] + r[2]) * (R)0.5;
+   out[0] = (S0[0] + r[0]) * (R)0.5;
+   out[1] = (S0[1] + r[1]) * (R)0.5;
+   out[2] = (S0[2] + r[2]) * (R)0.5;
 }
 
 // midpoint second half: S1 = R(S0; F(M, H(M))), written over S0
 template <typename R>
-__device__ __forceinline__ void mid_correct_finish(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
-                                                   const R M[3], const R H[3]) {
-   R r[3];
-   midpoint_rotate<R>(m.alpha, m.beta_mid, M, S0, H, r);
-   const R n2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+__device__ __forceinline__ void mid_correct(const LLGArgs<R>& a, const MatParams<R>& m, const R S0[3], const R M[3],
+                                            const R H[3], R out[3]) {
+   midpoint_rotate<R>(m.alpha, m.beta_mid, M, S0, H, out);
+   const R n2 = out[0] * out[0] + out[1] * out[1] + out[2] * out[2];
    if (!(n2 > (R)0.25 && n2 < (R)4)) atomicOr(a.status, 1);  // non-finite or runaway
-   a.ax[i] = r[0]; a.ay[i] = r[1]; a.az[i] = r[2];
+}
+
+// the half-steps of a pass variant
+template <typename R, int VAR>
+__device__ __forceinline__ void first_half(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                           const R H[3], R out[3]) {
+   if (VAR == VAR_MIDPOINT) mid_predict<R>(m, S0, H, out);
+   else llg_predict<R>(a, i, m, S0, H, out);
+}
+template <typename R, int VAR>
+__device__ __forceinline__ void second_half(const LLGArgs<R>& a, int i, const MatParams<R>& m, const R S0[3],
+                                            const R S1[3], const R H[3], R out[3]) {
+   if (VAR == VAR_MIDPOINT) mid_correct<R>(a, m, S0, S1, H, out);
+   else llg_correct<R>(a, i, m, S0, S1, H, out);
+}
+
+// Facts of a launch that the kernels for isotropic bonds are compiled for.
+// ISO_FIXED: the common case -- the Heun step, one coupling per atom (one
+// material per system), Philox noise, second-order uniaxial anisotropy at most,
+// no host dipole field, no field per material -- with the thermal term, a batch
+// (field ramp, temperature and noise stream per system) and the macrocell field
+// given by the other bits.  The branches on those facts and the parameter loads
+// behind them are gone: the resident step went from 741 to 374 warp
+// instructions per 32 atoms with them and the bond addresses in registers.
+constexpr int kIsoBlock = 256;
+enum IsoFeat : int { ISO_FIXED = 1, ISO_THERMAL = 2, ISO_BATCH = 4, ISO_CELL = 8 };
+#define VGPU_ISO_FEATURES(F) F(1) F(3) F(5) F(7) F(9) F(11)
+
+// the bits that hold for a (0 when a is not the ISO_FIXED case)
+template <typename R> inline int iso_features(const LLGArgs<R>& a, int fmt, int var) {
+   const bool batch = a.sys_off != nullptr;
+   const bool one_j = a.M == 1 || (batch && a.m_per_sys == 1);
+   if (fmt != FMT_ISO_TAB || var != VAR_HEUN || !one_j || a.hd_atom || a.cubic || a.aniso_ext || a.bq_off ||
+       a.noise_mode != VGPU_NOISE_PHILOX || (sizeof(R) == 4 && a.ex) || (batch && a.cell))
+      return 0;
+   if (!batch && (a.ramp_n || a.local_field)) return 0;
+   return ISO_FIXED | (a.thermal ? ISO_THERMAL : 0) | (batch ? ISO_BATCH : 0) | (a.cell ? ISO_CELL : 0);
+}
+
+// a with the facts of RF written in (equal to what a holds whenever
+// iso_features names RF)
+template <typename R, int RF> __device__ __forceinline__ LLGArgs<R> fold_iso(const LLGArgs<R>& in) {
+   LLGArgs<R> a = in;
+   if (RF & ISO_FIXED) {
+      a.hd_atom = nullptr;
+      a.cubic = 0;
+      a.aniso_ext = 0;
+      a.bq_off = nullptr;
+      a.noise_mode = VGPU_NOISE_PHILOX;
+      a.integrator = INTEG_HEUN;
+      a.thermal = (RF & ISO_THERMAL) ? 1 : 0;
+      if (sizeof(R) == 4) a.ex = a.ey = a.ez = nullptr;
+      if (!(RF & ISO_CELL)) a.cell = nullptr;
+      if (RF & ISO_BATCH) a.m_per_sys = 1;
+      if (!(RF & ISO_BATCH)) {
+         a.sys_off = nullptr;
+         a.ramp_n = 0;
+         a.local_field = 0;
+         a.mat = nullptr;
+      }
+   }
+   return a;
+}
+
+// The bonds of one atom, as the upload left them (read before pdl_begin), and
+// its exchange field over isotropic bonds of one coupling J.  Rows of six keep
+// their words in registers and have every neighbour's load in flight.  Same
+// products in the same order as exchange_gather_w and exchange_gather_row.
+struct IsoRow {
+   int base, w, j[6];
+};
+
+template <typename R> __device__ __forceinline__ IsoRow iso_row(const LLGArgs<R>& a, int i) {
+   IsoRow r;
+   const int off = __ldg(a.slice_off + (i >> 5));
+   r.w = (__ldg(a.slice_off + (i >> 5) + 1) - off) >> 5;
+   r.base = off + (i & 31);
+#pragma unroll
+   for (int k = 0; k < 6; ++k) r.j[k] = r.w == 6 ? __ldg(a.col + r.base + 32 * k) & a.idx_mask : 0;
+   return r;
+}
+
+template <typename R>
+__device__ __forceinline__ void iso_field(const LLGArgs<R>& a, const IsoRow& r, R J, const R* __restrict__ sx,
+                                          const R* __restrict__ sy, const R* __restrict__ sz, R& hx, R& hy, R& hz) {
+   auto add = [&](R x, R y, R z) { hx += J * x; hy += J * y; hz += J * z; };
+   if (r.w == 6) {
+      R x[6], y[6], z[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) { x[k] = __ldg(sx + r.j[k]); y[k] = __ldg(sy + r.j[k]); z[k] = __ldg(sz + r.j[k]); }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) add(x[k], y[k], z[k]);
+   } else {
+#pragma unroll 4
+      for (int k = 0; k < r.w; ++k) {
+         const int j = __ldg(a.col + r.base + 32 * k) & a.idx_mask;
+         add(__ldg(sx + j), __ldg(sy + j), __ldg(sz + j));
+      }
+   }
+}
+
+// One pass over isotropic bonds with the facts of RF (launch_fmt).  With a.gx
+// the predictor keeps the step's external field for the corrector, which then
+// neither draws the noise again nor recomputes the field (nothing it depends on
+// changes between the two passes of a step).
+template <typename R, int MODE, int RF>
+__global__ void __launch_bounds__(kIsoBlock) llg_iso_pass_kernel(const LLGArgs<R> in) {
+   const LLGArgs<R> a = fold_iso<R, RF>(in);
+   const int i = 32 * a.slice_first + blockIdx.x * blockDim.x + threadIdx.x;
+   const bool on = i < a.n_upd;
+   IsoRow r;
+   int mi = 0;
+   if (on) {
+      r = iso_row<R>(a, i);
+      mi = a.mat ? __ldg(a.mat + i) : 0;
+   }
+   pdl_begin();
+   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+   if (!on) return;
+   const MatParams<R>& m = a.mp[mi];
+   const R J = __ldg(a.jtab + mi * a.M + mi);
+   const R S0[3] = {a.ax[i], a.ay[i], a.az[i]};
+   R E[3], H[3], hx = 0, hy = 0, hz = 0, o[3];
+   if (MODE == PASS_PREDICTOR) {
+      iso_field<R>(a, r, J, a.ax, a.ay, a.az, hx, hy, hz);
+      external_field<R>(a, i, m, true, E);
+      if (a.gx) { a.gx[i] = E[0]; a.gy[i] = E[1]; a.gz[i] = E[2]; }
+      site_field<R, 0, false>(a, i, m, a.ax, a.ay, a.az, S0, hx, hy, hz, H);
+      H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
+      llg_predict<R>(a, i, m, S0, H, o);
+      a.bx[i] = o[0]; a.by[i] = o[1]; a.bz[i] = o[2];
+   } else {
+      const R S1[3] = {a.bx[i], a.by[i], a.bz[i]};
+      if (a.gx) { E[0] = a.gx[i]; E[1] = a.gy[i]; E[2] = a.gz[i]; }
+      iso_field<R>(a, r, J, a.bx, a.by, a.bz, hx, hy, hz);
+      if (!a.gx) external_field<R>(a, i, m, true, E);
+      site_field<R, 0, false>(a, i, m, a.bx, a.by, a.bz, S1, hx, hy, hz, H);
+      H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
+      llg_correct<R>(a, i, m, S0, S1, H, o);
+      a.ax[i] = o[0]; a.ay[i] = o[1]; a.az[i] = o[2];
+   }
 }
 
 // Predictor of atom i: s' = n(s0 + dt f(s0, H)) (Heun) or the midpoint M.
@@ -118,9 +273,11 @@ __device__ __forceinline__ void llg_predict_atom(const LLGArgs<R>& a, int i) {
    R H[3], E[3];
    spin_field<R, FMT, LOAD, false, VAR != VAR_HEUN>(a, i, mi, m, a.ax, a.ay, a.az, S0, H);
    external_field<R>(a, i, m, true, E);
+   if (a.gx) { a.gx[i] = E[0]; a.gy[i] = E[1]; a.gz[i] = E[2]; }  // kept for the corrector
    H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
-   if (VAR == VAR_MIDPOINT) mid_predict_finish<R>(a, i, m, S0, H);
-   else llg_predict_finish<R>(a, i, m, S0, H);
+   R o[3];
+   first_half<R, VAR>(a, i, m, S0, H, o);
+   a.bx[i] = o[0]; a.by[i] = o[1]; a.bz[i] = o[2];
 }
 
 // Corrector of atom i: s1 = n(s0 + dt/2 (f0 + f(s', H'))) (Heun) or the
@@ -132,11 +289,13 @@ __device__ __forceinline__ void llg_correct_atom(const LLGArgs<R>& a, int i) {
    const R S0[3] = {a.ax[i], a.ay[i], a.az[i]};
    const R S1[3] = {a.bx[i], a.by[i], a.bz[i]};
    R H[3], E[3];
+   if (a.gx) { E[0] = a.gx[i]; E[1] = a.gy[i]; E[2] = a.gz[i]; }
    spin_field<R, FMT, LOAD, false, VAR != VAR_HEUN>(a, i, mi, m, a.bx, a.by, a.bz, S1, H);
-   external_field<R>(a, i, m, true, E);
+   if (!a.gx) external_field<R>(a, i, m, true, E);
    H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
-   if (VAR == VAR_MIDPOINT) mid_correct_finish<R>(a, i, m, S0, S1, H);
-   else llg_correct_finish<R>(a, i, m, S0, S1, H);
+   R o[3];
+   second_half<R, VAR>(a, i, m, S0, S1, H, o);
+   a.ax[i] = o[0]; a.ay[i] = o[1]; a.az[i] = o[2];
 }
 
 template <typename R, int FMT, int MODE, int VAR>
@@ -175,6 +334,18 @@ inline cudaError_t launch_fmt(const LLGArgs<R>& a, int mode, cudaStream_t st) {
    const int bs = 256;
    const int grid = ((mode == PASS_FIELD ? a.n : a.n_upd - 32 * a.slice_first) + bs - 1) / bs;
    if (grid <= 0) return cudaSuccess;
+   if constexpr (FMT == FMT_ISO_TAB) {
+      const int var = a.integrator == INTEG_MIDPOINT ? VAR_MIDPOINT : VAR_HEUN;
+      switch (mode == PASS_FIELD ? 0 : iso_features<R>(a, FMT, var)) {
+#define VGPU_F(k)                                                                                             \
+   case k:                                                                                                    \
+      return launch_pdl(mode == PASS_PREDICTOR ? llg_iso_pass_kernel<R, PASS_PREDICTOR, k>                    \
+                                               : llg_iso_pass_kernel<R, PASS_CORRECTOR, k>,                   \
+                        dim3((a.n_upd - 32 * a.slice_first + kIsoBlock - 1) / kIsoBlock), dim3(kIsoBlock), 0, st, a);
+         VGPU_ISO_FEATURES(VGPU_F)
+#undef VGPU_F
+      }
+   }
    if (a.integrator == INTEG_MIDPOINT && mode != PASS_FIELD) return launch_mode<R, FMT, VAR_MIDPOINT>(a, mode, grid, bs, st);
    if (a.aniso_ext || a.bq_off) return launch_mode<R, FMT, VAR_HEUN_EXT>(a, mode, grid, bs, st);
    return launch_mode<R, FMT, VAR_HEUN>(a, mode, grid, bs, st);

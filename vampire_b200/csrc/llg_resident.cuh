@@ -1,0 +1,872 @@
+// Many LLG steps in one launch, for systems whose atoms fit the resident
+// threads of the GPU.
+//
+// A step is two dependent passes over the atoms.  As two launches each pass of
+// a small system costs what its launch costs the host, about 3 us, whatever its
+// size below some 50,000 atoms; above that every launch starts its loads cold
+// and draws the thermal noise again.  Here one cooperative launch runs all
+// steps: a thread owns K atoms, whose spins, predictor state and external field
+// stay in its registers and whose bond words stay in shared memory; only the
+// neighbours' spins travel.
+//
+// They travel with their time: a spin is stored as one 16-byte word {x, y, z,
+// half-step} (FP64: two words, the half-step in both), written and read whole,
+// and a reader that finds an older half-step reads again.  No barrier, no
+// flag and no fence is needed, so a half-step costs one store and one load
+// through L2 and its arithmetic.  (With a flag per block behind
+// release/acquire fences a half-step took 2.9 us, no better than a launch.)
+// Microseconds a step of a long launch, simple cubic, 300 K: 2.15 at 8,000 and
+// 1.98 at 32,768 atoms (5.0 in two launches), FP64 2.95 and 3.08; 151,951 atoms
+// 5.5 (11.0), where the issue of about 560 instructions per 32 atoms is the
+// bound; a 37,044-atom FCC alloy with DMI 5.0 (8.6).
+//
+// The two states keep apart what a reader may still need: an atom overwrites
+// its spin of the last step only after reading every neighbour's predictor
+// state, which those neighbours formed after reading that spin; and its
+// predictor state only after reading every neighbour's new spin.  That needs
+// neighbours to be mutual (res_mutual_kernel checks it at upload; a system with
+// one-sided bonds runs pass by pass).
+//
+// The thermal noise of the next step needs no neighbour and is drawn while the
+// stores travel.  Waits are bounded (1 s): a warp that gives up sets status bit
+// 2 (VGPU_ERR_TIMEOUT on the host) and leaves, and the others then give up too.
+// Half-steps are numbered through from launch to launch, so what an earlier
+// launch left is never taken for the present.
+//
+// The arithmetic is that of the passes (the same functions in the same order),
+// so the states are the same bit for bit.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "llg_kernels.cuh"
+
+namespace vgpu {
+
+constexpr int kResBlock = kResidentBlock;       // small blocks: a small system spreads over more SMs
+constexpr int kResSlices = kResBlock / 32;
+constexpr uint64_t kResWaitNs = 1000000000ull;  // 1 s
+constexpr int kResMaxMat = 32;                  // material rows kept in shared memory
+
+__device__ __forceinline__ uint64_t res_now() {
+   uint64_t t;
+   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+   return t;
+}
+
+// 16-byte words that are written and read whole (one access, so a reader sees
+// a value and its half-step together)
+__device__ __forceinline__ void res_store(void* p, uint64_t lo, uint64_t hi) {
+   asm volatile("{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p), "l"(lo),
+                "l"(hi)
+                : "memory");
+}
+__device__ __forceinline__ void res_load(const void* p, uint64_t& lo, uint64_t& hi) {
+   asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
+                : "=l"(lo), "=l"(hi)
+                : "l"(p)
+                : "memory");
+}
+
+// the spin of one atom and its half-step: FP32 one word {x, y, z, t}, FP64 two
+// words {x, low y, t}, {high y, z, t} (32-bit parts), `plane` bytes apart; p: the
+// atom's byte offset
+template <typename R> struct ResSpin;
+template <> struct ResSpin<float> {
+   static constexpr int kWords = 1;
+   uint64_t lo, hi;
+   __device__ __forceinline__ void load(const char* X, uint32_t, uint32_t p) { res_load(X + p, lo, hi); }
+   __device__ __forceinline__ uint32_t late(uint32_t t) const { return (uint32_t)(hi >> 32) ^ t; }
+   __device__ __forceinline__ float x() const { return __uint_as_float((uint32_t)lo); }
+   __device__ __forceinline__ float y() const { return __uint_as_float((uint32_t)(lo >> 32)); }
+   __device__ __forceinline__ float z() const { return __uint_as_float((uint32_t)hi); }
+   static __device__ __forceinline__ void store(char* X, uint32_t, uint32_t p, const float S[3], uint32_t t) {
+      res_store(X + p, (uint64_t)__float_as_uint(S[0]) | ((uint64_t)__float_as_uint(S[1]) << 32),
+                (uint64_t)__float_as_uint(S[2]) | ((uint64_t)t << 32));
+   }
+};
+template <> struct ResSpin<double> {
+   static constexpr int kWords = 2;
+   uint64_t a0, a1, b0, b1;
+   __device__ __forceinline__ void load(const char* X, uint32_t plane, uint32_t p) {
+      res_load(X + p, a0, a1);
+      res_load(X + plane + p, b0, b1);
+   }
+   __device__ __forceinline__ uint32_t late(uint32_t t) const {
+      return ((uint32_t)(a1 >> 32) ^ t) | ((uint32_t)(b1 >> 32) ^ t);
+   }
+   __device__ __forceinline__ double x() const { return __longlong_as_double((long long)a0); }
+   __device__ __forceinline__ double y() const { return __hiloint2double((int)(uint32_t)b1, (int)(uint32_t)a1); }
+   __device__ __forceinline__ double z() const { return __longlong_as_double((long long)b0); }
+   static __device__ __forceinline__ void store(char* X, uint32_t plane, uint32_t p, const double S[3], uint32_t t) {
+      const uint64_t y = (uint64_t)__double_as_longlong(S[1]), tt = (uint64_t)t << 32;
+      res_store(X + p, (uint64_t)__double_as_longlong(S[0]), (y & 0xffffffffull) | tt);
+      res_store(X + plane + p, (uint64_t)__double_as_longlong(S[2]), (y >> 32) | tt);
+   }
+};
+
+// The spins at byte offsets p[0..W-1] at half-step t, all their loads in flight;
+// while one of a warp's is late, all are read again.  All lanes of a warp call
+// together; false in every lane when one of them waited beyond the limit.
+template <typename R, int W>
+__device__ __forceinline__ bool res_read(const char* X, uint32_t plane, const uint32_t p[W], uint32_t t,
+                                         ResSpin<R> s[W]) {
+   uint32_t late = 0;
+#pragma unroll
+   for (int k = 0; k < W; ++k) s[k].load(X, plane, p[k]);
+#pragma unroll
+   for (int k = 0; k < W; ++k) late |= s[k].late(t);
+   if (!__any_sync(0xffffffffu, late != 0)) return true;
+   const uint64_t t0 = res_now();
+   for (int polls = 1;; ++polls) {
+      late = 0;
+#pragma unroll
+      for (int k = 0; k < W; ++k) s[k].load(X, plane, p[k]);
+#pragma unroll
+      for (int k = 0; k < W; ++k) late |= s[k].late(t);
+      if (!__any_sync(0xffffffffu, late != 0)) return true;
+      if ((polls & 255) == 0 && __any_sync(0xffffffffu, res_now() - t0 > kResWaitNs)) return false;
+   }
+}
+
+// bond words of a format kept in shared memory: neighbour | material bits
+// (FMT_ISO_TAB), neighbour | coupling index (FP32 FMT_DMI_TAB compact records)
+template <typename R, int FMT> constexpr bool res_words() {
+   return FMT == FMT_ISO_TAB || (FMT == FMT_DMI_TAB && sizeof(R) == 4);
+}
+
+// what one atom's gather needs besides the spins
+template <typename R> struct ResRow {
+   int base, w;          // SELL entry of the first bond, bonds
+   const uint32_t* w0;   // words in shared memory (res_words formats), stride 32
+   int mi;
+   bool one_j;           // one coupling for every bond of the atom: j0
+   R j0;
+   const float4* dict;
+};
+
+// coupling index or material of a bond word
+template <typename R, int FMT> __device__ __forceinline__ uint32_t res_coupling(const LLGArgs<R>& a, uint32_t c) {
+   if (FMT == FMT_DMI_TAB && sizeof(R) == 4) return c >> a.crec_shift;
+   return a.mat_shift ? c >> a.mat_shift : 0u;
+}
+
+// one bond of the exchange field, as in exchange_gather and its fixed-width and
+// compact-record forms
+// (q: coupling index of compact records, else the neighbour's material)
+template <typename R, int FMT>
+__device__ __forceinline__ void res_bond(const LLGArgs<R>& a, const ResRow<R>& r, int k, uint32_t q, R x, R y, R z,
+                                         R& hx, R& hy, R& hz) {
+   const int e = r.base + 32 * k;
+   if constexpr (FMT == FMT_DMI_TAB && sizeof(R) == 4) {
+      const float4 d = r.dict[q];
+      if (a.tab_scalar) {
+         dmi_bond<R>((R)d.x, (R)d.x, (R)d.x, (R)d.y, (R)d.z, (R)d.w, x, y, z, hx, hy, hz);
+      } else {
+         const float4 d2 = r.dict[a.cdict_n + q];
+         dmi_bond<R>((R)d.x, (R)d2.x, (R)d2.y, (R)d.y, (R)d.z, (R)d.w, x, y, z, hx, hy, hz);
+      }
+   } else if constexpr (FMT == FMT_ISO_TAB) {
+      const R J = r.one_j ? r.j0 : __ldg(a.jtab + r.mi * a.M + (int)q);
+      hx += J * x; hy += J * y; hz += J * z;
+   } else if constexpr (FMT == FMT_ISO_BOND) {
+      const R J = __ldg(a.jb[0] + e);
+      hx += J * x; hy += J * y; hz += J * z;
+   } else if constexpr (FMT == FMT_VEC_TAB || FMT == FMT_DMI_TAB) {
+      const R* t = a.jtab + 3 * (r.mi * a.M + (int)q);
+      if constexpr (FMT == FMT_VEC_TAB) {
+         hx += __ldg(t) * x; hy += __ldg(t + 1) * y; hz += __ldg(t + 2) * z;
+      } else {
+         const R dx = __ldg(a.jb[0] + e), dy = __ldg(a.jb[1] + e), dz = __ldg(a.jb[2] + e);
+         dmi_bond<R>(__ldg(t), __ldg(t + 1), __ldg(t + 2), dx, dy, dz, x, y, z, hx, hy, hz);
+      }
+   } else if constexpr (FMT == FMT_VEC_BOND) {
+      hx += __ldg(a.jb[0] + e) * x; hy += __ldg(a.jb[1] + e) * y; hz += __ldg(a.jb[2] + e) * z;
+   } else {
+      const R t0 = __ldg(a.jb[0] + e), t1 = __ldg(a.jb[1] + e), t2 = __ldg(a.jb[2] + e);
+      const R t3 = __ldg(a.jb[3] + e), t4 = __ldg(a.jb[4] + e), t5 = __ldg(a.jb[5] + e);
+      const R t6 = __ldg(a.jb[6] + e), t7 = __ldg(a.jb[7] + e), t8 = __ldg(a.jb[8] + e);
+      hx += (t0 * x + t1 * y + t2 * z);
+      hy += (t3 * x + t4 * y + t5 * z);
+      hz += (t6 * x + t7 * y + t8 * z);
+   }
+}
+
+// Exchange field of one atom at half-step t, W bonds at a time with all their
+// loads in flight.  The row width is the same for all lanes of a warp (a slice);
+// padded bonds read the atom's own spin (self, always in time) and add nothing.
+template <typename R, int FMT, int W>
+__device__ __forceinline__ bool res_gather(const LLGArgs<R>& a, const ResRow<R>& r, const char* X, uint32_t plane,
+                                           uint32_t self, uint32_t t, R& hx, R& hy, R& hz) {
+   constexpr bool COMPACT = FMT == FMT_DMI_TAB && sizeof(R) == 4;
+   const uint32_t mask = COMPACT ? (1u << a.crec_shift) - 1u : (uint32_t)a.idx_mask;
+   for (int k0 = 0; k0 < r.w; k0 += W) {
+      uint32_t c[W], p[W];
+      unsigned real = 0;
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+         c[k] = 0;
+         p[k] = self;
+         if (k0 + k < r.w) {  // the same for the whole warp
+            if constexpr (res_words<R, FMT>()) c[k] = r.w0[32 * (k0 + k)];
+            else c[k] = (uint32_t)__ldg(a.col + r.base + 32 * (k0 + k));
+            const uint32_t j = c[k] & mask;
+            if (j < (uint32_t)a.n) {
+               real |= 1u << k;
+               p[k] = 16u * j;
+            }
+         }
+      }
+      ResSpin<R> s[W];
+      if (!res_read<R, W>(X, plane, p, t, s)) return false;
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+         if ((real >> k) & 1u)
+            res_bond<R, FMT>(a, r, k0 + k, res_coupling<R, FMT>(a, c[k]), s[k].x(), s[k].y(), s[k].z(), hx, hy, hz);
+   }
+   return true;
+}
+
+// shared memory: slice offsets, materials, dictionary, words
+struct ResLayout {
+   int mats, dict, words, bytes;
+};
+template <typename R>
+__host__ __device__ inline ResLayout res_layout(int K, int M, int dict_bytes, int word_bytes) {
+   ResLayout l;
+   l.mats = ((kResSlices * K + 1 + 3) & ~3) * 4;
+   l.dict = (l.mats + (M <= kResMaxMat ? M * (int)sizeof(MatParams<R>) : 0) + 15) & ~15;
+   l.words = l.dict + dict_bytes;
+   l.bytes = l.words + word_bytes;
+   return l;
+}
+
+// blocks per SM that the registers are capped for: as many resident atoms as
+// the gather's loads in flight allow without spilling much
+template <typename R, int FMT, int VAR, int K> constexpr int res_min_blocks() {
+   if (sizeof(R) == 8) return 3;
+   if (FMT == FMT_DMI_TAB) return 4;
+   if (FMT == FMT_ISO_TAB && VAR == VAR_HEUN) return K == 1 ? 6 : K == 2 ? 5 : 4;
+   return 6;
+}
+
+// RF for formats other than FMT_ISO_TAB: the common facts written in -- thermal
+// noise from Philox, one system, no field per material, no host dipole field, a
+// scalar coupling table in the dictionary (FP32 DMI)
+constexpr int kResCommon = 1;
+template <typename R> inline int common_features(const LLGArgs<R>& a, int fmt, int var) {
+   const bool ok = var == VAR_HEUN && a.thermal && a.noise_mode == VGPU_NOISE_PHILOX && !a.sys_off && !a.ramp_n &&
+                   !a.local_field && !a.hd_atom && !(sizeof(R) == 4 && a.ex) &&
+                   !(fmt == FMT_DMI_TAB && sizeof(R) == 4 && !a.tab_scalar);
+   return ok ? kResCommon : 0;
+}
+template <typename R, int FMT, int RF> __device__ __forceinline__ LLGArgs<R> res_fold(const LLGArgs<R>& in) {
+   if (FMT == FMT_ISO_TAB) return fold_iso<R, RF>(in);
+   LLGArgs<R> a = in;
+   if (RF == kResCommon) {
+      a.thermal = 1;
+      a.noise_mode = VGPU_NOISE_PHILOX;
+      a.sys_off = nullptr;
+      a.ramp_n = 0;
+      a.local_field = 0;
+      a.hd_atom = nullptr;
+      if (sizeof(R) == 4) a.ex = a.ey = a.ez = nullptr;
+      if (FMT == FMT_DMI_TAB && sizeof(R) == 4) a.tab_scalar = 1;
+   }
+   return a;
+}
+
+// XA, XB: the tagged spins and predictor states of all threads' atoms (`plane`
+// bytes per word of a spin)
+template <typename R, int FMT, int VAR, int K, int RF>
+__global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR, K>()))
+    llg_resident_kernel(const LLGArgs<R> in, int nsteps, char* XA, char* XB, uint32_t plane, uint32_t epoch0,
+                        int nslices, int word_bytes) {
+   LLGArgs<R> a = res_fold<R, FMT, RF>(in);
+   constexpr bool WORDS = res_words<R, FMT>();
+   constexpr bool FIXED = FMT == FMT_ISO_TAB && (RF & ISO_FIXED) != 0;
+   extern __shared__ __align__(16) unsigned char res_smem[];
+   const int dict_bytes = WORDS && FMT == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
+   const ResLayout lay = res_layout<R>(K, a.M, dict_bytes, word_bytes);
+   int* s_off = reinterpret_cast<int*>(res_smem);
+   MatParams<R>* s_mat = reinterpret_cast<MatParams<R>*>(res_smem + lay.mats);
+   float4* s_dict = reinterpret_cast<float4*>(res_smem + lay.dict);
+   uint32_t* s_words = reinterpret_cast<uint32_t*>(res_smem + lay.words);
+   const int tid = threadIdx.x, blk = blockIdx.x;
+   // one coupling per atom: one material, or batched systems of one material
+   const bool one_j = FIXED || a.M == 1 || (a.sys_off && a.m_per_sys == 1);
+   R S0[K][3], P[K][3], E[K][3], j0[K];
+   int mi[K];
+#pragma unroll
+   for (int k = 0; k < K; ++k) {
+      const int i = (blk * K + k) * kResBlock + tid;
+      mi[k] = 0;
+      j0[k] = 0;
+      S0[k][0] = 1; S0[k][1] = 0; S0[k][2] = 0;  // threads past the last atom: a spin nobody reads
+      if (i < a.n_upd) {
+         mi[k] = a.mat ? __ldg(a.mat + i) : 0;
+         if (FMT == FMT_ISO_TAB) j0[k] = __ldg(a.jtab + mi[k] * a.M + mi[k]);
+         S0[k][0] = a.ax[i]; S0[k][1] = a.ay[i]; S0[k][2] = a.az[i];
+      }
+      P[k][0] = S0[k][0]; P[k][1] = S0[k][1]; P[k][2] = S0[k][2];
+      ResSpin<R>::store(XA, plane, 16u * (uint32_t)i, S0[k], epoch0);
+   }
+   const int s0 = blk * kResSlices * K, ns = min(kResSlices * K, nslices - s0);
+   const int o0 = __ldg(a.slice_off + s0);
+   if constexpr (WORDS) {
+      const int nw = __ldg(a.slice_off + s0 + ns) - o0;
+      const uint32_t* src = FMT == FMT_ISO_TAB ? reinterpret_cast<const uint32_t*>(a.col) : a.crec;
+      for (int q = tid; q < nw; q += kResBlock) s_words[q] = __ldg(src + o0 + q);
+      for (int q = tid; q < dict_bytes / 16; q += kResBlock) s_dict[q] = __ldg(a.cdict + q);
+   }
+   for (int q = tid; q <= kResSlices * K; q += kResBlock) s_off[q] = __ldg(a.slice_off + s0 + min(q, ns)) - o0;
+   if (a.M <= kResMaxMat) {
+      const int nw = a.M * (int)(sizeof(MatParams<R>) / 4);
+      for (int q = tid; q < nw; q += kResBlock)
+         reinterpret_cast<uint32_t*>(s_mat)[q] = __ldg(reinterpret_cast<const uint32_t*>(a.mp) + q);
+   }
+   const MatParams<R>* mpt = a.M <= kResMaxMat ? s_mat : a.mp;
+   __syncthreads();  // the last one: the steps order themselves by the tags
+   // FIXED, one atom per thread: the offsets of its six neighbours
+   constexpr bool REGS = FIXED && K <= 2;
+   uint32_t nb[REGS ? K : 1][6];
+   unsigned real[REGS ? K : 1];
+   bool six = false;
+   if constexpr (REGS) {
+      six = true;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+         const int sl = kResSlices * k + (tid >> 5), i = (blk * K + k) * kResBlock + tid;
+         const int off = s_off[sl], w = (s_off[sl + 1] - off) >> 5;
+         real[k] = 0;
+         six = six && w <= 6;
+#pragma unroll
+         for (int q = 0; q < 6; ++q) {
+            nb[k][q] = 16u * (uint32_t)i;
+            if (q < w) {
+               const uint32_t j = s_words[off + (tid & 31) + 32 * q] & (uint32_t)a.idx_mask;
+               if (j < (uint32_t)a.n) {
+                  real[k] |= 1u << q;
+                  nb[k][q] = 16u * j;
+               }
+            }
+         }
+      }
+   }
+   const uint64_t step0 = a.step;
+   auto field = [&](int k, int i, bool on, const char* X, uint32_t t, const R S[3], R H[3]) -> bool {
+      R hx = 0, hy = 0, hz = 0;
+      bool ok;
+      if (REGS && six) {
+         const int kk = REGS ? k : 0;
+         ResSpin<R> s[6];
+         ok = res_read<R, 6>(X, plane, nb[kk], t, s);
+#pragma unroll
+         for (int q = 0; q < 6; ++q)
+            if ((real[kk] >> q) & 1u) { hx += j0[k] * s[q].x(); hy += j0[k] * s[q].y(); hz += j0[k] * s[q].z(); }
+      } else {
+         const int sl = kResSlices * k + (tid >> 5);
+         const int off = s_off[sl];
+         const ResRow<R> r{o0 + off + (tid & 31), (s_off[sl + 1] - off) >> 5, s_words + off + (tid & 31), mi[k], one_j,
+                           j0[k], s_dict};
+         const uint32_t self = 16u * (uint32_t)i;
+         if constexpr (FMT == FMT_DMI_TAB && sizeof(R) == 4) {
+            // FCC rows: one round trip for all 12 neighbours
+            if (r.w == 12) ok = res_gather<R, FMT, 12>(a, r, X, plane, self, t, hx, hy, hz);
+            else ok = res_gather<R, FMT, 6>(a, r, X, plane, self, t, hx, hy, hz);
+         } else {
+            ok = res_gather<R, FMT, 6>(a, r, X, plane, self, t, hx, hy, hz);
+         }
+      }
+      if (ok && on) {
+         site_field<R, 0, VAR != VAR_HEUN>(a, i, mpt[mi[k]], nullptr, nullptr, nullptr, S, hx, hy, hz, H);
+         H[0] += E[k][0]; H[1] += E[k][1]; H[2] += E[k][2];
+      }
+      return ok;
+   };
+   bool ok = true;
+   for (int s = 0; s < nsteps && ok; ++s) {
+      a.step = step0 + (uint64_t)s;
+      set_ramp(a);
+      const uint32_t e = epoch0 + 2 * (uint32_t)s;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+         const int i = (blk * K + k) * kResBlock + tid;
+         if (i < a.n_upd) external_field<R>(a, i, mpt[mi[k]], true, E[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+         const int i = (blk * K + k) * kResBlock + tid;
+         const bool on = i < a.n_upd;
+         R H[3];
+         ok = ok && field(k, i, on, XA, e, S0[k], H);
+         if (ok) {
+            if (on) first_half<R, VAR>(a, i, mpt[mi[k]], S0[k], H, P[k]);
+            ResSpin<R>::store(XB, plane, 16u * (uint32_t)i, P[k], e + 1);
+         }
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+         const int i = (blk * K + k) * kResBlock + tid;
+         const bool on = i < a.n_upd;
+         R H[3], o[3];
+         ok = ok && field(k, i, on, XB, e + 1, P[k], H);
+         if (ok) {
+            if (on) {
+               second_half<R, VAR>(a, i, mpt[mi[k]], S0[k], P[k], H, o);
+               S0[k][0] = o[0]; S0[k][1] = o[1]; S0[k][2] = o[2];
+            }
+            ResSpin<R>::store(XA, plane, 16u * (uint32_t)i, S0[k], e + 2);
+         }
+      }
+   }
+   if (!ok) {
+      if ((tid & 31) == 0) atomicOr(a.status, 2);
+      return;
+   }
+#pragma unroll
+   for (int k = 0; k < K; ++k) {
+      const int i = (blk * K + k) * kResBlock + tid;
+      if (i < a.n_upd) {
+         a.ax[i] = S0[k][0]; a.ay[i] = S0[k][1]; a.az[i] = S0[k][2];
+         a.bx[i] = P[k][0]; a.by[i] = P[k][1]; a.bz[i] = P[k][2];
+      }
+   }
+}
+
+// ---------------------------------------------------------------------------
+// FP32 systems of isotropic bonds with at most 2,048 atoms: the system on one
+// thread-block cluster, the states in its distributed shared memory.
+//
+// A small system lives on a few SMs of one GPC, so its spins need not travel
+// through L2: each block keeps its atoms' spins and predictor states in shared
+// memory, neighbours are read from the block that has them, and the half-steps
+// are separated by the cluster's hardware barrier (arrive after the store, the
+// next noise drawn, then wait).  Microseconds a step against the tagged spins in
+// L2 above: 125 atoms 1.05 and 1.51, 990 atoms 1.49 and 2.02, 2,016 atoms 1.83
+// and 2.03; from 4,096 atoms the reads between SMs cost more than L2 (2.24 and
+// 1.97; 8,000 atoms 3.41 and 2.15), and FP64 gains nothing (990 atoms 3.4 and
+// 2.8), so those run above.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned res_cluster_rank() {
+   unsigned r;
+   asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+   return r;
+}
+__device__ __forceinline__ void res_cluster_arrive() {
+   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void res_cluster_wait() {
+   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// a spin in shared memory, padded to a power of two
+template <typename R> struct alignas(4 * sizeof(R)) ResVec {
+   R x, y, z, pad;
+};
+
+// address of `slot` of the spin array at shared address `arr` in block `rank`
+// of the cluster, and the spin at such an address
+template <typename R>
+__device__ __forceinline__ uint32_t res_address(uint32_t arr, uint32_t rank, uint32_t slot) {
+   uint32_t p;
+   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(arr), "r"(rank));
+   return p + (uint32_t)sizeof(ResVec<R>) * slot;
+}
+__device__ __forceinline__ void res_remote(uint32_t p, float& x, float& y, float& z) {
+   float pad;
+   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(pad) : "r"(p));
+}
+__device__ __forceinline__ void res_remote(uint32_t p, double& x, double& y, double& z) {
+   asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(p));
+   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(z) : "r"(p + 16u));
+}
+
+// the spin at p, in this block's own shared memory (`own`: a plain shared-memory
+// address) or in another block's.  The path between SMs is the narrow one, and
+// own neighbours are most.
+__device__ __forceinline__ void res_near(uint32_t p, bool own, float& x, float& y, float& z) {
+   float pad;
+   asm volatile(
+       "{\n .reg .pred o;\n setp.ne.u32 o, %5, 0;\n"
+       " @o ld.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+       " @!o ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+       : "=f"(x), "=f"(y), "=f"(z), "=f"(pad)
+       : "r"(p), "r"((uint32_t)own));
+}
+__device__ __forceinline__ void res_near(uint32_t p, bool own, double& x, double& y, double& z) {
+   asm volatile(
+       "{\n .reg .pred o;\n setp.ne.u32 o, %4, 0;\n"
+       " @o ld.shared::cta.v2.f64 {%0, %1}, [%3];\n @o ld.shared::cta.f64 %2, [%3 + 16];\n"
+       " @!o ld.shared::cluster.v2.f64 {%0, %1}, [%3];\n @!o ld.shared::cluster.f64 %2, [%3 + 16];\n}"
+       : "=d"(x), "=d"(y), "=d"(z)
+       : "r"(p), "r"((uint32_t)own));
+}
+
+// bond words of the cluster kernel: block << 12 | slot (the slot after the last
+// thread's: the zero spin that padded bonds read), coupling index or material << 16
+constexpr int kClusterBlock = kClusterAtoms / 16;
+constexpr uint32_t kResSlotBits = 12;
+
+template <typename R>
+__host__ __device__ inline ResLayout res_cluster_layout(int threads, int zmax, int M, int dict_bytes) {
+   ResLayout l;
+   const int vec = (threads + 1) * (int)sizeof(ResVec<R>);
+   l.mats = 2 * vec;
+   l.dict = (l.mats + (M <= kResMaxMat ? M * (int)sizeof(MatParams<R>) : 0) + 15) & ~15;
+   l.words = l.dict + dict_bytes;
+   l.bytes = l.words + 4 * threads * zmax;
+   return l;
+}
+
+// nsteps steps of all atoms, one per thread, in order over the blocks of one
+// cluster.  zmax: bonds of the widest row.
+template <typename R, int FMT, int VAR, int RF>
+__global__ void __launch_bounds__(kClusterBlock) llg_cluster_kernel(const LLGArgs<R> in, int nsteps, int zmax) {
+   static_assert(res_words<R, FMT>(), "formats whose bonds are one word");
+   LLGArgs<R> a = fold_iso<R, RF>(in);
+   extern __shared__ __align__(32) unsigned char res_smem[];
+   const int T = blockDim.x, tid = threadIdx.x;
+   const int dict_bytes = FMT == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
+   const ResLayout lay = res_cluster_layout<R>(T, zmax, a.M, dict_bytes);
+   ResVec<R>* sA = reinterpret_cast<ResVec<R>*>(res_smem);
+   ResVec<R>* sB = sA + T + 1;
+   MatParams<R>* s_mat = reinterpret_cast<MatParams<R>*>(res_smem + lay.mats);
+   float4* s_dict = reinterpret_cast<float4*>(res_smem + lay.dict);
+   uint32_t* s_words = reinterpret_cast<uint32_t*>(res_smem + lay.words);
+   const uint32_t rank = res_cluster_rank();
+   const int i = (int)rank * T + tid;
+   const bool on = i < a.n_upd;
+   const bool one_j = (RF & ISO_FIXED) != 0 || a.M == 1 || (a.sys_off && a.m_per_sys == 1);
+   ResRow<R> row{0, 0, nullptr, 0, one_j, (R)0, s_dict};
+   R S0[3] = {0, 0, 0}, P[3] = {0, 0, 0}, E[3] = {0, 0, 0};
+   const uint32_t zero_word = (rank << kResSlotBits) | (uint32_t)T;
+   if (on) {
+      const int off = __ldg(a.slice_off + (i >> 5));
+      row.base = off + (i & 31);
+      row.w = (__ldg(a.slice_off + (i >> 5) + 1) - off) >> 5;
+      row.mi = a.mat ? __ldg(a.mat + i) : 0;
+      if (FMT == FMT_ISO_TAB) row.j0 = __ldg(a.jtab + row.mi * a.M + row.mi);
+      for (int k = 0; k < row.w; ++k) {
+         const int e = row.base + 32 * k;
+         const uint32_t c = FMT == FMT_ISO_TAB ? (uint32_t)__ldg(a.col + e) : __ldg(a.crec + e);
+         const int j = (int)(c & (FMT == FMT_ISO_TAB ? (uint32_t)a.idx_mask : (1u << a.crec_shift) - 1u));
+         const uint32_t q = one_j && FMT == FMT_ISO_TAB ? 0u : res_coupling<R, FMT>(a, c);
+         uint32_t wd = zero_word;
+         if (j < a.n) wd = ((uint32_t)(j / T) << kResSlotBits) | (uint32_t)(j % T);
+         s_words[k * T + tid] = wd | (q << 16);
+      }
+   }
+   if (tid == 0) sA[T] = sB[T] = ResVec<R>{(R)0, (R)0, (R)0, (R)0};
+   for (int q = tid; q < dict_bytes / 16; q += T) s_dict[q] = __ldg(a.cdict + q);
+   if (a.M <= kResMaxMat) {
+      const int nw = a.M * (int)(sizeof(MatParams<R>) / 4);
+      for (int q = tid; q < nw; q += T)
+         reinterpret_cast<uint32_t*>(s_mat)[q] = __ldg(reinterpret_cast<const uint32_t*>(a.mp) + q);
+   }
+   const uint32_t arrA = (uint32_t)__cvta_generic_to_shared(sA), dB = (uint32_t)((T + 1) * (int)sizeof(ResVec<R>));
+   __syncthreads();  // materials and dictionary in place
+   const MatParams<R> m = a.M <= kResMaxMat ? s_mat[row.mi] : a.mp[row.mi];
+   if (a.sys_off && on) {
+      // the stream and atom numbering of this system (thermal_xi), once
+      const int k = row.mi / a.m_per_sys;
+      const uint64_t seed = (((uint64_t)a.seed_hi << 32) | a.seed_lo) + (uint64_t)k;
+      a.noise_base = 0u - (uint32_t)__ldg(a.sys_off + k);
+      a.seed_lo = (uint32_t)seed;
+      a.seed_hi = (uint32_t)(seed >> 32);
+   }
+   a.sys_off = nullptr;
+   // ISO_FIXED: the addresses of the six neighbours (rows of fewer: the zero slot)
+   constexpr uint32_t kSlot = (1u << kResSlotBits) - 1u;
+   uint32_t nb[6], own = 0;
+   if constexpr ((RF & ISO_FIXED) != 0) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+         const uint32_t c = k < row.w ? s_words[k * T + tid] : zero_word;
+         const uint32_t r = (c >> kResSlotBits) & 15u;
+         if (r == rank) own |= 1u << k;
+         nb[k] = r == rank ? arrA + (uint32_t)sizeof(ResVec<R>) * (c & kSlot) : res_address<R>(arrA, r, c & kSlot);
+      }
+   }
+   // everything above is as the upload or a copy on the stream left it; the spins
+   // and the dipole field are the previous kernel's
+   pdl_begin();
+   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+   if (on) { S0[0] = a.ax[i]; S0[1] = a.ay[i]; S0[2] = a.az[i]; }
+   sA[tid] = ResVec<R>{S0[0], S0[1], S0[2], (R)0};
+   res_cluster_arrive();
+   const uint64_t step0 = a.step;
+   // d: 0 for the spins, dB for the predictor states
+   auto field = [&](uint32_t d, const R S[3], R H[3]) {
+      R hx = 0, hy = 0, hz = 0;
+      if constexpr ((RF & ISO_FIXED) != 0) {
+         R x[6], y[6], z[6];
+#pragma unroll
+         for (int k = 0; k < 6; ++k) res_near(nb[k] + d, (own >> k) & 1u, x[k], y[k], z[k]);
+#pragma unroll
+         for (int k = 0; k < 6; ++k) { hx += row.j0 * x[k]; hy += row.j0 * y[k]; hz += row.j0 * z[k]; }
+      } else {
+         constexpr int W = sizeof(R) == 8 ? 4 : 6;  // loads in flight
+         for (int k0 = 0; k0 < row.w; k0 += W) {
+            uint32_t c[W];
+            R x[W], y[W], z[W];
+#pragma unroll
+            for (int k = 0; k < W; ++k) c[k] = k0 + k < row.w ? s_words[(k0 + k) * T + tid] : zero_word;
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+               res_remote(res_address<R>(arrA, (c[k] >> kResSlotBits) & 15u, c[k] & kSlot) + d, x[k], y[k], z[k]);
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+               if (k0 + k < row.w) res_bond<R, FMT>(a, row, k0 + k, c[k] >> 16, x[k], y[k], z[k], hx, hy, hz);
+         }
+      }
+      site_field<R, 0, VAR != VAR_HEUN>(a, i, m, nullptr, nullptr, nullptr, S, hx, hy, hz, H);
+      H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
+   };
+   for (int s = 0; s < nsteps; ++s) {
+      a.step = step0 + (uint64_t)s;
+      set_ramp(a);
+      if (on) external_field<R>(a, i, m, true, E);
+      res_cluster_wait();  // every block's spins of this step in place
+      if (on) {
+         R H[3];
+         field(0, S0, H);
+         first_half<R, VAR>(a, i, m, S0, H, P);
+         sB[tid] = ResVec<R>{P[0], P[1], P[2], (R)0};
+      }
+      res_cluster_arrive();
+      res_cluster_wait();  // every predictor state in place, every read of the spins done
+      if (on) {
+         R H[3], o[3];
+         field(dB, P, H);
+         second_half<R, VAR>(a, i, m, S0, P, H, o);
+         S0[0] = o[0]; S0[1] = o[1]; S0[2] = o[2];
+         sA[tid] = ResVec<R>{o[0], o[1], o[2], (R)0};
+      }
+      res_cluster_arrive();
+   }
+   if (on) {
+      a.ax[i] = S0[0]; a.ay[i] = S0[1]; a.az[i] = S0[2];
+      a.bx[i] = P[0]; a.by[i] = P[1]; a.bz[i] = P[2];
+   }
+   res_cluster_wait();  // no block leaves while its shared memory is read
+}
+
+// every bond i -> j has a bond j -> i (*bad set otherwise)
+template <typename R>
+__global__ void res_mutual_kernel(const LLGArgs<R> a, int* bad) {
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (i >= a.n) return;
+   const int off = a.slice_off[i >> 5], w = (a.slice_off[(i >> 5) + 1] - off) >> 5;
+   for (int k = 0; k < w; ++k) {
+      const int j = a.col[off + (i & 31) + 32 * k] & a.idx_mask;
+      if (j >= a.n) continue;  // padding entry
+      const int offj = a.slice_off[j >> 5], wj = (a.slice_off[(j >> 5) + 1] - offj) >> 5;
+      bool found = false;
+      for (int q = 0; q < wj && !found; ++q) found = (a.col[offj + (j & 31) + 32 * q] & a.idx_mask) == i;
+      if (!found) *bad = 1;
+   }
+}
+
+template <typename R> using ResidentFn = void (*)(LLGArgs<R>, int, char*, char*, uint32_t, uint32_t, int, int);
+
+// the kernel of a format, variant, number of atoms per thread and feature set
+// (nullptr: none; several atoms per thread are compiled for the two common
+// formats)
+template <typename R, int FMT, int K>
+inline ResidentFn<R> resident_heun(int feat) {
+   if constexpr (FMT == FMT_ISO_TAB) {
+      switch (feat) {
+#define VGPU_F(k) \
+   case k: return llg_resident_kernel<R, FMT, VAR_HEUN, K, k>;
+         VGPU_ISO_FEATURES(VGPU_F)
+#undef VGPU_F
+      }
+   } else if (feat == kResCommon) {
+      return llg_resident_kernel<R, FMT, VAR_HEUN, K, kResCommon>;
+   }
+   return llg_resident_kernel<R, FMT, VAR_HEUN, K, 0>;
+}
+
+// the feature set of a launch
+template <typename R> inline int resident_features(const LLGArgs<R>& a, int fmt, int var) {
+   return fmt == FMT_ISO_TAB ? iso_features<R>(a, fmt, var) : common_features<R>(a, fmt, var);
+}
+
+template <typename R, int FMT>
+inline ResidentFn<R> resident_fmt(int var, int K, int feat) {
+   if (var == VAR_HEUN) {
+      if (K == 1) return resident_heun<R, FMT, 1>(feat);
+      if constexpr (res_words<R, FMT>()) {
+         if (K == 2) return resident_heun<R, FMT, 2>(feat);
+         if (K == 4) return resident_heun<R, FMT, 4>(feat);
+      }
+      return nullptr;
+   }
+   if (K != 1) return nullptr;
+   if (var == VAR_HEUN_EXT) return llg_resident_kernel<R, FMT, VAR_HEUN_EXT, 1, 0>;
+   return llg_resident_kernel<R, FMT, VAR_MIDPOINT, 1, 0>;
+}
+
+template <typename R>
+inline ResidentFn<R> resident_fn(int fmt, int var, int K, int feat) {
+   switch (fmt) {
+      case FMT_ISO_TAB: return resident_fmt<R, FMT_ISO_TAB>(var, K, feat);
+      case FMT_ISO_BOND: return resident_fmt<R, FMT_ISO_BOND>(var, K, feat);
+      case FMT_VEC_TAB: return resident_fmt<R, FMT_VEC_TAB>(var, K, feat);
+      case FMT_VEC_BOND: return resident_fmt<R, FMT_VEC_BOND>(var, K, feat);
+      case FMT_DMI_TAB: return resident_fmt<R, FMT_DMI_TAB>(var, K, feat);
+      default: return resident_fmt<R, FMT_TENSOR_BOND>(var, K, feat);
+   }
+}
+
+// the cluster kernel of a variant and feature set (nullptr: none)
+template <typename R> using ClusterFn = void (*)(LLGArgs<R>, int, int);
+
+template <typename R>
+inline ClusterFn<R> cluster_fn(int fmt, int var, int feat) {
+   if constexpr (sizeof(R) == 4) {
+      if (fmt != FMT_ISO_TAB) return nullptr;
+      switch (feat) {
+#define VGPU_F(k) \
+   case k: return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN, k>;
+         VGPU_ISO_FEATURES(VGPU_F)
+#undef VGPU_F
+      }
+      if (var == VAR_HEUN) return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN, 0>;
+      if (var == VAR_HEUN_EXT) return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN_EXT, 0>;
+      return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_MIDPOINT, 0>;
+   }
+   return nullptr;
+}
+
+template <typename R>
+cudaError_t cluster_config(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, cudaLaunchConfig_t* cfg,
+                           cudaLaunchAttribute* attr, ClusterFn<R>* f) {
+   *f = cluster_fn<R>(fmt, var, c.zmax <= 6 ? iso_features<R>(a, fmt, var) : 0);
+   if (!*f) return cudaErrorInvalidValue;
+   const int dict = fmt == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
+   *cfg = cudaLaunchConfig_t{};
+   cfg->gridDim = dim3(c.size);
+   cfg->blockDim = dim3(c.threads);
+   cfg->dynamicSmemBytes = (size_t)res_cluster_layout<R>(c.threads, c.zmax, a.M, dict).bytes;
+   attr[0].id = cudaLaunchAttributeClusterDimension;
+   attr[0].val.clusterDim.x = c.size;
+   attr[0].val.clusterDim.y = 1;
+   attr[0].val.clusterDim.z = 1;
+   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   attr[1].val.programmaticStreamSerializationAllowed = 1;
+   cfg->attrs = attr;
+   cfg->numAttrs = 2;
+   return cudaSuccess;
+}
+
+// clusters of a shape that the GPU holds at once, whatever the parameters turn
+// out to be (0: it cannot run): the least over the generic kernel and the
+// compiled features
+template <typename R>
+cudaError_t cluster_capacity(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, int* clusters) {
+   *clusters = 0;
+   if (!cluster_fn<R>(fmt, var, 0)) return cudaSuccess;
+   cudaLaunchConfig_t cfg;
+   cudaLaunchAttribute attr[2];
+   ClusterFn<R> f;
+   cudaError_t e = cluster_config<R>(a, fmt, var, c, &cfg, attr, &f);
+   if (e != cudaSuccess) return e;
+   if (cfg.dynamicSmemBytes > kStageSmemLimit) return cudaSuccess;
+   std::vector<int> feats{0};
+   if (fmt == FMT_ISO_TAB && var == VAR_HEUN && c.zmax <= 6) {
+#define VGPU_F(k) feats.push_back(k);
+      VGPU_ISO_FEATURES(VGPU_F)
+#undef VGPU_F
+   }
+   int least = 1 << 30;
+   for (int feat : feats) {
+      f = cluster_fn<R>(fmt, var, feat);
+      if (c.size > 8) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+      int n = 0;
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, f, &cfg);
+      if (e != cudaSuccess) return e;
+      least = std::min(least, n);
+   }
+   *clusters = least;
+   return cudaSuccess;
+}
+
+template <typename R>
+cudaError_t launch_llg_cluster(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ClusterShape& c,
+                               cudaStream_t st) {
+   cudaLaunchConfig_t cfg;
+   cudaLaunchAttribute attr[2];
+   ClusterFn<R> f;
+   cudaError_t e = cluster_config<R>(a, fmt, var, c, &cfg, attr, &f);
+   if (e != cudaSuccess) return e;
+   cfg.stream = st;
+   return cudaLaunchKernelEx(&cfg, f, a, nsteps, c.zmax);
+}
+
+// dynamic shared memory of a plan
+template <typename R>
+static int resident_smem(const LLGArgs<R>& a, int fmt, const ResidentPlan& p) {
+   const bool words = fmt == FMT_ISO_TAB || (fmt == FMT_DMI_TAB && sizeof(R) == 4);
+   const int dict = words && fmt == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
+   return res_layout<R>(p.K, a.M, dict, words ? p.word_bytes : 0).bytes;
+}
+
+template <typename R>
+cudaError_t resident_capacity(const LLGArgs<R>& a, int fmt, int var, const ResidentPlan& p, int sms, int* blocks) {
+   *blocks = 0;
+   const int smem = resident_smem<R>(a, fmt, p);
+   if (!resident_fn<R>(fmt, var, p.K, 0) || smem > kStageSmemLimit) return cudaSuccess;
+   std::vector<int> feats{0};  // whatever the parameters turn out to be: the least over the compiled features
+   if (fmt == FMT_ISO_TAB && var == VAR_HEUN) {
+#define VGPU_F(k) feats.push_back(k);
+      VGPU_ISO_FEATURES(VGPU_F)
+#undef VGPU_F
+   } else if (var == VAR_HEUN) {
+      feats.push_back(kResCommon);
+   }
+   int least = 1 << 30;
+   for (int feat : feats) {
+      const ResidentFn<R> f = resident_fn<R>(fmt, var, p.K, feat);
+      cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+      int per_sm = 0;
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kResBlock, smem);
+      if (e != cudaSuccess) return e;
+      least = std::min(least, per_sm * sms);
+   }
+   *blocks = least;
+   return cudaSuccess;
+}
+
+template <typename R>
+cudaError_t launch_resident_check(const LLGArgs<R>& a, int* bad, cudaStream_t st) {
+   res_mutual_kernel<R><<<(a.n + 255) / 256, 256, 0, st>>>(a, bad);
+   return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t launch_llg_resident(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ResidentPlan& p, int nslices,
+                                cudaStream_t st) {
+   const ResidentFn<R> f = resident_fn<R>(fmt, var, p.K, resident_features<R>(a, fmt, var));
+   if (!f) return cudaErrorInvalidValue;
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(p.grid);
+   cfg.blockDim = dim3(kResBlock);
+   cfg.dynamicSmemBytes = (size_t)resident_smem<R>(a, fmt, p);
+   cfg.stream = st;
+   cudaLaunchAttribute attr[1];
+   attr[0].id = cudaLaunchAttributeCooperative;  // every block resident: threads wait on one another's spins
+   attr[0].val.cooperative = 1;
+   cfg.attrs = attr;
+   cfg.numAttrs = 1;
+   char* X = static_cast<char*>(p.spins);
+   const uint32_t plane = 16u * (uint32_t)(p.grid * p.K * kResBlock);
+   return cudaLaunchKernelEx(&cfg, f, a, nsteps, X, X + (size_t)ResSpin<R>::kWords * plane, plane, p.epoch, nslices,
+                             p.word_bytes);
+}
+
+}  // namespace vgpu

@@ -188,6 +188,67 @@ static int validate(vgpu_ctx* h, const vgpu_system_desc* d) {
    return VGPU_OK;
 }
 
+// Plan of the resident steps: the fewest atoms per thread at which the Heun
+// kernel's blocks are resident together (none: larger systems, and systems with
+// one-sided bonds, run one launch per pass).
+template <typename R>
+static int plan_resident(vgpu_ctx* h) {
+   SysDev& S = h->sys;
+   S.res = ResidentPlan();
+   S.one = ClusterShape();
+   S.zmax = 0;
+   for (int s = 0; s < S.nslices; ++s) S.zmax = std::max(S.zmax, (S.off_host[s + 1] - S.off_host[s]) / 32);
+   if (S.fmt == FMT_DMI_TAB && sizeof(R) == 4 && !S.crec) return VGPU_OK;  // the kernel reads compact records
+   {
+      // one cluster: a block up to 128 atoms, else up to 16 blocks of at least 64
+      // (us a step, simple cubic: 125 atoms 1.02 in one block, 1.22 in two; 990
+      // atoms 1.45 in 16 blocks, 1.50 in 8, 1.97 in 2)
+      ClusterShape c;
+      c.size = 1;
+      while (c.size < 16 && (c.size == 1 ? 128 : 64) * c.size < S.n) c.size *= 2;
+      c.threads = std::max(64, ((S.n + c.size - 1) / c.size + 31) / 32 * 32);
+      c.zmax = S.zmax;
+      if (S.n <= kClusterAtoms) {
+         if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, VAR_HEUN, c, &c.cap), "cluster plan")) return rc;
+         c.cap_var = VAR_HEUN;
+         if (c.cap > 0) S.one = c;
+      }
+   }
+   int sms = 0;
+   if (int rc = cuda_err(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device), "device")) return rc;
+   const LLGArgs<R> a = make_args<R>(h);
+   constexpr int per = kResidentBlock / 32;  // slices of a block and atom per thread
+   for (int K : {1, 2, 4}) {
+      ResidentPlan p;
+      p.K = K;
+      p.grid = (S.nslices + per * K - 1) / (per * K);
+      if (p.grid > sms * (2048 / kResidentBlock)) continue;  // 2,048 threads per SM
+      for (int b = 0; b < p.grid; ++b)
+         p.word_bytes = std::max(p.word_bytes,
+                                 4 * (S.off_host[std::min(S.nslices, per * K * (b + 1))] - S.off_host[per * K * b]));
+      int blocks = 0;
+      if (int rc = cuda_err(h, resident_capacity<R>(a, S.fmt, VAR_HEUN, p, sms, &blocks), "resident plan")) return rc;
+      if (blocks < p.grid) continue;
+      p.cap_var = VAR_HEUN;
+      p.cap_blocks = blocks;
+      // two states of one (FP32) or two (FP64) 16-byte words per thread's atom
+      const size_t bytes = 2 * (sizeof(R) == 8 ? 2 : 1) * 16 * (size_t)p.grid * K * kResidentBlock;
+      p.spins = h->alloc(bytes);
+      if (!p.spins) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the resident plan");
+      int bad = 0;
+      int rc = cuda_err(h, cudaMemsetAsync(p.spins, 0, bytes, h->stream), "resident plan");
+      if (!rc) rc = cuda_err(h, launch_resident_check<R>(a, S.status, h->stream), "resident plan");
+      if (!rc)
+         rc = cuda_err(h, cudaMemcpyAsync(&bad, S.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "resident plan");
+      if (!rc) rc = cuda_err(h, cudaStreamSynchronize(h->stream), "resident plan");
+      if (!rc && bad) return cuda_err(h, cudaMemsetAsync(S.status, 0, sizeof(int), h->stream), "status");
+      if (rc) return rc;
+      S.res = p;
+      return VGPU_OK;
+   }
+   return VGPU_OK;
+}
+
 template <typename R>
 static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
    const int n = d->num_atoms;
@@ -307,7 +368,6 @@ static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
             S.crec_shift = shift;
             S.cdict_n = ndict;
             S.crec_host = std::move(crec);
-            S.off_host = off;
          }
       }
    }
@@ -330,8 +390,10 @@ static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
    S.status = (int*)h->alloc(sizeof(int));
    if (!S.status) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for status word");
    if ((rc = cuda_err(h, cudaMemsetAsync(S.status, 0, sizeof(int), h->stream), "status"))) return rc;
+   S.off_host = std::move(off);
    S.uploaded = true;
-   return h->refresh_materials();
+   if ((rc = h->refresh_materials())) return rc;
+   return plan_resident<R>(h);
 }
 
 template <typename R>
@@ -452,6 +514,7 @@ LLGArgs<R> make_args(vgpu_ctx* h) {
    a.sys_off = S.sys_off;
    a.m_per_sys = S.m_per_sys;
    a.ramp_n = S.ramp_n;
+   set_ramp(a);
    return a;
 }
 template LLGArgs<float> make_args<float>(vgpu_ctx*);
@@ -562,9 +625,17 @@ static int ensure_window_plan(vgpu_ctx* h) {
    return VGPU_OK;
 }
 
-// increment buffers and the staged launch shape, before any pass
+// whether the passes draw thermal noise (worth keeping the external field
+// for: 24 bytes an atom and step against the generator and its transforms)
+static bool thermal_philox(const vgpu_ctx* h) {
+   return h->params.thermal_enabled && h->any_sigma && h->noise_mode == VGPU_NOISE_PHILOX;
+}
+
+// increment buffers and the staged launch shape, before any pass; whole_steps:
+// the caller runs both passes of every step, so that the external field may be
+// kept between them
 template <typename R>
-static int prepare_passes(vgpu_ctx* h, bool* staged_out, int integrator = INTEG_HEUN) {
+static int prepare_passes(vgpu_ctx* h, bool* staged_out, int integrator = INTEG_HEUN, bool whole_steps = false) {
    int rc0 = ensure_increment<R>(h);
    if (rc0) return rc0;
    const bool staged = integrator == INTEG_HEUN && use_staged<R>(h);
@@ -585,7 +656,7 @@ static int prepare_passes(vgpu_ctx* h, bool* staged_out, int integrator = INTEG_
       if (e != cudaSuccess) return cuda_err(h, e, "staged pass setup (tile records exceed shared memory?)");
       h->sys.stage = c;
    }
-   if (staged && !h->sys.stage.win && !h->sys.g_store[0]) {
+   if ((staged ? !h->sys.stage.win : whole_steps && thermal_philox(h)) && !h->sys.g_store[0]) {
       // the step's external field, passed from the predictor to the corrector
       const size_t len = ((size_t)h->sys.n_alloc + 3) & ~(size_t)3;
       for (int q = 0; q < 3; ++q) {
@@ -602,12 +673,12 @@ static int prepare_passes(vgpu_ctx* h, bool* staged_out, int integrator = INTEG_
 // completes the step (counter, dipole cadence)
 template <typename R>
 static int run_pass(vgpu_ctx* h, int mode, bool staged, int integrator = INTEG_HEUN, int first_slice = 0,
-                    int end = -1) {
+                    int end = -1, bool whole_steps = false) {
    LLGArgs<R> a = make_args<R>(h);
    a.integrator = integrator;
    a.slice_first = first_slice;
    if (end >= 0) a.n_upd = end;
-   if (staged && !h->sys.stage.win) {
+   if (staged ? !h->sys.stage.win : whole_steps && thermal_philox(h)) {
       a.gx = (R*)h->sys.g_store[0]; a.gy = (R*)h->sys.g_store[1]; a.gz = (R*)h->sys.g_store[2];
    }
    const int kind = mode == PASS_PREDICTOR ? PROF_PREDICTOR : PROF_CORRECTOR;
@@ -621,14 +692,90 @@ static int run_pass(vgpu_ctx* h, int mode, bool staged, int integrator = INTEG_H
    return h->after_step();
 }
 
+// How the next steps run.  Resident forms need a plan that fits for this
+// variant and nothing that asks for the separate passes (per-launch timing, a
+// pass option set by the caller, a shard, a second neighbour list).
+enum StepMode { STEP_PASSES, STEP_GRID, STEP_CLUSTER };
+
+template <typename R>
+static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
+   SysDev& S = h->sys;
+   *mode = STEP_PASSES;
+   if (h->prof_on || S.n_owned != S.n || S.bq_off || h->staged >= 0 || h->stage_sl > 0 || h->stage_nbuf > 0 ||
+       h->compact >= 0 || h->window >= 0 || h->stage_warps >= 0 || h->stage_wait_test)
+      return VGPU_OK;
+   *var = integrator == INTEG_MIDPOINT ? VAR_MIDPOINT : S.aniso_ext ? VAR_HEUN_EXT : VAR_HEUN;
+   if (S.one.size) {
+      if (S.one.cap_var != *var) {
+         if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, *var, S.one, &S.one.cap), "cluster plan"))
+            return rc;
+         S.one.cap_var = *var;
+      }
+      if (S.one.cap > 0) {
+         *mode = STEP_CLUSTER;
+         return VGPU_OK;
+      }
+   }
+   if (!S.res.K) return VGPU_OK;
+   if (S.res.cap_var != *var) {
+      int sms = 0;
+      int rc = cuda_err(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device), "device");
+      if (!rc)
+         rc = cuda_err(h, resident_capacity<R>(make_args<R>(h), S.fmt, *var, S.res, sms, &S.res.cap_blocks),
+                       "resident plan");
+      if (rc) return rc;
+      S.res.cap_var = *var;
+   }
+   if (S.res.cap_blocks >= S.res.grid) *mode = STEP_GRID;
+   return VGPU_OK;
+}
+
+// `n` resident steps, none of which but the last ends with a dipole update
+template <typename R>
+static int run_resident(vgpu_ctx* h, uint64_t n, StepMode mode, int var) {
+   SysDev& S = h->sys;
+   const LLGArgs<R> a = make_args<R>(h);
+   const cudaError_t e = mode == STEP_CLUSTER ? launch_llg_cluster<R>(a, S.fmt, var, (int)n, S.one, h->stream)
+                                              : launch_llg_resident<R>(a, S.fmt, var, (int)n, S.res, S.nslices, h->stream);
+   if (e != cudaSuccess) return cuda_err(h, e, "resident llg launch");
+   h->kernel_launches += 1;
+   if (mode == STEP_GRID) S.res.epoch += 2 * (uint32_t)n;
+   h->step += n;
+   return h->after_step();
+}
+
 template <typename R>
 static int llg_steps_typed(vgpu_ctx* h, uint64_t n_steps, int integrator = INTEG_HEUN) {
-   bool staged = false;
-   int rc = prepare_passes<R>(h, &staged, integrator);
-   for (uint64_t t = 0; t < n_steps && !rc; ++t) {
-      rc = h->fields_ready();
-      if (!rc) rc = run_pass<R>(h, PASS_PREDICTOR, staged, integrator);
-      if (!rc) rc = run_pass<R>(h, PASS_CORRECTOR, staged, integrator);
+   StepMode mode = STEP_PASSES;
+   int var = VAR_HEUN;
+   int rc = step_mode<R>(h, integrator, &mode, &var);
+   if (rc) return rc;
+   bool staged = false, prepared = false;
+   if (mode == STEP_PASSES) {
+      rc = prepare_passes<R>(h, &staged, integrator, true);
+      prepared = true;
+   } else {
+      rc = ensure_increment<R>(h);
+   }
+   const uint64_t most = mode == STEP_CLUSTER ? kClusterSteps
+                         : h->sys.n <= kGridSmallAtoms ? kGridSmallSteps
+                                                       : kGridSteps;
+   while (n_steps > 0 && !rc) {
+      if ((rc = h->fields_ready())) break;
+      uint64_t n = 1;
+      if (mode != STEP_PASSES) n = std::min(std::min(n_steps, dipole_steps_left(h)), most);
+      // a single step: a cooperative launch (6.2 us) costs more than two passes (5.0)
+      if (mode == STEP_CLUSTER || (mode == STEP_GRID && n > 1)) {
+         rc = run_resident<R>(h, n, mode, var);
+      } else {
+         if (!prepared) {
+            rc = prepare_passes<R>(h, &staged, integrator, true);
+            prepared = true;
+         }
+         if (!rc) rc = run_pass<R>(h, PASS_PREDICTOR, staged, integrator, 0, -1, true);
+         if (!rc) rc = run_pass<R>(h, PASS_CORRECTOR, staged, integrator, 0, -1, true);
+      }
+      n_steps -= n;
    }
    return rc;
 }

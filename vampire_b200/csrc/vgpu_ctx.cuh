@@ -30,6 +30,9 @@ struct SysDev {
    int crec_shift = 0, cdict_n = 0;
    std::vector<uint32_t> crec_host;  // host copy of crec (window planning)
    std::vector<int> off_host;        // host copy of slice_off
+   ResidentPlan res;                 // resident steps (systems that fit the GPU's resident threads)
+   ClusterShape one;                 // the system on one cluster (systems of at most 16 x 1,024 atoms)
+   int zmax = 0;                     // bonds of the widest row
    // window plan of the window-staged passes (built on first use for the tile
    // shape and owned-atom count it was made for)
    int win_sl = 0, win_nupd = -1;
@@ -102,6 +105,7 @@ void torque_destroy(vgpu_ctx* h);
 void cmc_destroy(vgpu_ctx* h);
 int torque_reset(vgpu_ctx* h);
 const double* batch_ramp(vgpu_ctx* h);
+uint64_t dipole_steps_left(vgpu_ctx* h);  // steps up to and including the next dipole update (UINT64_MAX: none)
 
 }  // namespace vgpu
 

@@ -90,7 +90,8 @@ struct LLGArgs {
    const R* bq_j;            // isotropic J_bq [T] per entry
    R hx, hy, hz;             // global applied field
    int local_field;          // add MatParams::hl*
-   uint64_t ramp_n;          // > 0: add MatParams::dh * min(step, ramp_n) / ramp_n
+   uint64_t ramp_n;          // > 0: add MatParams::dh * ramp_f
+   R ramp_f;                 // min(step, ramp_n) / ramp_n (set_ramp)
    const int* sys_off;       // batched systems: first atom of each system, or nullptr
    int m_per_sys;            // materials per system (system = material / m_per_sys)
    int thermal;              // add sigma * xi
@@ -109,12 +110,17 @@ struct LLGArgs {
    R* bx; R* by; R* bz;      // state B: s' (predictor output)
    R* fx; R* fy; R* fz;      // field output (field-only mode)
    R* ex; R* ey; R* ez;      // stored predictor increment f(s0), or nullptr (recovered)
-   R* gx; R* gy; R* gz;      // staged passes: the step's external field (thermal, applied,
-                             // macrocell dipole), written by the predictor and read back by
-                             // the corrector, or nullptr
+   R* gx; R* gy; R* gz;      // the step's external field (thermal, applied, macrocell
+                             // dipole), written by the predictor and read back by the
+                             // corrector, or nullptr (the corrector computes it)
    int* status;              // device status word (non-finite spin flag)
    int stage_extra_tx;       // staged passes: extra bytes each tile expects (0; > 0 tests the bounded wait)
 };
+
+// the sweep's fraction at a.step, with every change of the step
+template <typename R> __host__ __device__ inline void set_ramp(LLGArgs<R>& a) {
+   a.ramp_f = a.ramp_n ? (R)(a.step < a.ramp_n ? a.step : a.ramp_n) / (R)a.ramp_n : (R)0;
+}
 
 // FP32 DMI record layout a kernel is compiled for (exchange_field)
 enum RecLayout : int { REC_ANY = 0, REC_WIDE = 1, REC_COMPACT = 2, REC_WINDOW = 3 };
@@ -154,6 +160,44 @@ inline int staged_smem_bytes(int sl, int nbuf, int buf_bytes, int dict_bytes, in
 int stage_tile_bytes(const std::vector<int>& slice_off, int sl);
 cudaError_t prepare_llg_staged(StageCfg& c, int nslices, int device);
 cudaError_t launch_llg_staged(const LLGArgs<float>& a, int mode, int nslices, const StageCfg& c, cudaStream_t st);
+
+// Resident steps (llg_resident.cuh): many steps in one cooperative launch,
+// K atoms per thread.
+constexpr int kResidentBlock = 128;  // threads per block
+// steps of one launch.  A cooperative launch keeps its threads on the SMs until
+// it ends, and programs hold small systems by the dozen: those take turns.
+constexpr int kGridSmallAtoms = 16384, kGridSmallSteps = 10, kGridSteps = 4096;
+struct ResidentPlan {
+   int K = 0;                 // atoms per thread (0: no plan)
+   int grid = 0;              // blocks
+   int word_bytes = 0;        // bond words of the largest block, in bytes
+   void* spins = nullptr;     // tagged spins and predictor states (16-byte words)
+   uint32_t epoch = 1;        // number of the next half-step (0: what the cleared buffer holds)
+   int cap_var = -1, cap_blocks = 0;  // blocks of a variant's kernel that the GPU holds at once
+};
+// The system on one cluster, one atom per thread (llg_resident.cuh).
+constexpr int kClusterAtoms = 2048;
+constexpr int kClusterSteps = 5;  // steps of one launch
+struct ClusterShape {
+   int size = 0;              // blocks per cluster (0: none)
+   int threads = 0;           // threads per block
+   int zmax = 0;              // bonds of the widest row
+   int cap_var = -1, cap = 0; // clusters of a variant's kernel that the GPU holds at once
+};
+template <typename R>
+cudaError_t cluster_capacity(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, int* clusters);
+template <typename R>
+cudaError_t launch_llg_cluster(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ClusterShape& c,
+                               cudaStream_t st);
+
+// blocks of the variant's kernel that are resident together (0: no such kernel)
+template <typename R>
+cudaError_t resident_capacity(const LLGArgs<R>& a, int fmt, int var, const ResidentPlan& p, int sms, int* blocks);
+template <typename R>
+cudaError_t launch_resident_check(const LLGArgs<R>& a, int* bad, cudaStream_t st);
+template <typename R>
+cudaError_t launch_llg_resident(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ResidentPlan& p, int nslices,
+                                cudaStream_t st);
 
 // write the Philox thermal Gaussians of step a.step into a.fx/fy/fz
 template <typename R>

@@ -99,6 +99,29 @@ def test_applied_field_of_each_call(vgpu_lib):
 
 
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_spins_set_between_calls(vgpu_lib, prec):
+    """A launch starts from the spins it finds, not from the words that the one
+    before left behind (many blocks, so that some start late)."""
+    from vampire_b200 import system as S
+    from vampire_b200 import vgpu
+    s = S.config_sc_llg(36, temperature=300.0)
+    starts = [S.random_spins(s.n, k) for k in range(6)]
+    out = []
+    for passes in (False, True):
+        with vgpu.Simulation(s, precision=prec, noise_seed=5) as sim:
+            if passes:
+                sim.set_option(vgpu.OPT_STAGED_RECORDS, 1)
+            got = []
+            for sp in starts:
+                sim.set_spins(sp)
+                sim.llg_heun(2)
+                got.append(sim.spins())
+            out.append(got)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
 def test_batch(vgpu_lib, prec):
     from vampire_b200 import batch as B
     from vampire_b200 import vgpu

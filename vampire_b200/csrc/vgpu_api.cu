@@ -739,7 +739,8 @@ static int run_resident(vgpu_ctx* h, uint64_t n, StepMode mode, int var) {
                                               : launch_llg_resident<R>(a, S.fmt, var, (int)n, S.res, S.nslices, h->stream);
    if (e != cudaSuccess) return cuda_err(h, e, "resident llg launch");
    h->kernel_launches += 1;
-   if (mode == STEP_GRID) S.res.epoch += 2 * (uint32_t)n;
+   // past every number of this launch: its last spins are not the next one's first
+   if (mode == STEP_GRID) S.res.epoch += 2 * (uint32_t)n + 2;
    h->step += n;
    return h->after_step();
 }

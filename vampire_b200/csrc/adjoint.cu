@@ -38,7 +38,7 @@
 #include <cstring>
 #include <vector>
 
-#include "llg_kernels.cuh"
+#include "llg_resident.cuh"
 #include "vgpu_ctx.cuh"
 
 namespace vgpu {
@@ -420,6 +420,210 @@ __global__ void mz_kernel(int n, const R* __restrict__ sz, const int* __restrict
    }
 }
 
+// ---------------------------------------------------------------------------
+// The same backward pass with resident threads (systems with a plan of one atom
+// per thread).
+//
+// Per step the launches above take four kernels, and the forward sweeps two
+// launches and a sum each: some 40 us a step at 32,768 atoms, where the
+// arithmetic takes one or two -- bound by the launches.  What does not depend on
+// the adjoint vector -- the recomputed s', f, H(s) exchange and H(s') exchange of
+// kernels (1) and (2) -- is computed for a run of steps at once
+// (adj_states_kernel, adj_fields_kernel: every step and atom in parallel).  The
+// rest runs step after step in one cooperative launch whose threads keep lambda
+// and the gradient sums in registers; only Hbar / mu_s of the two transposed
+// gathers travels, as tagged words (llg_resident.cuh), and the parameter
+// gradients are reduced once at the end.  The sweeps forward run resident too
+// (llg_path_kernel).
+// ---------------------------------------------------------------------------
+template <typename R> struct AdjRun {
+   const R* S;        // states of the run's steps, 3 stride values each
+   R *sp, *ex0, *f0, *ex1;  // [steps][3 stride]
+   R* nv;             // [steps][stride]
+};
+
+// kernel (1) for every step (blockIdx.y) of the run
+template <typename R, int FMT>
+__global__ void __launch_bounds__(256) adj_states_kernel(const LLGArgs<R> a, const AdjRun<R> w, int n, int st) {
+   pdl_begin();
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (i >= n) return;
+   const size_t o = 3 * (size_t)st * blockIdx.y;
+   const R* x = w.S + o;
+   const int mi = a.mat ? a.mat[i] : 0;
+   const MatParams<R> m = a.mp[mi];
+   const R S[3] = {x[i], x[st + i], x[2 * st + i]};
+   R ex[3] = {0, 0, 0}, Ha[3], d[3], v[3];
+   exchange_gather<R, FMT>(a, i, mi, x, x + st, x + 2 * st, ex[0], ex[1], ex[2]);
+   aniso_h(a, m, S, Ha);
+   const R H[3] = {ex[0] + Ha[0] + a.hx, ex[1] + Ha[1] + a.hy, ex[2] + Ha[2] + a.hz};
+   llg_rhs<R>(m.A, m.B, S, H, d);
+   for (int k = 0; k < 3; ++k) {
+      w.ex0[o + k * st + i] = ex[k];
+      w.f0[o + k * st + i] = d[k];
+      v[k] = S[k] + d[k] * a.dt;
+   }
+   const R L = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+   w.nv[(size_t)st * blockIdx.y + i] = L;
+   for (int k = 0; k < 3; ++k) w.sp[o + k * st + i] = v[k] / L;
+}
+
+// the exchange field of s' (kernel (2)) for every step of the run
+template <typename R, int FMT>
+__global__ void __launch_bounds__(256) adj_fields_kernel(const LLGArgs<R> a, const AdjRun<R> w, int n, int st) {
+   pdl_begin();
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (i >= n) return;
+   const size_t o = 3 * (size_t)st * blockIdx.y;
+   const R* x = w.sp + o;
+   const int mi = a.mat ? a.mat[i] : 0;
+   R ex[3] = {0, 0, 0};
+   exchange_gather<R, FMT>(a, i, mi, x, x + st, x + 2 * st, ex[0], ex[1], ex[2]);
+   for (int k = 0; k < 3; ++k) w.ex1[o + k * st + i] = ex[k];
+}
+
+// kernels (2)-(4) of steps t0 + nsteps - 1 down to t0 (w: the run from step t0)
+template <typename R, int FMT, bool PAIR>
+__global__ void __launch_bounds__(kResBlock, sizeof(R) == 8 ? 3 : 4)
+    adj_backward_kernel(const LLGArgs<R> a, const AdjBufs<R> b, const AdjRun<R> w, int64_t t0, int nsteps, char* XA,
+                        char* XB, uint32_t plane, uint32_t epoch0, int nslices, int word_bytes) {
+   extern __shared__ __align__(16) unsigned char res_smem[];
+   __shared__ double s_pair[PAIR ? 1 + kAdjMaxPairMat * kAdjMaxPairMat : 1];
+   if (PAIR)
+      for (int k = threadIdx.x; k < 1 + a.M * a.M; k += kResBlock) s_pair[k] = 0.0;
+   const ResBlockData<R, FMT> d(a, res_smem, nslices, word_bytes);
+   const int st = b.stride, i = blockIdx.x * kResBlock + threadIdx.x;
+   const bool on = i < b.n;
+   const uint32_t self = 16u * (uint32_t)i;
+   const ResRow<R> r = d.row(a, on ? i : 0);
+   const MatParams<R> m = d.mat(a, r.mi);
+   const R mu = m.mu_s_muB;
+   double gv[5] = {0, 0, 0, 0, 0};
+   R l[3] = {0, 0, 0};
+   if (on)
+      for (int k = 0; k < 3; ++k) l[k] = b.lam[k * st + i];
+   bool ok = true;
+   for (int q = nsteps - 1; q >= 0; --q) {
+      const size_t o = 3 * (size_t)st * q;
+      const uint32_t e = epoch0 + 2 * (uint32_t)(nsteps - 1 - q);
+      R S[3] = {1, 0, 0}, Sp[3] = {1, 0, 0}, ex0[3] = {0, 0, 0}, ex1[3] = {0, 0, 0}, ub[3] = {0, 0, 0},
+        spb[3] = {0, 0, 0}, hb1[3] = {0, 0, 0}, send[3] = {0, 0, 0}, nv = 1, sb[3] = {0, 0, 0}, hb0[3] = {0, 0, 0};
+      if (on) {
+         R f0[3];
+         for (int k = 0; k < 3; ++k) {
+            const size_t at = o + (size_t)k * st + i;
+            S[k] = w.S[at]; Sp[k] = w.sp[at]; ex0[k] = w.ex0[at]; ex1[k] = w.ex1[at]; f0[k] = w.f0[at];
+         }
+         nv = w.nv[(size_t)st * q + i];
+         R Ha[3], f1[3], u[3];
+         aniso_h(a, m, Sp, Ha);
+         const R H1[3] = {ex1[0] + Ha[0] + a.hx, ex1[1] + Ha[1] + a.hy, ex1[2] + Ha[2] + a.hz};
+         llg_rhs<R>(m.A, m.B, Sp, H1, f1);
+         for (int k = 0; k < 3; ++k) u[k] = S[k] + (R)0.5 * a.dt * (f0[k] + f1[k]);
+         const R L = sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+         const R s1[3] = {u[0] / L, u[1] / L, u[2] / L};
+         const R ls = l[0] * s1[0] + l[1] * s1[1] + l[2] * s1[2];
+         R a1[3], hb[3];
+         for (int k = 0; k < 3; ++k) { ub[k] = (l[k] - ls * s1[k]) / L; a1[k] = (R)0.5 * a.dt * ub[k]; }
+         f_vjp(m.A, m.B, Sp, H1, a1, spb, hb);
+         const R imu = (R)1 / m.mu_s_muB;  // Hbar / mu_s for the transposed gather
+         for (int k = 0; k < 3; ++k) send[k] = hb[k] * imu;
+         ResSpin<R>::store(XA, plane, self, send, e + 1);
+         for (int k = 0; k < 3; ++k) {
+            hb1[k] = send[k] * mu;
+            gv[0] += (double)hb[k] * (double)ex1[k];
+            gv[2 + k] += (double)hb[k];
+         }
+         if (PAIR) pair_grads<R, FMT>(a, i, r.mi, w.sp + o, w.sp + o + st, w.sp + o + 2 * st, hb, s_pair);
+         if (a.uniaxial) gv[1] += ku_grad(m, hb, Sp);
+      } else {
+         ResSpin<R>::store(XA, plane, self, send, e + 1);
+      }
+      R t[3] = {0, 0, 0};
+      ok = res_gather<R, FMT, 6>(a, r, XA, plane, self, e + 1, t[0], t[1], t[2]);
+      if (!ok) break;
+      if (on) {
+         R spbar[3], vb[3], a0[3], Ha[3], H0[3], sdir[3], hb[3];
+         for (int k = 0; k < 3; ++k) spbar[k] = spb[k] + t[k] * mu;
+         aniso_vjp(a, m, Sp, hb1, spbar);
+         const R sps = spbar[0] * Sp[0] + spbar[1] * Sp[1] + spbar[2] * Sp[2];
+         for (int k = 0; k < 3; ++k) {
+            vb[k] = (spbar[k] - sps * Sp[k]) / nv;
+            a0[k] = (R)0.5 * a.dt * ub[k] + a.dt * vb[k];
+         }
+         aniso_h(a, m, S, Ha);
+         for (int k = 0; k < 3; ++k) H0[k] = ex0[k] + Ha[k] + (k == 0 ? a.hx : k == 1 ? a.hy : a.hz);
+         f_vjp(m.A, m.B, S, H0, a0, sdir, hb);
+         for (int k = 0; k < 3; ++k) send[k] = hb[k] / mu;
+         ResSpin<R>::store(XB, plane, self, send, e + 2);
+         for (int k = 0; k < 3; ++k) {
+            hb0[k] = send[k] * mu;
+            sb[k] = ub[k] + vb[k] + sdir[k];
+            gv[0] += (double)hb[k] * (double)ex0[k];
+            gv[2 + k] += (double)hb[k];
+         }
+         if (PAIR) pair_grads<R, FMT>(a, i, r.mi, w.S + o, w.S + o + st, w.S + o + 2 * st, hb, s_pair);
+         if (a.uniaxial) gv[1] += ku_grad(m, hb, S);
+      } else {
+         ResSpin<R>::store(XB, plane, self, send, e + 2);
+      }
+      R tg[3] = {0, 0, 0};
+      ok = res_gather<R, FMT, 6>(a, r, XB, plane, self, e + 2, tg[0], tg[1], tg[2]);
+      if (!ok) break;
+      if (on) {
+         const int64_t s = t0 + q;
+         for (int k = 0; k < 3; ++k) l[k] = sb[k] + tg[k] * mu;
+         aniso_vjp(a, m, S, hb0, l);
+         if (s >= 1) l[2] += (R)(2.0 * b.w * (b.mz[s] - b.target[s - 1]) * (double)m.mu_s_muB / b.musum);
+      }
+   }
+   if (!ok) {
+      if ((threadIdx.x & 31) == 0) atomicOr(a.status, 2);
+   } else if (on) {
+      for (int k = 0; k < 3; ++k) b.lam[k * st + i] = l[k];
+   }
+   // every thread of the block: the parameter gradients of the whole run
+   __syncthreads();
+   if (PAIR)
+      for (int k = threadIdx.x; k < 1 + a.M * a.M; k += kResBlock)
+         if (s_pair[k] != 0.0) atomicAdd(b.gp + k, s_pair[k]);
+   grad_add(gv, b.g);
+}
+
+// sums over the warps of nsteps rows into out[0 .. nsteps - 1]
+__global__ void __launch_bounds__(128) mz_rows_kernel(const double* __restrict__ rows, int warps, double* __restrict__ out) {
+   pdl_begin();
+   double v = 0.0;
+   for (int k = threadIdx.x; k < warps; k += blockDim.x) v += rows[(size_t)blockIdx.x * warps + k];
+   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+   __shared__ double red[4];
+   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+   __syncthreads();
+   if (threadIdx.x == 0) out[blockIdx.x] = red[0] + red[1] + red[2] + red[3];
+}
+
+template <typename R> using BackwardFn = void (*)(LLGArgs<R>, AdjBufs<R>, AdjRun<R>, int64_t, int, char*, char*,
+                                                 uint32_t, uint32_t, int, int);
+template <typename R> using RunFn = void (*)(LLGArgs<R>, AdjRun<R>, int, int);
+template <typename R> struct AdjFns {
+   RunFn<R> states, fields;
+   BackwardFn<R> back;
+};
+template <typename R, int FMT> static AdjFns<R> adj_fns_fmt(bool pair) {
+   return {adj_states_kernel<R, FMT>, adj_fields_kernel<R, FMT>,
+           pair ? adj_backward_kernel<R, FMT, true> : adj_backward_kernel<R, FMT, false>};
+}
+template <typename R> static AdjFns<R> adj_fns(int fmt, bool pair) {
+   switch (fmt) {
+      case FMT_ISO_TAB: return adj_fns_fmt<R, FMT_ISO_TAB>(pair);
+      case FMT_ISO_BOND: return adj_fns_fmt<R, FMT_ISO_BOND>(pair);
+      case FMT_VEC_TAB: return adj_fns_fmt<R, FMT_VEC_TAB>(pair);
+      case FMT_VEC_BOND: return adj_fns_fmt<R, FMT_VEC_BOND>(pair);
+      case FMT_DMI_TAB: return adj_fns_fmt<R, FMT_DMI_TAB>(pair);
+      default: return adj_fns_fmt<R, FMT_TENSOR_BOND>(pair);
+   }
+}
+
 template <typename R, int FMT>
 static void adj_step(const LLGArgs<R>& a, const AdjBufs<R>& b, int64_t t, cudaStream_t st) {
    const int g = (b.n + 255) / 256;
@@ -483,6 +687,39 @@ int forward_step(vgpu_ctx* h, LLGArgs<R> a, R* x, R* pb, R* eb, int stride) {
    return cuda_err(h, e, "adjoint forward");
 }
 
+// steps of the backward run whose states and fields are held at once
+constexpr int kAdjRun = 64;
+
+// whether the sweeps (and, given its kernel, the backward run) can run resident
+template <typename R>
+int adjoint_resident(vgpu_ctx* h, const LLGArgs<R>& a, BackwardFn<R> back, bool* use) {
+   *use = false;
+   const ResidentPlan& p = h->sys.res;
+   if (p.K != 1 || passes_asked(h)) return VGPU_OK;
+   bool fits = false;
+   cudaError_t e = path_fits<R>(a, h->sys.fmt, p, h->device, &fits);
+   if (e == cudaSuccess && fits && back) e = one_atom_fits<R>(back, a, h->sys.fmt, p, h->device, &fits);
+   if (e != cudaSuccess) return cuda_err(h, e, "adjoint plan");
+   *use = fits;
+   return VGPU_OK;
+}
+
+// n forward steps of x in one launch; mz_out: also the sum of mu s_z after each
+// (rows: [n][warps] workspace), traj: also the state after each
+template <typename R>
+int forward_run(vgpu_ctx* h, const LLGArgs<R>& a, int n, R* x, R* inc, int stride, R* traj, double* rows,
+                double* mz_out) {
+   ResidentPlan& p = h->sys.res;
+   cudaError_t e = launch_llg_path<R>(a, h->sys.fmt, n, p, h->sys.nslices, x, inc, stride, traj, mz_out ? rows : nullptr,
+                                      h->stream);
+   p.epoch += 2 * (uint32_t)n + 2;
+   if (e == cudaSuccess && mz_out)
+      e = launch_pdl(mz_rows_kernel, dim3(n), dim3(128), 0, h->stream, (const double*)rows, p.grid * (kResBlock / 32),
+                     mz_out);
+   h->kernel_launches += mz_out ? 2 : 1;
+   return cuda_err(h, e, "adjoint forward");
+}
+
 int check_adjoint_ok(vgpu_ctx* h) {
    if (!h) return set_err(nullptr, VGPU_ERR_ARG, "null handle");
    if (!h->sys.uploaded) return set_err(h, VGPU_ERR_STATE, "no system uploaded");
@@ -515,7 +752,15 @@ int mz_trajectory_typed(vgpu_handle h, uint64_t n_steps, double* mz_out) {
       cudaMemcpyAsync(cur.p + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
    cudaMemsetAsync(mz.p, 0, sizeof(double) * (n_steps + 1), h->stream);
    LLGArgs<R> a = make_args<R>(h);
-   for (uint64_t t = 0; t < n_steps; ++t) {
+   bool resident = false;
+   if (int rc = adjoint_resident<R>(h, a, nullptr, &resident)) return rc;
+   DevVec<double> rows;
+   if (resident && (e = rows.alloc((size_t)kAdjRun * S.res.grid * (kResBlock / 32)))) return cuda_err(h, e, "trajectory buffers");
+   for (uint64_t t = 0; resident && t < n_steps; t += kAdjRun) {
+      const int n = (int)std::min<uint64_t>(kAdjRun, n_steps - t);
+      if (int rc = forward_run<R>(h, a, n, cur.p, eb.p, st, nullptr, rows.p, mz.p + t + 1)) return rc;
+   }
+   for (uint64_t t = 0; !resident && t < n_steps; ++t) {
       if (int rc = forward_step<R>(h, a, cur.p, pb.p, eb.p, st)) return rc;
       launch_pdl(mz_kernel<R>, dim3((S.n + 255) / 256), dim3(256), 0, h->stream, (int)S.n,
                  (const R*)(cur.p + 2 * (size_t)st), (const int*)S.mat, (const MatParams<R>*)S.mp,
@@ -578,7 +823,24 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    R* cur = seg.p;  // first slot doubles as the running state
    for (int q = 0; q < 3; ++q)
       cudaMemcpyAsync(cur + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
-   for (int64_t t = 0; t < N; ++t) {
+   const AdjFns<R> fns = adj_fns<R>(S.fmt, pair_out != nullptr);
+   bool resident = false;
+   if ((rc = adjoint_resident<R>(h, a, fns.back, &resident))) return rc;
+   const int run = (int)std::min<int64_t>(C, kAdjRun);
+   DevVec<R> held;       // states and fields of a run: s', H(s) and H(s') exchange, f, |v|
+   DevVec<double> rows;
+   if (resident && ((e = held.alloc((4 * v3 + st) * run)) ||
+                    (e = rows.alloc((size_t)kAdjRun * S.res.grid * (kResBlock / 32))))) {
+      cudaGetLastError();
+      resident = false;  // without the room for it, launch by launch
+   }
+   for (int64_t t = 0; resident && t < N;) {
+      if (t % C == 0) cudaMemcpyAsync(cp.p + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+      const int n1 = (int)std::min<int64_t>(std::min<int64_t>(kAdjRun, C - t % C), N - t);
+      if ((rc = forward_run<R>(h, a, n1, cur, eb.p, st, nullptr, rows.p, mz.p + t + 1))) return rc;
+      t += n1;
+   }
+   for (int64_t t = 0; !resident && t < N; ++t) {
       if (t % C == 0) cudaMemcpyAsync(cp.p + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
       if ((rc = forward_step<R>(h, a, cur, pb.p, eb.p, st))) return rc;
       launch_pdl(mz_kernel<R>, dim3((n + 255) / 256), dim3(256), 0, h->stream, (int)n,
@@ -611,6 +873,39 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    for (int64_t c = ncp - 1; c >= 0; --c) {
       const int64_t t0 = c * C, t1 = std::min(t0 + C, N);
       cudaMemcpyAsync(seg.p, cp.p + v3 * c, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+      if (resident) {
+         // the segment's states, then its steps backwards a run at a time
+         if (t1 - t0 > 1) {
+            cudaMemcpyAsync(pb.p, seg.p, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+            for (int64_t t = t0; t < t1 - 1;) {
+               const int n1 = (int)std::min<int64_t>(kGridSteps, t1 - 1 - t);
+               if ((rc = forward_run<R>(h, a, n1, pb.p, eb.p, st, seg.p + v3 * (t - t0 + 1), nullptr, nullptr))) return rc;
+               t += n1;
+            }
+         }
+         for (int64_t hi = t1; hi > t0;) {
+            const int n1 = (int)std::min<int64_t>(run, hi - t0);
+            const int64_t lo = hi - n1;
+            AdjRun<R> w;
+            w.S = seg.p + v3 * (lo - t0);
+            w.sp = held.p; w.ex0 = held.p + v3 * run; w.f0 = held.p + 2 * v3 * run; w.ex1 = held.p + 3 * v3 * run;
+            w.nv = held.p + 4 * v3 * run;
+            ResidentPlan& p = S.res;
+            char* X = static_cast<char*>(p.spins);
+            const uint32_t plane = 16u * (uint32_t)(p.grid * kResBlock);
+            const dim3 g((n + 255) / 256, n1), bl(256);
+            e = launch_pdl(fns.states, g, bl, 0, h->stream, a, w, n, st);
+            if (e == cudaSuccess) e = launch_pdl(fns.fields, g, bl, 0, h->stream, a, w, n, st);
+            if (e == cudaSuccess)
+               e = launch_one_atom<R>(fns.back, a, S.fmt, p, h->stream, LLGArgs<R>(a), AdjBufs<R>(b), AdjRun<R>(w), lo, n1, X,
+                                      X + (size_t)ResSpin<R>::kWords * plane, plane, p.epoch, S.nslices, p.word_bytes);
+            if (e != cudaSuccess) return cuda_err(h, e, "adjoint backward");
+            p.epoch += 2 * (uint32_t)n1 + 2;
+            h->kernel_launches += 3;
+            hi = lo;
+         }
+         continue;
+      }
       for (int64_t t = t0; t < t1 - 1; ++t) {
          R* nxt = seg.p + v3 * (t - t0 + 1);
          cudaMemcpyAsync(nxt, seg.p + v3 * (t - t0), sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
@@ -624,9 +919,12 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
       if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(h, e, "adjoint backward");
    }
    std::vector<double> gh(5 + np);
+   int status = 0;
    e = cudaMemcpyAsync(gh.data(), g.p, sizeof(double) * gh.size(), cudaMemcpyDeviceToHost, h->stream);
+   if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint result");
+   if (status & 2) return h->check_status();  // a resident wait ran out
    *loss_out = loss;
    for (int k = 0; k < 5; ++k) grad_out[k] = gh[k];
    if (pair_out)

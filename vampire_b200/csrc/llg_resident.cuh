@@ -252,6 +252,54 @@ template <typename R, int FMT, int VAR, int K> constexpr int res_min_blocks() {
    return 6;
 }
 
+// What a block of kResBlock threads with one atom each keeps in shared memory,
+// filled by the constructor (ends with a block barrier).
+template <typename R, int FMT> struct ResBlockData {
+   int o0;
+   bool one_j;
+   const int* off;
+   const MatParams<R>* mats;
+   const float4* dict;
+   const uint32_t* words;
+   __device__ ResBlockData(const LLGArgs<R>& a, unsigned char* smem, int nslices, int word_bytes) {
+      constexpr bool WORDS = res_words<R, FMT>();
+      const int dict_bytes = WORDS && FMT == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
+      const ResLayout lay = res_layout<R>(1, a.M, dict_bytes, word_bytes);
+      int* s_off = reinterpret_cast<int*>(smem);
+      MatParams<R>* s_mat = reinterpret_cast<MatParams<R>*>(smem + lay.mats);
+      float4* s_dict = reinterpret_cast<float4*>(smem + lay.dict);
+      uint32_t* s_words = reinterpret_cast<uint32_t*>(smem + lay.words);
+      const int tid = threadIdx.x, s0 = blockIdx.x * kResSlices, ns = min(kResSlices, nslices - s0);
+      o0 = __ldg(a.slice_off + s0);
+      one_j = a.M == 1 || (a.sys_off && a.m_per_sys == 1);
+      if (WORDS) {
+         const int nw = __ldg(a.slice_off + s0 + ns) - o0;
+         const uint32_t* src = FMT == FMT_ISO_TAB ? reinterpret_cast<const uint32_t*>(a.col) : a.crec;
+         for (int q = tid; q < nw; q += kResBlock) s_words[q] = __ldg(src + o0 + q);
+         for (int q = tid; q < dict_bytes / 16; q += kResBlock) s_dict[q] = __ldg(a.cdict + q);
+      }
+      for (int q = tid; q <= kResSlices; q += kResBlock) s_off[q] = __ldg(a.slice_off + s0 + min(q, ns)) - o0;
+      if (a.M <= kResMaxMat) {
+         const int nw = a.M * (int)(sizeof(MatParams<R>) / 4);
+         for (int q = tid; q < nw; q += kResBlock)
+            reinterpret_cast<uint32_t*>(s_mat)[q] = __ldg(reinterpret_cast<const uint32_t*>(a.mp) + q);
+      }
+      off = s_off;
+      mats = a.M <= kResMaxMat ? s_mat : a.mp;
+      dict = s_dict;
+      words = s_words;
+      __syncthreads();
+   }
+   __device__ const MatParams<R>& mat(const LLGArgs<R>&, int mi) const { return mats[mi]; }
+   // the row of this thread's atom (i: the atom, 0 for a thread past the last)
+   __device__ ResRow<R> row(const LLGArgs<R>& a, int i) const {
+      const int sl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+      const int mi = a.mat ? __ldg(a.mat + i) : 0;
+      return ResRow<R>{o0 + off[sl] + lane, (off[sl + 1] - off[sl]) >> 5, words + off[sl] + lane, mi, one_j,
+                       FMT == FMT_ISO_TAB ? __ldg(a.jtab + mi * a.M + mi) : (R)0, dict};
+   }
+};
+
 // RF for formats other than FMT_ISO_TAB: the common facts written in -- thermal
 // noise from Philox, one system, no field per material, no host dipole field, a
 // scalar coupling table in the dictionary (FP32 DMI)
@@ -434,6 +482,69 @@ __global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR, K>()))
          a.bx[i] = P[k][0]; a.by[i] = P[k][1]; a.bz[i] = P[k][2];
       }
    }
+}
+
+// Deterministic Heun steps that also leave a trace, for the adjoint: the state
+// after each step (traj, 3 stride values a step) or each warp's sum of mu s_z
+// (mz, [nsteps][warps]), in FP64.  Starts from, and ends in, the state x of 3
+// stride values; inc (3 stride) takes the predictor increments.  The step is
+// llg_resident_kernel's with one atom per thread.
+template <typename R, int FMT>
+__global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR_HEUN_EXT, 1>()))
+    llg_path_kernel(const LLGArgs<R> in, int nsteps, char* XA, char* XB, uint32_t plane, uint32_t epoch0, int nslices,
+                    int word_bytes, R* x, R* inc, int stride, R* traj, double* mz) {
+   LLGArgs<R> a = in;
+   a.thermal = 0;
+   a.ex = inc; a.ey = inc + stride; a.ez = inc + 2 * stride;
+   extern __shared__ __align__(16) unsigned char res_smem[];
+   const ResBlockData<R, FMT> d(a, res_smem, nslices, word_bytes);
+   const int i = blockIdx.x * kResBlock + threadIdx.x;
+   const bool on = i < a.n;
+   const uint32_t self = 16u * (uint32_t)i;
+   R S0[3] = {1, 0, 0}, P[3] = {1, 0, 0}, E[3] = {0, 0, 0};
+   const ResRow<R> r = d.row(a, on ? i : 0);
+   if (on) {
+      for (int c = 0; c < 3; ++c) S0[c] = x[(size_t)c * stride + i];
+      external_field<R>(a, i, d.mat(a, r.mi), false, E);
+   }
+   ResSpin<R>::store(XA, plane, self, S0, epoch0);
+   auto field = [&](const char* X, uint32_t t, const R S[3], R H[3]) -> bool {
+      R hx = 0, hy = 0, hz = 0;
+      if (!res_gather<R, FMT, 6>(a, r, X, plane, self, t, hx, hy, hz)) return false;
+      site_field<R, 0, false>(a, i, d.mat(a, r.mi), nullptr, nullptr, nullptr, S, hx, hy, hz, H);
+      H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
+      return true;
+   };
+   bool ok = true;
+   for (int s = 0; s < nsteps && ok; ++s) {
+      const uint32_t e = epoch0 + 2 * (uint32_t)s;
+      R H[3], o[3];
+      ok = field(XA, e, S0, H);
+      if (!ok) break;
+      if (on) llg_predict<R>(a, i, d.mat(a, r.mi), S0, H, P);
+      ResSpin<R>::store(XB, plane, self, P, e + 1);
+      ok = field(XB, e + 1, P, H);
+      if (!ok) break;
+      if (on) {
+         llg_correct<R>(a, i, d.mat(a, r.mi), S0, P, H, o);
+         S0[0] = o[0]; S0[1] = o[1]; S0[2] = o[2];
+      }
+      ResSpin<R>::store(XA, plane, self, S0, e + 2);
+      if (traj && on)
+         for (int c = 0; c < 3; ++c) traj[(3 * (size_t)s + c) * stride + i] = S0[c];
+      if (mz) {
+         double v = on ? (double)S0[2] * (double)d.mat(a, r.mi).mu_s_muB : 0.0;
+         for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+         const int warps = gridDim.x * (kResBlock / 32);
+         if ((threadIdx.x & 31) == 0) mz[(size_t)s * warps + (i >> 5)] = v;
+      }
+   }
+   if (!ok) {
+      if ((threadIdx.x & 31) == 0) atomicOr(a.status, 2);
+      return;
+   }
+   if (on)
+      for (int c = 0; c < 3; ++c) x[(size_t)c * stride + i] = S0[c];
 }
 
 // ---------------------------------------------------------------------------
@@ -840,6 +951,64 @@ cudaError_t resident_capacity(const LLGArgs<R>& a, int fmt, int var, const Resid
    }
    *blocks = least;
    return cudaSuccess;
+}
+
+// cooperative launch of a kernel of one atom per thread (p.K == 1)
+template <typename R, typename... Args>
+inline cudaError_t launch_one_atom(void (*f)(Args...), const LLGArgs<R>& a, int fmt, const ResidentPlan& p,
+                                   cudaStream_t st, Args... args) {
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(p.grid);
+   cfg.blockDim = dim3(kResBlock);
+   cfg.dynamicSmemBytes = (size_t)resident_smem<R>(a, fmt, p);
+   cfg.stream = st;
+   cudaLaunchAttribute attr[1];
+   attr[0].id = cudaLaunchAttributeCooperative;
+   attr[0].val.cooperative = 1;
+   cfg.attrs = attr;
+   cfg.numAttrs = 1;
+   return cudaLaunchKernelEx(&cfg, f, args...);
+}
+
+// whether a kernel of one atom per thread is resident with the plan's grid
+template <typename R, typename F>
+inline cudaError_t one_atom_fits(F* f, const LLGArgs<R>& a, int fmt, const ResidentPlan& p, int device, bool* fits) {
+   *fits = false;
+   const int smem = resident_smem<R>(a, fmt, p);
+   int sms = 0, per_sm = 0;
+   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kResBlock, smem);
+   *fits = per_sm * sms >= p.grid;
+   return e;
+}
+
+template <typename R> using PathFn = void (*)(LLGArgs<R>, int, char*, char*, uint32_t, uint32_t, int, int, R*, R*, int,
+                                             R*, double*);
+template <typename R> inline PathFn<R> path_fn(int fmt) {
+   switch (fmt) {
+      case FMT_ISO_TAB: return llg_path_kernel<R, FMT_ISO_TAB>;
+      case FMT_ISO_BOND: return llg_path_kernel<R, FMT_ISO_BOND>;
+      case FMT_VEC_TAB: return llg_path_kernel<R, FMT_VEC_TAB>;
+      case FMT_VEC_BOND: return llg_path_kernel<R, FMT_VEC_BOND>;
+      case FMT_DMI_TAB: return llg_path_kernel<R, FMT_DMI_TAB>;
+      default: return llg_path_kernel<R, FMT_TENSOR_BOND>;
+   }
+}
+
+template <typename R>
+cudaError_t path_fits(const LLGArgs<R>& a, int fmt, const ResidentPlan& p, int device, bool* fits) {
+   return one_atom_fits<R>(path_fn<R>(fmt), a, fmt, p, device, fits);
+}
+
+template <typename R>
+cudaError_t launch_llg_path(const LLGArgs<R>& a, int fmt, int nsteps, const ResidentPlan& p, int nslices, R* x, R* inc,
+                            int stride, R* traj, double* mz, cudaStream_t st) {
+   char* X = static_cast<char*>(p.spins);
+   const uint32_t plane = 16u * (uint32_t)(p.grid * kResBlock);
+   return launch_one_atom<R>(path_fn<R>(fmt), a, fmt, p, st, LLGArgs<R>(a), nsteps, X,
+                             X + (size_t)ResSpin<R>::kWords * plane, plane, p.epoch, nslices, p.word_bytes, x, inc,
+                             stride, traj, mz);
 }
 
 template <typename R>

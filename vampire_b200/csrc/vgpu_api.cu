@@ -693,17 +693,14 @@ static int run_pass(vgpu_ctx* h, int mode, bool staged, int integrator = INTEG_H
 }
 
 // How the next steps run.  Resident forms need a plan that fits for this
-// variant and nothing that asks for the separate passes (per-launch timing, a
-// pass option set by the caller, a shard, a second neighbour list).
+// variant and nothing that asks for the separate passes (passes_asked).
 enum StepMode { STEP_PASSES, STEP_GRID, STEP_CLUSTER };
 
 template <typename R>
 static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
    SysDev& S = h->sys;
    *mode = STEP_PASSES;
-   if (h->prof_on || S.n_owned != S.n || S.bq_off || h->staged >= 0 || h->stage_sl > 0 || h->stage_nbuf > 0 ||
-       h->compact >= 0 || h->window >= 0 || h->stage_warps >= 0 || h->stage_wait_test)
-      return VGPU_OK;
+   if (passes_asked(h)) return VGPU_OK;
    *var = integrator == INTEG_MIDPOINT ? VAR_MIDPOINT : S.aniso_ext ? VAR_HEUN_EXT : VAR_HEUN;
    if (S.one.size) {
       if (S.one.cap_var != *var) {

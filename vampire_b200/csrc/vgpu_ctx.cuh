@@ -162,3 +162,12 @@ struct vgpu_ctx {
 namespace vgpu {
 template <typename R> LLGArgs<R> make_args(vgpu_ctx* h);
 }
+
+namespace vgpu {
+// something asks for one launch per pass: per-launch timing, a pass option set
+// by the caller, a shard, a second neighbour list
+inline bool passes_asked(const vgpu_ctx* h) {
+   return h->prof_on || h->sys.n_owned != h->sys.n || h->sys.bq_off || h->staged >= 0 || h->stage_sl > 0 ||
+          h->stage_nbuf > 0 || h->compact >= 0 || h->window >= 0 || h->stage_warps >= 0 || h->stage_wait_test;
+}
+}  // namespace vgpu

@@ -199,6 +199,14 @@ template <typename R>
 cudaError_t launch_llg_resident(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ResidentPlan& p, int nslices,
                                 cudaStream_t st);
 
+// deterministic Heun steps of the state x with a trace of the states or of the
+// warps' sums of mu s_z (llg_path_kernel; plans of one atom per thread)
+template <typename R>
+cudaError_t path_fits(const LLGArgs<R>& a, int fmt, const ResidentPlan& p, int device, bool* fits);
+template <typename R>
+cudaError_t launch_llg_path(const LLGArgs<R>& a, int fmt, int nsteps, const ResidentPlan& p, int nslices, R* x, R* inc,
+                            int stride, R* traj, double* mz, cudaStream_t st);
+
 // write the Philox thermal Gaussians of step a.step into a.fx/fy/fz
 template <typename R>
 cudaError_t launch_thermal_noise(const LLGArgs<R>& a, cudaStream_t st);
@@ -209,6 +217,20 @@ cudaError_t launch_thermal_noise(const LLGArgs<R>& a, cudaStream_t st);
 // bodies must not instantiate their own copies.
 extern template cudaError_t launch_llg_pass<float>(const LLGArgs<float>&, int, int, int, cudaStream_t);
 extern template cudaError_t launch_llg_pass<double>(const LLGArgs<double>&, int, int, int, cudaStream_t);
+#define VGPU_EXTERN(R)                                                                                        \
+   extern template cudaError_t resident_capacity<R>(const LLGArgs<R>&, int, int, const ResidentPlan&, int, int*); \
+   extern template cudaError_t launch_resident_check<R>(const LLGArgs<R>&, int*, cudaStream_t);                \
+   extern template cudaError_t launch_llg_resident<R>(const LLGArgs<R>&, int, int, int, const ResidentPlan&, int, \
+                                                      cudaStream_t);                                          \
+   extern template cudaError_t cluster_capacity<R>(const LLGArgs<R>&, int, int, const ClusterShape&, int*);    \
+   extern template cudaError_t launch_llg_cluster<R>(const LLGArgs<R>&, int, int, int, const ClusterShape&,    \
+                                                     cudaStream_t);                                           \
+   extern template cudaError_t path_fits<R>(const LLGArgs<R>&, int, const ResidentPlan&, int, bool*);          \
+   extern template cudaError_t launch_llg_path<R>(const LLGArgs<R>&, int, int, const ResidentPlan&, int, R*, R*, int, \
+                                                  R*, double*, cudaStream_t);
+VGPU_EXTERN(float)
+VGPU_EXTERN(double)
+#undef VGPU_EXTERN
 extern template cudaError_t launch_thermal_noise<float>(const LLGArgs<float>&, cudaStream_t);
 extern template cudaError_t launch_thermal_noise<double>(const LLGArgs<double>&, cudaStream_t);
 

@@ -62,3 +62,24 @@ def test_alloy(vgpu_lib, prec, pairs):
     s = S.config_fcc_tensor(5, temperature=0.0)
     s.params.H_applied = 0.3
     _compare(s, prec, 30, 0, pairs)
+
+
+def test_workspace_between_calls(vgpu_lib):
+    """One handle, calls of different length and checkpointing in turn: each
+    equals the same call on a handle of its own."""
+    from vampire_b200 import adjoint as A
+    from vampire_b200 import vgpu as V
+    s = A.system(11.2e-21, 6.69e-24, (0.1, 0.0, 0.4), 6)
+
+    def grad(sim, steps, every):
+        target = np.full(steps, 0.9)
+        g, loss = np.zeros(5), C.c_double()
+        sim._check(V.lib().vgpu_adjoint_llg(sim.handle, C.c_uint64(steps), target.ctypes.data_as(V._D),
+                                            C.c_double(1e-16), C.c_int32(every), C.byref(loss), g.ctypes.data_as(V._D)))
+        return np.r_[loss.value, g]
+
+    with V.Simulation(s, precision="fp64") as sim:
+        for steps, every in ((10, 0), (90, 7), (3, 0), (150, 0), (90, 90)):
+            with V.Simulation(s, precision="fp64") as fresh:
+                want = grad(fresh, steps, every)
+            assert np.abs(grad(sim, steps, every) - want).max() <= 1e-12 * np.abs(want).max()

@@ -38,6 +38,8 @@
 #include <cstring>
 #include <vector>
 
+#include <type_traits>
+
 #include "llg_resident.cuh"
 #include "vgpu_ctx.cuh"
 
@@ -503,18 +505,33 @@ __global__ void __launch_bounds__(kResBlock, sizeof(R) == 8 ? 3 : 4)
    if (on)
       for (int k = 0; k < 3; ++k) l[k] = b.lam[k * st + i];
    bool ok = true;
+   // the own data of a step; in FP32 read one step ahead, so that the loads lie
+   // under the waits (FP64 has no registers to hold them)
+   constexpr bool AHEAD = sizeof(R) == 4;
+   R own[16];
+   auto fetch = [&](int q) {
+      const size_t o = 3 * (size_t)st * q + i;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+         const size_t at = o + (size_t)k * st;
+         own[k] = __ldg(w.S + at); own[3 + k] = __ldg(w.sp + at); own[6 + k] = __ldg(w.ex0 + at);
+         own[9 + k] = __ldg(w.ex1 + at); own[12 + k] = __ldg(w.f0 + at);
+      }
+      own[15] = __ldg(w.nv + (size_t)st * q + i);
+   };
+   if (on && AHEAD) fetch(nsteps - 1);
    for (int q = nsteps - 1; q >= 0; --q) {
       const size_t o = 3 * (size_t)st * q;
       const uint32_t e = epoch0 + 2 * (uint32_t)(nsteps - 1 - q);
       R S[3] = {1, 0, 0}, Sp[3] = {1, 0, 0}, ex0[3] = {0, 0, 0}, ex1[3] = {0, 0, 0}, ub[3] = {0, 0, 0},
         spb[3] = {0, 0, 0}, hb1[3] = {0, 0, 0}, send[3] = {0, 0, 0}, nv = 1, sb[3] = {0, 0, 0}, hb0[3] = {0, 0, 0};
       if (on) {
+         if (!AHEAD) fetch(q);
          R f0[3];
          for (int k = 0; k < 3; ++k) {
-            const size_t at = o + (size_t)k * st + i;
-            S[k] = w.S[at]; Sp[k] = w.sp[at]; ex0[k] = w.ex0[at]; ex1[k] = w.ex1[at]; f0[k] = w.f0[at];
+            S[k] = own[k]; Sp[k] = own[3 + k]; ex0[k] = own[6 + k]; ex1[k] = own[9 + k]; f0[k] = own[12 + k];
          }
-         nv = w.nv[(size_t)st * q + i];
+         nv = own[15];
          R Ha[3], f1[3], u[3];
          aniso_h(a, m, Sp, Ha);
          const R H1[3] = {ex1[0] + Ha[0] + a.hx, ex1[1] + Ha[1] + a.hy, ex1[2] + Ha[2] + a.hz};
@@ -529,6 +546,7 @@ __global__ void __launch_bounds__(kResBlock, sizeof(R) == 8 ? 3 : 4)
          const R imu = (R)1 / m.mu_s_muB;  // Hbar / mu_s for the transposed gather
          for (int k = 0; k < 3; ++k) send[k] = hb[k] * imu;
          ResSpin<R>::store(XA, plane, self, send, e + 1);
+         if (AHEAD && q > 0) fetch(q - 1);
          for (int k = 0; k < 3; ++k) {
             hb1[k] = send[k] * mu;
             gv[0] += (double)hb[k] * (double)ex1[k];
@@ -689,6 +707,10 @@ int forward_step(vgpu_ctx* h, LLGArgs<R> a, R* x, R* pb, R* eb, int stride) {
 
 // steps of the backward run whose states and fields are held at once
 constexpr int kAdjRun = 64;
+// workspace that a handle keeps between calls (allocating and freeing it took 5
+// to 15 ms of a 15 ms gradient): 1 GiB of the 180, the states of 2,500 steps of
+// 32,768 spins
+constexpr size_t kAdjKeepBytes = (size_t)1 << 30;
 
 // whether the sweeps (and, given its kernel, the backward run) can run resident
 template <typename R>
@@ -778,15 +800,14 @@ int mz_trajectory_typed(vgpu_handle h, uint64_t n_steps, double* mz_out) {
 // the couplings must be reciprocal in SI units for the transposed gather
 template <typename R>
 int check_reciprocal(vgpu_ctx* h) {
-   int* bad = nullptr;
-   cudaError_t e = cudaMalloc(&bad, sizeof(int));
-   if (e != cudaSuccess) return cuda_err(h, e, "adjoint check");
+   SysDev& S = h->sys;
+   if (!S.adj_bad) S.adj_bad = (int*)h->alloc(sizeof(int));
+   if (!S.adj_bad) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the adjoint check");
    int hb = 0;
-   e = cudaMemsetAsync(bad, 0, sizeof(int), h->stream);
-   if (e == cudaSuccess) e = launch_reciprocal<R>(h->sys.fmt, make_args<R>(h), bad, h->stream);
-   if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+   cudaError_t e = cudaMemsetAsync(S.adj_bad, 0, sizeof(int), h->stream);
+   if (e == cudaSuccess) e = launch_reciprocal<R>(S.fmt, make_args<R>(h), S.adj_bad, h->stream);
+   if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, S.adj_bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-   cudaFree(bad);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint check");
    h->kernel_launches++;
    if (hb)
@@ -804,58 +825,104 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    SysDev& S = h->sys;
    const int n = S.n, st = S.n_alloc;
    const int64_t N = (int64_t)n_steps;
-   const int64_t C = every > 0 ? every : (int64_t)std::ceil(std::sqrt((double)N));
-   const int64_t ncp = (N + C - 1) / C;
    const size_t v3 = 3 * (size_t)st;
    const int np = 1 + M * M;
-   DevVec<R> cp, seg, pb, eb, work;
-   DevVec<double> mz, tg, g;
-   cudaError_t e;
-   if ((e = cp.alloc(v3 * ncp)) || (e = seg.alloc(v3 * (C + 1))) || (e = pb.alloc(v3)) || (e = eb.alloc(v3)) ||
-       (e = mz.alloc(N + 1)) || (e = tg.alloc(N)) || (e = g.alloc(5 + np)) || (e = work.alloc(v3 * 10 + st)))
-      return cuda_err(h, e, "adjoint buffers");
-   cudaMemcpyAsync(tg.p, target, sizeof(double) * N, cudaMemcpyHostToDevice, h->stream);
-   cudaMemsetAsync(mz.p, 0, sizeof(double) * (N + 1), h->stream);
-   cudaMemsetAsync(g.p, 0, sizeof(double) * (5 + np), h->stream);
    LLGArgs<R> a = make_args<R>(h);
    a.thermal = 0;
-   // forward from the current spins (left untouched), checkpoint every C steps
-   R* cur = seg.p;  // first slot doubles as the running state
-   for (int q = 0; q < 3; ++q)
-      cudaMemcpyAsync(cur + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
    const AdjFns<R> fns = adj_fns<R>(S.fmt, pair_out != nullptr);
    bool resident = false;
    if ((rc = adjoint_resident<R>(h, a, fns.back, &resident))) return rc;
-   const int run = (int)std::min<int64_t>(C, kAdjRun);
-   DevVec<R> held;       // states and fields of a run: s', H(s) and H(s') exchange, f, |v|
-   DevVec<double> rows;
-   if (resident && ((e = held.alloc((4 * v3 + st) * run)) ||
-                    (e = rows.alloc((size_t)kAdjRun * S.res.grid * (kResBlock / 32))))) {
-      cudaGetLastError();
-      resident = false;  // without the room for it, launch by launch
+   // Checkpoints every C steps (default ceil(sqrt(N))), their segments recomputed;
+   // with resident threads and the default, all states are kept instead where
+   // the workspace stays within what is kept between calls.
+   int64_t C = 0, ncp = 0;
+   int run = 0;
+   bool all = resident && every <= 0;
+   struct { R *cp, *seg, *pb, *eb, *work, *held; double *mz, *tg, *g, *rows; } ws;
+   for (;;) {
+      C = all ? N : every > 0 ? every : (int64_t)std::ceil(std::sqrt((double)N));
+      ncp = all ? 0 : (N + C - 1) / C;
+      run = (int)std::min<int64_t>(C, kAdjRun);
+      size_t bytes = 0;
+      char* base = nullptr;
+      auto take = [&](auto*& q, size_t count) {
+         q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(base + bytes);
+         bytes += (count * sizeof(*q) + 255) & ~(size_t)255;
+      };
+      auto layout = [&](void* at) {
+         base = (char*)at;
+         bytes = 0;
+         take(ws.cp, v3 * ncp); take(ws.seg, v3 * (C + 1)); take(ws.pb, v3); take(ws.eb, v3);
+         take(ws.work, resident ? v3 : v3 * 10 + st);
+         take(ws.held, resident ? (4 * v3 + st) * run : 0);
+         take(ws.mz, N + 1); take(ws.tg, N); take(ws.g, 5 + np);
+         take(ws.rows, resident ? (size_t)kAdjRun * S.res.grid * (kResBlock / 32) : 0);
+      };
+      layout(nullptr);
+      if (all && bytes > kAdjKeepBytes) {
+         all = false;
+         continue;
+      }
+      if (S.adj_ws_bytes < bytes) {
+         h->release(S.adj_ws);
+         S.adj_ws = h->alloc(bytes);
+         S.adj_ws_bytes = S.adj_ws ? bytes : 0;
+      }
+      if (S.adj_ws) {
+         layout(S.adj_ws);
+         break;
+      }
+      // less, where there is not the room: checkpoints, then launch by launch
+      if (all) all = false;
+      else if (resident) resident = false;
+      else return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the adjoint buffers (%zu bytes)", bytes);
+   }
+   struct Release {  // a workspace beyond the limit goes back when the call is done
+      vgpu_ctx* h;
+      ~Release() {
+         if (h->sys.adj_ws_bytes <= kAdjKeepBytes) return;
+         cudaStreamSynchronize(h->stream);
+         h->release(h->sys.adj_ws);
+         h->sys.adj_ws = nullptr;
+         h->sys.adj_ws_bytes = 0;
+      }
+   } release{h};
+   cudaError_t e;
+   cudaMemcpyAsync(ws.tg, target, sizeof(double) * N, cudaMemcpyHostToDevice, h->stream);
+   cudaMemsetAsync(ws.mz, 0, sizeof(double) * (N + 1), h->stream);
+   cudaMemsetAsync(ws.g, 0, sizeof(double) * (5 + np), h->stream);
+   // forward from the current spins (left untouched), checkpoint every C steps
+   R* cur = all ? ws.pb : ws.seg;  // the running state (checkpoints: in the first segment slot)
+   for (int q = 0; q < 3; ++q) {
+      cudaMemcpyAsync(cur + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
+      if (all)
+         cudaMemcpyAsync(ws.seg + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
    }
    for (int64_t t = 0; resident && t < N;) {
-      if (t % C == 0) cudaMemcpyAsync(cp.p + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+      if (!all && t % C == 0)
+         cudaMemcpyAsync(ws.cp + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
       const int n1 = (int)std::min<int64_t>(std::min<int64_t>(kAdjRun, C - t % C), N - t);
-      if ((rc = forward_run<R>(h, a, n1, cur, eb.p, st, nullptr, rows.p, mz.p + t + 1))) return rc;
+      if ((rc = forward_run<R>(h, a, n1, cur, ws.eb, st, all ? ws.seg + v3 * (t + 1) : nullptr, ws.rows, ws.mz + t + 1)))
+         return rc;
       t += n1;
    }
    for (int64_t t = 0; !resident && t < N; ++t) {
-      if (t % C == 0) cudaMemcpyAsync(cp.p + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
-      if ((rc = forward_step<R>(h, a, cur, pb.p, eb.p, st))) return rc;
+      if (t % C == 0)
+         cudaMemcpyAsync(ws.cp + v3 * (t / C), cur, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+      if ((rc = forward_step<R>(h, a, cur, ws.pb, ws.eb, st))) return rc;
       launch_pdl(mz_kernel<R>, dim3((n + 255) / 256), dim3(256), 0, h->stream, (int)n,
                  (const R*)(cur + 2 * (size_t)st), (const int*)S.mat, (const MatParams<R>*)S.mp,
-                 (double*)(mz.p + t + 1));
+                 (double*)(ws.mz + t + 1));
    }
    // loss on the host from m_z(t)
    std::vector<double> mzh(N + 1);
-   e = cudaMemcpyAsync(mzh.data(), mz.p, sizeof(double) * (N + 1), cudaMemcpyDeviceToHost, h->stream);
+   e = cudaMemcpyAsync(mzh.data(), ws.mz, sizeof(double) * (N + 1), cudaMemcpyDeviceToHost, h->stream);
    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint forward");
    const double musum = moment_sum(h);
    // m_z was summed unnormalised: scale the device copy once
    for (int64_t t = 0; t <= N; ++t) mzh[t] /= musum;
-   cudaMemcpyAsync(mz.p, mzh.data(), sizeof(double) * (N + 1), cudaMemcpyHostToDevice, h->stream);
+   cudaMemcpyAsync(ws.mz, mzh.data(), sizeof(double) * (N + 1), cudaMemcpyHostToDevice, h->stream);
    double loss = 0.0;
    for (int64_t t = 1; t <= N; ++t) {
       const double r = mzh[t] - target[t - 1];
@@ -863,23 +930,26 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    }
    AdjBufs<R> b;
    std::memset(&b, 0, sizeof b);
-   R* wk = work.p;
-   b.sp = wk; b.ex0 = wk + v3; b.ex1 = wk + 2 * v3; b.f0 = wk + 3 * v3; b.ub = wk + 4 * v3;
-   b.spb = wk + 5 * v3; b.sb = wk + 6 * v3; b.Hb0 = wk + 7 * v3; b.Hb1 = wk + 8 * v3; b.lam = wk + 9 * v3;
-   b.nv = wk + 10 * v3;
-   b.g = g.p; b.mz = mz.p; b.target = tg.p; b.w = w; b.musum = musum; b.n = n; b.stride = st;
-   b.gp = pair_out ? g.p + 5 : nullptr;
+   R* wk = ws.work;
+   b.lam = wk;
+   if (!resident) {
+      b.sp = wk + v3; b.ex0 = wk + 2 * v3; b.ex1 = wk + 3 * v3; b.f0 = wk + 4 * v3; b.ub = wk + 5 * v3;
+      b.spb = wk + 6 * v3; b.sb = wk + 7 * v3; b.Hb0 = wk + 8 * v3; b.Hb1 = wk + 9 * v3;
+      b.nv = wk + 10 * v3;
+   }
+   b.g = ws.g; b.mz = ws.mz; b.target = ws.tg; b.w = w; b.musum = musum; b.n = n; b.stride = st;
+   b.gp = pair_out ? ws.g + 5 : nullptr;
    adj_lambda_init<R><<<(n + 255) / 256, 256, 0, h->stream>>>(a, b, N);
-   for (int64_t c = ncp - 1; c >= 0; --c) {
+   for (int64_t c = all ? 0 : ncp - 1; c >= 0; --c) {
       const int64_t t0 = c * C, t1 = std::min(t0 + C, N);
-      cudaMemcpyAsync(seg.p, cp.p + v3 * c, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+      if (!all) cudaMemcpyAsync(ws.seg, ws.cp + v3 * c, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
       if (resident) {
          // the segment's states, then its steps backwards a run at a time
-         if (t1 - t0 > 1) {
-            cudaMemcpyAsync(pb.p, seg.p, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+         if (!all && t1 - t0 > 1) {
+            cudaMemcpyAsync(ws.pb, ws.seg, sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
             for (int64_t t = t0; t < t1 - 1;) {
                const int n1 = (int)std::min<int64_t>(kGridSteps, t1 - 1 - t);
-               if ((rc = forward_run<R>(h, a, n1, pb.p, eb.p, st, seg.p + v3 * (t - t0 + 1), nullptr, nullptr))) return rc;
+               if ((rc = forward_run<R>(h, a, n1, ws.pb, ws.eb, st, ws.seg + v3 * (t - t0 + 1), nullptr, nullptr))) return rc;
                t += n1;
             }
          }
@@ -887,9 +957,9 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
             const int n1 = (int)std::min<int64_t>(run, hi - t0);
             const int64_t lo = hi - n1;
             AdjRun<R> w;
-            w.S = seg.p + v3 * (lo - t0);
-            w.sp = held.p; w.ex0 = held.p + v3 * run; w.f0 = held.p + 2 * v3 * run; w.ex1 = held.p + 3 * v3 * run;
-            w.nv = held.p + 4 * v3 * run;
+            w.S = ws.seg + v3 * (lo - t0);
+            w.sp = ws.held; w.ex0 = ws.held + v3 * run; w.f0 = ws.held + 2 * v3 * run; w.ex1 = ws.held + 3 * v3 * run;
+            w.nv = ws.held + 4 * v3 * run;
             ResidentPlan& p = S.res;
             char* X = static_cast<char*>(p.spins);
             const uint32_t plane = 16u * (uint32_t)(p.grid * kResBlock);
@@ -907,12 +977,12 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
          continue;
       }
       for (int64_t t = t0; t < t1 - 1; ++t) {
-         R* nxt = seg.p + v3 * (t - t0 + 1);
-         cudaMemcpyAsync(nxt, seg.p + v3 * (t - t0), sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
-         if ((rc = forward_step<R>(h, a, nxt, pb.p, eb.p, st))) return rc;
+         R* nxt = ws.seg + v3 * (t - t0 + 1);
+         cudaMemcpyAsync(nxt, ws.seg + v3 * (t - t0), sizeof(R) * v3, cudaMemcpyDeviceToDevice, h->stream);
+         if ((rc = forward_step<R>(h, a, nxt, ws.pb, ws.eb, st))) return rc;
       }
       for (int64_t t = t1 - 1; t >= t0; --t) {
-         b.S = seg.p + v3 * (t - t0);
+         b.S = ws.seg + v3 * (t - t0);
          adj_step_fmt<R>(S.fmt, a, b, t, h->stream);
          h->kernel_launches += 4;
       }
@@ -920,7 +990,7 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    }
    std::vector<double> gh(5 + np);
    int status = 0;
-   e = cudaMemcpyAsync(gh.data(), g.p, sizeof(double) * gh.size(), cudaMemcpyDeviceToHost, h->stream);
+   e = cudaMemcpyAsync(gh.data(), ws.g, sizeof(double) * gh.size(), cudaMemcpyDeviceToHost, h->stream);
    if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint result");

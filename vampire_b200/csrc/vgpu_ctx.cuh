@@ -64,6 +64,9 @@ struct SysDev {
    double* mus_SI = nullptr;     // [M] moments in J/T
    void* hd_atom = nullptr;
    void* hm_atom = nullptr;  // per-atom mu0 Hd field for the magnetostatic energy
+   void* adj_ws = nullptr;   // adjoint workspace, kept between calls up to kAdjKeepBytes (adjoint.cu)
+   size_t adj_ws_bytes = 0;
+   int* adj_bad = nullptr;   // result of the reciprocity check
    void* mc_tab = nullptr;   // Monte Carlo per-material tables
    std::vector<unsigned char> mc_tab_host;  // last contents copied to mc_tab
    const int* sys_off = nullptr;  // batched systems: first atom of each system

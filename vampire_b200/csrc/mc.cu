@@ -50,6 +50,9 @@ struct MCState {
    std::vector<int> colour_off;       // [ncolours+1] offsets into the atom list
    int* atoms = nullptr;              // [n] atoms sorted by colour
    int4* entries = nullptr;           // [n] per list position: atom, first SELL entry, row width, material
+   int sms = 1;                       // multiprocessors of the device
+   int width = 0;                     // bonds per trial row below (0: no trial rows, the sweeps read entries)
+   int* rows = nullptr;               // trial rows in list order (see mc_rows_kernel)
    unsigned long long* rejects = nullptr;
    void* replay = nullptr;            // [4n] (x|y|z gaussians, uniform) in R
    bool use_replay = false;
@@ -74,15 +77,22 @@ struct MCArgs {
    LLGArgs<R> a;
    const int4* entries;  // the colour's trials (list positions)
    int count;
+   const int* rows;      // trial rows (mc_rows_kernel): all colours'
+   int first;            // the colour's first list position
+   int shift;            // material bits of a row word (31: one material)
    const MCMat<R>* mat;  // [M]
    const R* replay;      // [4n] or nullptr
    uint64_t sweep;
    unsigned long long* rejects;
 };
 
+// the value is formed here as written: no later operation is contracted with it
+__device__ __forceinline__ void keep_value(float& x) { asm volatile("" : "+f"(x)); }
+__device__ __forceinline__ void keep_value(double& x) { asm volatile("" : "+d"(x)); }
+
 // dE of atom i (material mi) for the move S -> T in the fixed exchange field
 // h; P: any record with ku2, kux, kuy, kuz, kc4 (MatParams or MCMat)
-template <typename R, typename P>
+template <typename R, bool PLAIN = false, typename P>
 __device__ __forceinline__ R site_energy_delta(const LLGArgs<R>& a, int i, int mi, const P& m, const R S[3],
                                                const R T[3], const R h[3]) {
    // dE = E(T) - E(S) for the single-spin energy (exchange field h fixed)
@@ -92,6 +102,8 @@ __device__ __forceinline__ R site_energy_delta(const LLGArgs<R>& a, int i, int m
       const R et = T[0] * m.kux + T[1] * m.kuy + T[2] * m.kuz;
       d += -m.ku2 * (et * et - es * es);
    }
+   keep_value(d);
+   if (PLAIN) return d;
    if (a.cubic) {
       const R s4 = S[0] * S[0] * S[0] * S[0] + S[1] * S[1] * S[1] * S[1] + S[2] * S[2] * S[2] * S[2];
       const R t4 = T[0] * T[0] * T[0] * T[0] + T[1] * T[1] * T[1] * T[1] + T[2] * T[2] * T[2] * T[2];
@@ -105,92 +117,169 @@ __device__ __forceinline__ R site_energy_delta(const LLGArgs<R>& a, int i, int m
    return d;
 }
 
-// The trial's list entry holds its atom, row and material, so the row's bond
-// words, the own spin and the material record are all requested one load
-// after the thread starts (the atom list, the slice offsets and the material
-// id were three dependent loads before), and rows of width 6 or 12 (simple
-// cubic, FCC) are read with every bond word and neighbour spin in flight at
-// once.  Same arithmetic in the same bond order as the generic row loop.
-// Blocks of 256, at least VGPU_MC_MIN_BLOCKS per SM: 4 (64 registers, no
-// spills) measured fastest on SC 50^3 x 31 temperatures -- 2.905e10
-// spin-moves/s against 2.853e10 with 5 (48 registers), 2.70e10 with 6 (40)
-// and 2.56e10 with 7 or 8 (spilling); the sweep rate after 500 warm-up sweeps.
-#ifndef VGPU_MC_MIN_BLOCKS
-#define VGPU_MC_MIN_BLOCKS 4
-#endif
+// One trial of atom i (material mi) in its exchange field h; returns whether
+// the move was rejected.
+template <typename R, bool PLAIN = false>
+__device__ __forceinline__ bool mc_trial(const MCArgs<R>& p, int i, int mi, R h[3]) {
+   const LLGArgs<R>& a = p.a;
+   const MCMat<R> mm = p.mat[mi];
+   // magnetostatic energy uses the mu0 Hd field (energy.cpp:123-126)
+   if (PLAIN) {
+   } else if (a.cell) {
+      const int c = __ldg(a.cell + i);
+      h[0] += __ldg(a.cell_hd + c);
+      h[1] += __ldg(a.cell_hd + a.ncells + c);
+      h[2] += __ldg(a.cell_hd + 2 * a.ncells + c);
+   } else if (a.hm_atom) {
+      h[0] += __ldg(a.hm_atom + i); h[1] += __ldg(a.hm_atom + a.n + i); h[2] += __ldg(a.hm_atom + 2 * a.n + i);
+   }
+   const R S[3] = {a.ax[i], a.ay[i], a.az[i]};
+   R g0, g1, g2, u;
+   if (!PLAIN && p.replay) {
+      g0 = p.replay[i]; g1 = p.replay[a.n + i]; g2 = p.replay[2 * a.n + i]; u = p.replay[3 * a.n + i];
+   } else {
+      // keyed by the global atom index (a shard's atom i is atom noise_base + i)
+      const uint32_t gi = (uint32_t)i + a.noise_base;
+      const u32x4 c = {gi, (uint32_t)p.sweep, (uint32_t)(p.sweep >> 32), RNG_MC_MOVE};
+      const u32x4 r = philox4x32_10(c, a.seed_lo, a.seed_hi);
+      if (sizeof(R) == 4) {
+         // Box-Muller on the fast approximations (each Gaussian within 1e-5)
+         float s1, c1;
+         const float r1 = bm_radius_fast(r.x);
+         bm_angle_fast(r.y, c1, s1);
+         g0 = r1 * c1; g1 = r1 * s1; g2 = bm_radius_fast(r.z) * bm_cos_fast(r.w);
+         // u01f keeps the top 24 bits: the low bytes of r.y, r.z, r.w
+         u = (R)u01f(((r.y & 0xffu) << 8) | ((r.z & 0xffu) << 16) | (r.w << 24));
+      } else {
+         const u32x4 c2 = {gi, (uint32_t)p.sweep, (uint32_t)(p.sweep >> 32), RNG_MC_ACCEPT};
+         const u32x4 r2 = philox4x32_10(c2, a.seed_lo, a.seed_hi);
+         double s1, c1, s2, c2d;
+         const double r1 = sqrt(-2.0 * log(u01d(r.x)));
+         const double rr = sqrt(-2.0 * log(u01d(r.z)));
+         sincospi(2.0 * u01d(r.y), &s1, &c1);
+         sincospi(2.0 * u01d(r.w), &s2, &c2d);
+         g0 = (R)(r1 * c1); g1 = (R)(r1 * s1); g2 = (R)(rr * c2d);
+         u = (R)u01d(r2.x);
+      }
+   }
+   // the two instances round alike: neither takes these sums and products apart
+   for (int k = 0; k < 3; ++k) keep_value(h[k]);
+   keep_value(g0); keep_value(g1); keep_value(g2); keep_value(u);
+   const R sg = mm.sigma;
+   R T[3] = {S[0] + g0 * sg, S[1] + g1 * sg, S[2] + g2 * sg};
+   const R r = rsqrt_<R>(T[0] * T[0] + T[1] * T[1] + T[2] * T[2]);
+   T[0] *= r; T[1] *= r; T[2] *= r;
+   const R dE = site_energy_delta<R, PLAIN>(a, i, mi, mm, S, T, h) * mm.mu_ratio;
+   bool accept = dE < (R)0;
+   if (!accept) {
+      const R x = -dE * mm.beta;
+      accept = (sizeof(R) == 4 ? (R)expf((float)x) : (R)exp((double)x)) >= u;
+   }
+   if (accept) {
+      a.ax[i] = T[0]; a.ay[i] = T[1]; a.az[i] = T[2];
+   }
+   return !accept;
+}
+
+// A colour's trials on trial rows: word 0 of a row is the trial's atom, words
+// 1..W its bond words, all in the packed form index | material bits; the rows
+// of 32 consecutive list positions interleaved, so that a warp's word is one
+// 128-byte line.  Used where every bond is the table's (FMT_ISO_TAB) and no
+// row is wider than 12; rows narrower than W are filled up with bonds to the
+// zero spin.  The generic kernel below reads the slices of the neighbour list,
+// where a colour uses only every ncolours-th word of a line, and waits for its
+// list entry before it can ask for them.  Bound by the latency of the spin
+// gather, so a thread runs several trials and has the next one's row in flight
+// meanwhile; the first row is read, and the next colour's launch begun, before
+// the previous colour is done (the rows are written at the setup only).
+// PLAIN: no term beyond exchange, the applied field and the uniaxial
+// anisotropy, and no replayed numbers (a trial is 409 instructions a warp
+// with all the tests, and their issue is what remains).
+// A colour of simple cubic 50^3 x 31 temperatures (1.94 million trials): 65 us
+// on the neighbour list, 37 on trial rows, 32 PLAIN; with 6 or 10 blocks of
+// 128 per SM in place of 8 (64 registers) 32.5 and 33.
+constexpr int kMCBlock = 128;
+template <typename R>
+constexpr int mc_row_blocks(int w) {
+   return sizeof(R) == 8 ? 4 : w <= 8 ? 8 : 5;
+}
+template <typename R, int W, bool PLAIN>
+__global__ void __launch_bounds__(kMCBlock, mc_row_blocks<R>(W))
+   mc_rows_kernel(const MCArgs<R> p) {
+   const LLGArgs<R>& a = p.a;
+   const int end = p.first + p.count, stride = gridDim.x * kMCBlock;
+   // list positions from the warp boundary below the colour's first
+   int t = (p.first & ~31) + blockIdx.x * kMCBlock + threadIdx.x;
+   int c[W + 1];
+   auto load = [&](int q) {
+      const int* r = p.rows + (size_t)(q >> 5) * (32 * (W + 1)) + (q & 31);
+#pragma unroll
+      for (int k = 0; k <= W; ++k) c[k] = __ldcs(r + 32 * k);
+   };
+   if (t < end) load(t);
+   pdl_begin();
+   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+   int rejected = 0;
+   for (; t < end; t += stride) {
+      const bool mine = t >= p.first;
+      const int i = c[0] & a.idx_mask, mi = c[0] >> p.shift;
+      R x[W], y[W], z[W], J[W];
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+         const int j = c[k + 1] & a.idx_mask;
+         x[k] = __ldg(a.ax + j); y[k] = __ldg(a.ay + j); z[k] = __ldg(a.az + j);
+         J[k] = __ldg(a.jtab + mi * a.M + (c[k + 1] >> p.shift));
+      }
+      if (t + stride < end) load(t + stride);
+      R h[3] = {0, 0, 0};
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+         h[0] += J[k] * x[k]; h[1] += J[k] * y[k]; h[2] += J[k] * z[k];
+      }
+      if (mine) rejected += mc_trial<R, PLAIN>(p, i, mi, h);
+   }
+   rejected = __reduce_add_sync(0xffffffffu, rejected);
+   if ((threadIdx.x & 31) == 0 && rejected) atomicAdd(p.rejects, (unsigned long long)rejected);
+}
+
+// One trial per thread on the neighbour list itself: any bond format and row
+// width.  The trial's list entry holds its atom, row and material, so the row's
+// bond words, the own spin and the material record are all requested one load
+// after the thread starts; rows of 6 or 12 table bonds (the single-spin moves of
+// the hybrid constrained steps) are read with every bond in flight at once.
 template <typename R, int FMT>
-__global__ void __launch_bounds__(256, VGPU_MC_MIN_BLOCKS) mc_colour_kernel(const MCArgs<R> p) {
+__global__ void __launch_bounds__(256, 4) mc_colour_kernel(const MCArgs<R> p) {
    pdl_begin();  // launched by launch_pdl: the previous colour is done
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    bool rejected = false;
    if (t < p.count) {
-      const LLGArgs<R>& a = p.a;
       const int4 en = __ldg(p.entries + t);
-      const int i = en.x, base = en.y, w = en.z, mi = en.w;
-      const MCMat<R> mm = p.mat[mi];
+      const int i = en.x, mi = en.w;
       R h[3] = {0, 0, 0};
-      if (FMT == FMT_ISO_TAB && w == 6)
-         exchange_gather_w<R, FMT, 6, 0, false>(a, base, mi, a.ax, a.ay, a.az, h[0], h[1], h[2], nullptr);
-      else if (FMT == FMT_ISO_TAB && w == 12)
-         exchange_gather_w<R, FMT, 12, 0, false>(a, base, mi, a.ax, a.ay, a.az, h[0], h[1], h[2], nullptr);
+      if (FMT == FMT_ISO_TAB && en.z == 6)
+         exchange_gather_w<R, FMT, 6, 0, false>(p.a, en.y, mi, p.a.ax, p.a.ay, p.a.az, h[0], h[1], h[2], nullptr);
+      else if (FMT == FMT_ISO_TAB && en.z == 12)
+         exchange_gather_w<R, FMT, 12, 0, false>(p.a, en.y, mi, p.a.ax, p.a.ay, p.a.az, h[0], h[1], h[2], nullptr);
       else
-         exchange_gather_row<R, FMT>(a, base, w, mi, a.ax, a.ay, a.az, h[0], h[1], h[2]);
-      // magnetostatic energy uses the mu0 Hd field (energy.cpp:123-126)
-      if (a.cell) {
-         const int c = __ldg(a.cell + i);
-         h[0] += __ldg(a.cell_hd + c);
-         h[1] += __ldg(a.cell_hd + a.ncells + c);
-         h[2] += __ldg(a.cell_hd + 2 * a.ncells + c);
-      } else if (a.hm_atom) {
-         h[0] += __ldg(a.hm_atom + i); h[1] += __ldg(a.hm_atom + a.n + i); h[2] += __ldg(a.hm_atom + 2 * a.n + i);
-      }
-      const R S[3] = {a.ax[i], a.ay[i], a.az[i]};
-      R g0, g1, g2, u;
-      if (p.replay) {
-         g0 = p.replay[i]; g1 = p.replay[a.n + i]; g2 = p.replay[2 * a.n + i]; u = p.replay[3 * a.n + i];
-      } else {
-         // keyed by the global atom index (a shard's atom i is atom noise_base + i)
-         const uint32_t gi = (uint32_t)i + a.noise_base;
-         const u32x4 c = {gi, (uint32_t)p.sweep, (uint32_t)(p.sweep >> 32), RNG_MC_MOVE};
-         const u32x4 r = philox4x32_10(c, a.seed_lo, a.seed_hi);
-         if (sizeof(R) == 4) {
-            // Box-Muller on the fast approximations (each Gaussian within 1e-5)
-            float s1, c1;
-            const float r1 = bm_radius_fast(r.x);
-            bm_angle_fast(r.y, c1, s1);
-            g0 = r1 * c1; g1 = r1 * s1; g2 = bm_radius_fast(r.z) * bm_cos_fast(r.w);
-            // u01f keeps the top 24 bits: the low bytes of r.y, r.z, r.w
-            u = (R)u01f(((r.y & 0xffu) << 8) | ((r.z & 0xffu) << 16) | (r.w << 24));
-         } else {
-            const u32x4 c2 = {gi, (uint32_t)p.sweep, (uint32_t)(p.sweep >> 32), RNG_MC_ACCEPT};
-            const u32x4 r2 = philox4x32_10(c2, a.seed_lo, a.seed_hi);
-            double s1, c1, s2, c2d;
-            const double r1 = sqrt(-2.0 * log(u01d(r.x)));
-            const double rr = sqrt(-2.0 * log(u01d(r.z)));
-            sincospi(2.0 * u01d(r.y), &s1, &c1);
-            sincospi(2.0 * u01d(r.w), &s2, &c2d);
-            g0 = (R)(r1 * c1); g1 = (R)(r1 * s1); g2 = (R)(rr * c2d);
-            u = (R)u01d(r2.x);
-         }
-      }
-      const R sg = mm.sigma;
-      R T[3] = {S[0] + g0 * sg, S[1] + g1 * sg, S[2] + g2 * sg};
-      const R r = rsqrt_<R>(T[0] * T[0] + T[1] * T[1] + T[2] * T[2]);
-      T[0] *= r; T[1] *= r; T[2] *= r;
-      const R dE = site_energy_delta<R>(a, i, mi, mm, S, T, h) * mm.mu_ratio;
-      bool accept = dE < (R)0;
-      if (!accept) {
-         const R x = -dE * mm.beta;
-         accept = (sizeof(R) == 4 ? (R)expf((float)x) : (R)exp((double)x)) >= u;
-      }
-      if (accept) {
-         a.ax[i] = T[0]; a.ay[i] = T[1]; a.az[i] = T[2];
-      } else {
-         rejected = true;
-      }
+         exchange_gather_row<R, FMT>(p.a, en.y, en.z, mi, p.a.ax, p.a.ay, p.a.az, h[0], h[1], h[2]);
+      rejected = mc_trial<R>(p, i, mi, h);
    }
    const unsigned ballot = __ballot_sync(0xffffffffu, rejected);
    if ((threadIdx.x & 31) == 0 && ballot) atomicAdd(p.rejects, (unsigned long long)__popc(ballot));
+}
+
+// trial rows of the colour-sorted atoms (rows of bonds to the zero spin past the last)
+__global__ void mc_rows_fill_kernel(const int* __restrict__ atoms, int count, const int* __restrict__ slice_off,
+                                    const int* __restrict__ col, const int* __restrict__ mat, int mat_shift, int pad,
+                                    int width, int* __restrict__ rows) {
+   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+   if (t >= ((count + 31) & ~31)) return;
+   int* r = rows + (size_t)(t >> 5) * (32 * (width + 1)) + (t & 31);
+   const int i = t < count ? atoms[t] : pad;
+   const int off = t < count ? slice_off[i >> 5] : 0;
+   const int w = t < count ? (slice_off[(i >> 5) + 1] - off) >> 5 : 0;
+   r[0] = t < count && mat_shift ? i | (mat[i] << mat_shift) : i;
+   for (int k = 0; k < width; ++k) r[32 * (k + 1)] = k < w ? col[off + 32 * k + (i & 31)] : pad;
 }
 
 // list entries of the colour-sorted atoms (rows from the slice offsets)
@@ -201,6 +290,28 @@ __global__ void mc_entries_kernel(const int* __restrict__ atoms, int count, cons
    const int i = atoms[t];
    const int off = slice_off[i >> 5];
    out[t] = make_int4(i, off + (i & 31), (slice_off[(i >> 5) + 1] - off) >> 5, mat ? mat[i] : 0);
+}
+
+template <typename R, int W, bool PLAIN>
+static cudaError_t launch_mc_rows(const MCArgs<R>& p, int sms, cudaStream_t st) {
+   if (p.count == 0) return cudaSuccess;
+   const int trials = p.count + (p.first & 31);
+   const int blocks = std::min((trials + kMCBlock - 1) / kMCBlock, sms * mc_row_blocks<R>(W));
+   return launch_pdl(mc_rows_kernel<R, W, PLAIN>, dim3(blocks), dim3(kMCBlock), 0, st, p);
+}
+
+template <typename R, bool PLAIN>
+static cudaError_t mc_rows_width(const MCArgs<R>& p, int width, int sms, cudaStream_t st) {
+   if (width == 6) return launch_mc_rows<R, 6, PLAIN>(p, sms, st);
+   if (width == 8) return launch_mc_rows<R, 8, PLAIN>(p, sms, st);
+   return launch_mc_rows<R, 12, PLAIN>(p, sms, st);
+}
+
+template <typename R>
+static cudaError_t mc_rows_dispatch(const MCArgs<R>& p, int width, int sms, cudaStream_t st) {
+   const LLGArgs<R>& a = p.a;
+   const bool plain = !p.replay && !a.cell && !a.hm_atom && !a.cubic && !a.aniso_ext && !a.bq_off;
+   return plain ? mc_rows_width<R, true>(p, width, sms, st) : mc_rows_width<R, false>(p, width, sms, st);
 }
 
 template <typename R, int FMT>
@@ -229,6 +340,7 @@ void mc_destroy(vgpu_ctx* h) {
    cmc_destroy(h);  // its pairing follows this colouring
    cudaFree(s->atoms);
    cudaFree(s->entries);
+   cudaFree(s->rows);
    cudaFree(s->rejects);
    cudaFree(s->replay);
    delete s;
@@ -304,10 +416,25 @@ extern "C" int vgpu_mc_setup(vgpu_handle h, const int32_t* colour_in, int32_t* n
    for (int i = 0; i < nu; ++i) order[fill[colour[i]]++] = i;
    cudaError_t e;
    if ((e = cudaMalloc(&s->atoms, sizeof(int) * order.size())) != cudaSuccess) return cuda_err(h, e, "mc atoms");
-   if ((e = cudaMalloc(&s->entries, sizeof(int4) * order.size())) != cudaSuccess) return cuda_err(h, e, "mc entries");
+   if ((e = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, h->device)) != cudaSuccess)
+      return cuda_err(h, e, "device");
+   if (S.fmt == FMT_ISO_TAB && S.zmax <= 12) {
+      s->width = S.zmax <= 6 ? 6 : S.zmax <= 8 ? 8 : 12;
+      if (cudaMalloc(&s->rows, sizeof(int) * 32 * (size_t)(s->width + 1) * ((nu + 31) / 32 + 1)) != cudaSuccess) {
+         (void)cudaGetLastError();  // no room: the sweeps read the neighbour list
+         s->width = 0;
+      }
+   }
+   if (!s->width && (e = cudaMalloc(&s->entries, sizeof(int4) * order.size())) != cudaSuccess)
+      return cuda_err(h, e, "mc entries");
    if ((e = cudaMalloc(&s->rejects, sizeof(unsigned long long))) != cudaSuccess) return cuda_err(h, e, "mc counter");
    cudaMemcpyAsync(s->atoms, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, h->stream);
-   if (nu > 0) {
+   if (nu > 0 && s->width) {
+      mc_rows_fill_kernel<<<(nu + 255) / 256, 256, 0, h->stream>>>(
+         s->atoms, nu, (const int*)S.slice_off, (const int*)S.col, (const int*)S.mat, S.mat_shift, S.n_alloc - 1,
+         s->width, s->rows);
+      if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(h, e, "mc trial rows");
+   } else if (nu > 0) {
       mc_entries_kernel<<<(nu + 255) / 256, 256, 0, h->stream>>>(s->atoms, nu, (const int*)S.slice_off,
                                                                    (const int*)S.mat, s->entries);
       if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(h, e, "mc entries");
@@ -415,10 +542,13 @@ static int mc_run_colour(vgpu_handle h, const R* tab, int c) {
    p.replay = s->use_replay ? (const R*)s->replay : nullptr;
    p.sweep = s->sweep;
    p.rejects = s->rejects;
-   p.entries = s->entries + s->colour_off[c];
+   p.first = s->colour_off[c];
    p.count = s->colour_off[c + 1] - s->colour_off[c];
+   p.rows = s->rows;
+   p.shift = p.a.mat_shift ? p.a.mat_shift : 31;
+   p.entries = s->width ? nullptr : s->entries + p.first;
    h->prof_begin(PROF_MC);
-   cudaError_t e = mc_dispatch<R>(p, S.fmt, h->stream);
+   cudaError_t e = s->width ? mc_rows_dispatch<R>(p, s->width, s->sms, h->stream) : mc_dispatch<R>(p, S.fmt, h->stream);
    h->prof_end(PROF_MC);
    if (e != cudaSuccess) return cuda_err(h, e, "mc launch");
    h->kernel_launches++;

@@ -22,14 +22,9 @@ enum : uint32_t { RNG_THERMAL = 0u, RNG_MC_MOVE = 1u, RNG_MC_ACCEPT = 2u, RNG_TH
 struct u32x4 { uint32_t x, y, z, w; };
 
 VGPU_HD void mulhilo32(uint32_t a, uint32_t b, uint32_t& hi, uint32_t& lo) {
-#ifdef __CUDA_ARCH__
-   lo = a * b;
-   hi = __umulhi(a, b);
-#else
-   uint64_t p = (uint64_t)a * (uint64_t)b;
+   const uint64_t p = (uint64_t)a * (uint64_t)b;  // one wide multiply on the device too
    lo = (uint32_t)p;
    hi = (uint32_t)(p >> 32);
-#endif
 }
 
 VGPU_HD u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1) {

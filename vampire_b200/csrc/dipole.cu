@@ -207,10 +207,15 @@ __global__ void near_ell_kernel(int npairs, int nc, int maxp, const int* __restr
 // Near-field correction and final scaling (update.cpp:56-99).  The pairs' FP64
 // tensors are the bytes of this kernel (52 B a pair, about 33 pairs a cell),
 // so what counts is how many loads are in flight.  L = 1: a thread per cell,
-// four pairs' loads issued together; L = 8: eight lanes per cell, for grids
-// with too few cells to fill the GPU with one thread each.
+// two pairs' loads issued together, eight blocks per SM; the tensors, more than
+// the L2 holds from one update to the next, are read as a stream and leave it
+// to the moments (125,000 cells: 40 us, 4.9 TB/s of tensors; 49 with four
+// pairs in four blocks and without the hint, 46 and 44 with one of the two
+// changes, 51 with one pair in twelve blocks, 53 and 59 with two and four lanes
+// per cell).  L = 8: eight lanes per cell, four pairs each, for grids with too
+// few cells to fill the GPU with one thread each; their tensors stay in the L2.
 template <typename R, int L>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, L == 1 ? 8 : 4)
     cell_finish_kernel(int nc, const int* __restrict__ near_cnt, const int* __restrict__ near_je,
                        const double* __restrict__ near_te, int maxp, const double* __restrict__ mag,
                        const double* __restrict__ self, const float4* __restrict__ pos, double* __restrict__ field,
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(128)
    if (i < nc && near_cnt) {
       const size_t qs = (size_t)maxp * nc;
       const int cnt = near_cnt[i];
-      constexpr int U = 4;
+      constexpr int U = L == 1 ? 2 : 4;
       for (int k0 = lane; k0 < cnt; k0 += U * L) {
          int j[U];
          double T[U][6];
@@ -232,9 +237,9 @@ __global__ void __launch_bounds__(128)
          for (int u = 0; u < U; ++u) {
             const size_t e = (size_t)(k0 + u * L) * nc + i;
             const bool on = k0 + u * L < cnt;
-            j[u] = on ? near_je[e] : -1;
+            j[u] = !on ? -1 : L == 1 ? __ldcs(near_je + e) : near_je[e];
 #pragma unroll
-            for (int q = 0; q < 6; ++q) T[u][q] = on ? near_te[q * qs + e] : 0.0;
+            for (int q = 0; q < 6; ++q) T[u][q] = !on ? 0.0 : L == 1 ? __ldcs(near_te + q * qs + e) : near_te[q * qs + e];
          }
 #pragma unroll
          for (int u = 0; u < U; ++u) {

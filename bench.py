@@ -347,10 +347,9 @@ def bench_adjoint(device, L=32, steps=2000):
     gradient of the trajectory loss w.r.t. (J, Ku, H) at J=11.2e-21 J,
     Ku=6.69e-24 J, H=(0,0,0.4) T against the target m_z(t) of J=10e-21 J,
     Ku=5e-24 J, H=(0,0,0.5) T; the FP32 production build (FP64 sums for m_z,
-    the loss and the gradients), sqrt(N) checkpointing, with the FP64 debug
+    the loss and the gradients), every state kept, with the FP64 debug
     build timed beside it.  Timed around AdjointRunner.loss_and_grad: the
-    system set-up and upload and the C-ABI call (forward with checkpoints,
-    segment recomputation and the backward sweep); the median of five calls
+    system set-up and upload and the C-ABI call (forward and backward sweep); the median of five calls
     after two warm-up calls."""
     from vampire_b200 import adjoint as A
     run = A.AdjointRunner(L=L, device=device, precision="fp32")
@@ -358,8 +357,8 @@ def bench_adjoint(device, L=32, steps=2000):
     target = run64.trajectory(10e-21, 5e-24, (0.0, 0.0, 0.5), steps)
     for _ in range(2):  # warm-up (module loading, first allocations)
         run.loss_and_grad(11.2e-21, 6.69e-24, (0.0, 0.0, 0.4), target)
-    # five timed gradients, the median reported: the host wall clock around
-    # ~20,000 launches varies between runs on a shared host
+    # five timed gradients, the median reported: the host wall clock (set-up and
+    # upload are most of it) varies between runs on a shared host
     times = []
     for _ in range(5):
         t0 = time.perf_counter()
@@ -392,7 +391,7 @@ def bench_adjoint(device, L=32, steps=2000):
                            "max_rel_grad_dev_fp32": float(np.max(np.abs(grad - grad64)[[0, 1, 4]] /
                                                                  np.abs(grad64)[[0, 1, 4]]))},
             "loss": loss,
-            "grad": [float(g) for g in grad], "checkpoints": int(-(-steps // int(steps ** 0.5 + 0.999999))),
+            "grad": [float(g) for g in grad],
             "error_vs_fd": {"max_rel_dev": float(max(rel)), "components": ["J", "Ku", "Hz"],
                             "against": "central differences (h = 1e-6 relative) of the FP64 forward loss"}}
 

@@ -688,8 +688,9 @@ int vgpu_batch_system_range(vgpu_handle h, int32_t k, int32_t* first_atom, int32
  * (m_z: moment-weighted mean of s_z after step t) and
  *   grad[0] = dL/d(common scale of every exchange coupling),
  *   grad[1] = dL/dKu_SI (ku2 = Ku/mu_s), grad[2..4] = dL/dH_applied [1/T],
- * by the adjoint of the step with checkpoints every `every` steps
- * (0: ceil(sqrt(n_steps))).  Every exchange format (isotropic, vectorial,
+ * by the adjoint of the step with checkpoints every `every` steps (0: every
+ * state is kept where a workspace of 1 GiB holds them, else checkpoints every
+ * ceil(sqrt(n_steps))).  Every exchange format (isotropic, vectorial,
  * diagonal + DMI, full tensor) and any number of materials, provided the
  * couplings are reciprocal in SI units (mu_s,j J_ji = (mu_s,i J_ij)^T, as a
  * symmetric exchange matrix and the three-site DMI give; checked on the

@@ -7,7 +7,7 @@
 //   s' = n(v),  v = s + dt f(s, H(s)),   s1 = n(u),  u = s + dt/2 (f(s,H(s)) + f(s',H(s')))
 //   f(s,H) = A s x H + B s x (s x H),   H(s)_i = sum_j J_ij s_j + anisotropy(s_i) + H_app
 //
-// backwards with four fused per-atom kernels per step: (1) recompute H(s), f,
+// backwards with four fused per-atom stages per step: (1) recompute H(s), f,
 // s'; (2) recompute H(s'), f', s1 and push lambda through n(u), f' and H(s');
 // (3) the transposed exchange gather of H(s')-bar, through n(v), f and H(s);
 // (4) the transposed gather of H(s)-bar plus dL_t/ds_t gives lambda_t.
@@ -26,8 +26,9 @@
 // scaled together, Ku, H_app; and per pair of materials (a, b) the scale of
 // the couplings of the bonds from atoms of a to atoms of b (the diagonal,
 // exchange-matrix part for the diagonal + DMI format), plus the common scale
-// of the DMI vectors.  States are checkpointed every ceil(sqrt(N)) steps and
-// recomputed segment by segment with the forward passes.
+// of the DMI vectors.  The states of all steps are kept where the workspace
+// has the room and no interval is asked for; else they are checkpointed every
+// ceil(sqrt(N)) steps and recomputed segment by segment.
 //
 // Precision: the state, the recomputed steps and the adjoint vectors are in
 // the handle's precision (FP32 in production, FP64 in the debug build); the

@@ -31,7 +31,8 @@
 // arithmetic: with lines of 128 points the grids are 3 x 3.3 MB.  At 125,000
 // cells (50^3, P = 128) the five launches measured take the place of radix-2
 // passes through shared memory over complex lines (two barriers and integer
-// divisions per point and stage): 376 us then; see fft_z_kernel for the split.
+// divisions per point and stage): 376 us then, 46 now (x 7, y 5, z 24, y 5,
+// x 4); see fft_z_kernel for the split.
 //
 // Precision follows the handle: in the FP64 build every step is FP64, so the
 // result equals the direct FP64 sum to rounding (~1e-15 of the field); the

@@ -159,3 +159,29 @@ def test_two_handles_in_two_threads(vgpu_lib):
     [t.start() for t in th]
     [t.join() for t in th]
     assert np.array_equal(got[0], want) and np.array_equal(got[1], want)
+
+
+@pytest.mark.parametrize("name", ["sc6_open_t300", "sc20_t0", "fcc4_dmi_t0"])
+def test_steps_recorded_into_a_graph(vgpu_lib, name):
+    """Steps recorded on the handle's stream and replayed twice do at T = 0 what
+    twice as many steps do (the replays cannot reuse a resident launch)."""
+    import torch
+    from vampire_b200 import vgpu
+    s, _ = load_golden(name)
+    s.params.temperature = 0.0
+    with vgpu.Simulation(s) as sim:
+        sim.llg_heun(2 + 2 * 6)
+        want = sim.spins()
+    with vgpu.Simulation(s) as sim:
+        sim.llg_heun(2)
+        sim.synchronize()
+        stream = torch.cuda.ExternalStream(sim.stream_ptr())
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream, capture_error_mode="relaxed"):
+            sim.llg_heun(6)
+        with torch.cuda.stream(stream):
+            g.replay()
+            g.replay()
+        torch.cuda.synchronize()
+        got = sim.spins()
+    assert np.array_equal(got, want)

@@ -234,7 +234,10 @@ static int plan_resident(vgpu_ctx* h) {
       // two states of one (FP32) or two (FP64) 16-byte words per thread's atom
       const size_t bytes = 2 * (sizeof(R) == 8 ? 2 : 1) * 16 * (size_t)p.grid * K * kResidentBlock;
       p.spins = h->alloc(bytes);
-      if (!p.spins) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the resident plan");
+      if (!p.spins) {  // no room: one launch per pass
+         (void)cudaGetLastError();
+         return VGPU_OK;
+      }
       int bad = 0;
       int rc = cuda_err(h, cudaMemsetAsync(p.spins, 0, bytes, h->stream), "resident plan");
       if (!rc) rc = cuda_err(h, launch_resident_check<R>(a, S.status, h->stream), "resident plan");
@@ -631,6 +634,12 @@ static bool thermal_philox(const vgpu_ctx* h) {
    return h->params.thermal_enabled && h->any_sigma && h->noise_mode == VGPU_NOISE_PHILOX;
 }
 
+// the caller records the handle's stream into a graph
+static bool capturing(vgpu_ctx* h) {
+   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+   return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 // increment buffers and the staged launch shape, before any pass; whole_steps:
 // the caller runs both passes of every step, so that the external field may be
 // kept between them
@@ -656,12 +665,19 @@ static int prepare_passes(vgpu_ctx* h, bool* staged_out, int integrator = INTEG_
       if (e != cudaSuccess) return cuda_err(h, e, "staged pass setup (tile records exceed shared memory?)");
       h->sys.stage = c;
    }
-   if ((staged ? !h->sys.stage.win : whole_steps && thermal_philox(h)) && !h->sys.g_store[0]) {
-      // the step's external field, passed from the predictor to the corrector
+   if ((staged ? !h->sys.stage.win : whole_steps && thermal_philox(h) && !capturing(h)) && !h->sys.g_store[0]) {
+      // the step's external field, passed from the predictor to the corrector;
+      // where there is no room (or no allocation allowed) the unstaged corrector
+      // computes it again
       const size_t len = ((size_t)h->sys.n_alloc + 3) & ~(size_t)3;
-      for (int q = 0; q < 3; ++q) {
-         h->sys.g_store[q] = h->alloc(len * sizeof(R));
-         if (!h->sys.g_store[q]) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the external-field buffers");
+      for (int q = 0; q < 3; ++q) h->sys.g_store[q] = h->alloc(len * sizeof(R));
+      if (!h->sys.g_store[0] || !h->sys.g_store[1] || !h->sys.g_store[2]) {
+         for (int q = 0; q < 3; ++q) {
+            h->release(h->sys.g_store[q]);
+            h->sys.g_store[q] = nullptr;
+         }
+         (void)cudaGetLastError();
+         if (staged) return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the external-field buffers");
       }
    }
    *staged_out = staged;
@@ -700,7 +716,8 @@ template <typename R>
 static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
    SysDev& S = h->sys;
    *mode = STEP_PASSES;
-   if (passes_asked(h)) return VGPU_OK;
+   // a captured launch would run again with the half-step numbers of its first run
+   if (passes_asked(h) || capturing(h)) return VGPU_OK;
    *var = integrator == INTEG_MIDPOINT ? VAR_MIDPOINT : S.aniso_ext ? VAR_HEUN_EXT : VAR_HEUN;
    if (S.one.size) {
       if (S.one.cap_var != *var) {

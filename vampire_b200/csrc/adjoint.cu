@@ -404,6 +404,22 @@ __global__ void adj_lambda_init(const LLGArgs<R> a, AdjBufs<R> b, int64_t N) {
    b.lam[2 * st + i] = (R)(2.0 * b.w * (b.mz[N] - b.target[N - 1]) * (double)a.mp[mi].mu_s_muB / b.musum);
 }
 
+// Rows narrower than their slice are filled up with bonds to the padding atom
+// (entry stride - 1), whose spin has to be zero: the coupling of such a bond is
+// not, in the table formats.  The kernels write the atoms' entries only, so the
+// padding entry of every plane that neighbours are gathered from is cleared here,
+// after each layout of the workspace (whose memory held something else before).
+template <typename R> struct AdjPlanes {
+   R* at[4];
+   int planes[4];
+};
+template <typename R>
+__global__ void adj_clear_pads_kernel(const AdjPlanes<R> p, int stride) {
+   const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+   for (int r = 0; r < 4; ++r)
+      for (int k = t; k < p.planes[r]; k += nt) p.at[r][(size_t)k * stride + stride - 1] = (R)0;
+}
+
 // m_z after a step: block sums of mu s_z added into out[0]
 template <typename R>
 __global__ void mz_kernel(int n, const R* __restrict__ sz, const int* __restrict__ mat,
@@ -692,6 +708,15 @@ struct DevVec {
    cudaError_t alloc(size_t n) { return cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1)); }
 };
 
+template <typename R>
+cudaError_t clear_pads(const AdjPlanes<R>& p, int stride, cudaStream_t st) {
+   int most = 0;
+   for (int k : p.planes) most = std::max(most, k);
+   if (most == 0) return cudaSuccess;
+   adj_clear_pads_kernel<R><<<std::min((most + 127) / 128, 1024), 128, 0, st>>>(p, stride);
+   return cudaGetLastError();
+}
+
 // one Heun step (the ordinary passes, no thermal term) of the state in `x`
 // (3 * stride values, x|y|z), the predictor increment stored
 template <typename R>
@@ -774,6 +799,7 @@ int mz_trajectory_typed(vgpu_handle h, uint64_t n_steps, double* mz_out) {
    for (int q = 0; q < 3; ++q)
       cudaMemcpyAsync(cur.p + (size_t)q * st, S.s[q], sizeof(R) * st, cudaMemcpyDeviceToDevice, h->stream);
    cudaMemsetAsync(mz.p, 0, sizeof(double) * (n_steps + 1), h->stream);
+   if ((e = clear_pads<R>({{pb.p}, {3}}, st, h->stream))) return cuda_err(h, e, "trajectory buffers");
    LLGArgs<R> a = make_args<R>(h);
    bool resident = false;
    if (int rc = adjoint_resident<R>(h, a, nullptr, &resident)) return rc;
@@ -888,7 +914,12 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
          h->sys.adj_ws_bytes = 0;
       }
    } release{h};
-   cudaError_t e;
+   // gathered: the states, s', and without resident threads also Hb0 and Hb1 (in
+   // work; resident ones skip the padding)
+   cudaError_t e = clear_pads<R>({{ws.seg, ws.pb, ws.held, ws.work},
+                                  {(int)(3 * (C + 1)), 3, resident ? 3 * run : 0, resident ? 0 : 30}}, st, h->stream);
+   if (e != cudaSuccess) return cuda_err(h, e, "adjoint buffers");
+   h->kernel_launches++;
    cudaMemcpyAsync(ws.tg, target, sizeof(double) * N, cudaMemcpyHostToDevice, h->stream);
    cudaMemsetAsync(ws.mz, 0, sizeof(double) * (N + 1), h->stream);
    cudaMemsetAsync(ws.g, 0, sizeof(double) * (5 + np), h->stream);

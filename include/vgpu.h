@@ -262,6 +262,13 @@ int vgpu_set_noise_replay(vgpu_handle h, const double* xi);
  * buffers and no block-wide barrier; 0 or -1 (default) = the tile passes.
  * The results are the same bit for bit. */
 #define VGPU_OPT_STAGE_WARPS 10
+/* VGPU_OPT_RESIDENT_WAIT_TEST: 1 = the spins that a resident launch (several
+ * steps of a small or medium system at once, and the adjoint's sweeps) starts
+ * from are marked with a half-step that nobody waits for, so the threads'
+ * bounded waits for their neighbours (1 s) run out and the call, or the next
+ * one that synchronises, fails with VGPU_ERR_TIMEOUT (test of the timeout path;
+ * the handle stays usable after setting it back to 0). */
+#define VGPU_OPT_RESIDENT_WAIT_TEST 11
 /* Bond-record layout the next FP32 pass reads: *layout = VGPU_RECORDS_WINDOW
  * (compact words with window staging), VGPU_RECORDS_COMPACT,
  * VGPU_RECORDS_WIDE (16-byte records) or VGPU_RECORDS_NONE (formats without

@@ -768,6 +768,12 @@ int forward_run(vgpu_ctx* h, const LLGArgs<R>& a, int n, R* x, R* inc, int strid
    return cuda_err(h, e, "adjoint forward");
 }
 
+// the device status word, when the stream has come to here
+cudaError_t read_status(vgpu_ctx* h, int* status) {
+   const cudaError_t e = cudaMemcpyAsync(status, h->sys.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+   return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+}
+
 int check_adjoint_ok(vgpu_ctx* h) {
    if (!h) return set_err(nullptr, VGPU_ERR_ARG, "null handle");
    if (!h->sys.uploaded) return set_err(h, VGPU_ERR_STATE, "no system uploaded");
@@ -803,6 +809,7 @@ int mz_trajectory_typed(vgpu_handle h, uint64_t n_steps, double* mz_out) {
    LLGArgs<R> a = make_args<R>(h);
    bool resident = false;
    if (int rc = adjoint_resident<R>(h, a, nullptr, &resident)) return rc;
+   if (resident) a.wait_test = h->resident_wait_test;
    DevVec<double> rows;
    if (resident && (e = rows.alloc((size_t)kAdjRun * S.res.grid * (kResBlock / 32)))) return cuda_err(h, e, "trajectory buffers");
    for (uint64_t t = 0; resident && t < n_steps; t += kAdjRun) {
@@ -816,9 +823,11 @@ int mz_trajectory_typed(vgpu_handle h, uint64_t n_steps, double* mz_out) {
                  (double*)(mz.p + t + 1));
    }
    std::vector<double> host(n_steps + 1);
+   int status = 0;
    e = cudaMemcpyAsync(host.data(), mz.p, sizeof(double) * (n_steps + 1), cudaMemcpyDeviceToHost, h->stream);
-   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+   if (e == cudaSuccess) e = read_status(h, &status);
    if (e != cudaSuccess) return cuda_err(h, e, "trajectory");
+   if (status & 2) return h->check_status();  // a resident wait ran out
    const double ms = moment_sum(h);
    for (uint64_t t = 0; t < n_steps; ++t) mz_out[t] = host[t + 1] / ms;
    return VGPU_OK;
@@ -859,6 +868,7 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    const AdjFns<R> fns = adj_fns<R>(S.fmt, pair_out != nullptr);
    bool resident = false;
    if ((rc = adjoint_resident<R>(h, a, fns.back, &resident))) return rc;
+   if (resident) a.wait_test = h->resident_wait_test;
    // Checkpoints every C steps (default ceil(sqrt(N))), their segments recomputed;
    // with resident threads and the default, all states are kept instead where
    // the workspace stays within what is kept between calls.
@@ -948,9 +958,11 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
    }
    // loss on the host from m_z(t)
    std::vector<double> mzh(N + 1);
+   int status = 0;
    e = cudaMemcpyAsync(mzh.data(), ws.mz, sizeof(double) * (N + 1), cudaMemcpyDeviceToHost, h->stream);
-   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+   if (e == cudaSuccess) e = read_status(h, &status);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint forward");
+   if (status & 2) return h->check_status();  // a resident wait ran out
    const double musum = moment_sum(h);
    // m_z was summed unnormalised: scale the device copy once
    for (int64_t t = 0; t <= N; ++t) mzh[t] /= musum;
@@ -1021,10 +1033,8 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
       if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(h, e, "adjoint backward");
    }
    std::vector<double> gh(5 + np);
-   int status = 0;
    e = cudaMemcpyAsync(gh.data(), ws.g, sizeof(double) * gh.size(), cudaMemcpyDeviceToHost, h->stream);
-   if (e == cudaSuccess) e = cudaMemcpyAsync(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+   if (e == cudaSuccess) e = read_status(h, &status);
    if (e != cudaSuccess) return cuda_err(h, e, "adjoint result");
    if (status & 2) return h->check_status();  // a resident wait ran out
    *loss_out = loss;

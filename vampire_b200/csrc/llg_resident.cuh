@@ -31,7 +31,8 @@
 // stores travel.  Waits are bounded (1 s): a warp that gives up sets status bit
 // 2 (VGPU_ERR_TIMEOUT on the host) and leaves, and the others then give up too.
 // Half-steps are numbered through from launch to launch, so what an earlier
-// launch left is never taken for the present.
+// launch left is never taken for the present.  a.wait_test marks the first words
+// with the number before, which no wait asks for.
 //
 // The arithmetic is that of the passes (the same functions in the same order),
 // so the states are the same bit for bit.
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR, K>()))
          S0[k][0] = a.ax[i]; S0[k][1] = a.ay[i]; S0[k][2] = a.az[i];
       }
       P[k][0] = S0[k][0]; P[k][1] = S0[k][1]; P[k][2] = S0[k][2];
-      ResSpin<R>::store(XA, plane, 16u * (uint32_t)i, S0[k], epoch0);
+      ResSpin<R>::store(XA, plane, 16u * (uint32_t)i, S0[k], a.wait_test ? epoch0 - 1 : epoch0);
    }
    const int s0 = blk * kResSlices * K, ns = min(kResSlices * K, nslices - s0);
    const int o0 = __ldg(a.slice_off + s0);
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR_HEUN_EX
       for (int c = 0; c < 3; ++c) S0[c] = x[(size_t)c * stride + i];
       external_field<R>(a, i, d.mat(a, r.mi), false, E);
    }
-   ResSpin<R>::store(XA, plane, self, S0, epoch0);
+   ResSpin<R>::store(XA, plane, self, S0, a.wait_test ? epoch0 - 1 : epoch0);
    auto field = [&](const char* X, uint32_t t, const R S[3], R H[3]) -> bool {
       R hx = 0, hy = 0, hz = 0;
       if (!res_gather<R, FMT, 6>(a, r, X, plane, self, t, hx, hy, hz)) return false;

@@ -16,7 +16,7 @@
 // Waits on the mbarriers are bounded (1 s of wall time, and a poll count): if
 // a copy has not landed by then the block records status bit 2
 // (VGPU_ERR_TIMEOUT on the host), waits -- bounded again -- for its copies
-// still in flight, and returns.  a.stage_extra_tx > 0 makes every tile expect
+// still in flight, and returns.  a.wait_test > 0 makes every tile expect
 // that many bytes more than its copy delivers, so the wait runs out: the test
 // of this path.
 #pragma once
@@ -91,7 +91,7 @@ enum StageFeat : int { FEAT_FIXED = 1, FEAT_THERMAL = 2, FEAT_UNIAXIAL = 4, FEAT
 // the bits that hold for a (0 when a is not the FEAT_FIXED case)
 inline int stage_features(const LLGArgs<float>& a) {
    if (a.ramp_n || a.local_field || a.hd_atom || a.ex || a.sys_off || a.noise_mode != VGPU_NOISE_PHILOX || a.bq_off ||
-       a.aniso_ext || a.stage_extra_tx)
+       a.aniso_ext || a.wait_test)
       return 0;
    return FEAT_FIXED | (a.thermal ? FEAT_THERMAL : 0) | (a.uniaxial ? FEAT_UNIAXIAL : 0) |
           (a.cubic ? FEAT_CUBIC : 0) | (a.tab_scalar ? FEAT_TABSCALAR : 0);
@@ -111,7 +111,7 @@ __device__ __forceinline__ LLGArgs<float> fold_features(const LLGArgs<float>& in
       a.noise_mode = VGPU_NOISE_PHILOX;
       a.bq_off = 0;
       a.aniso_ext = 0;
-      a.stage_extra_tx = 0;
+      a.wait_test = 0;
       a.thermal = (FEAT & FEAT_THERMAL) ? 1 : 0;
       a.uniaxial = (FEAT & FEAT_UNIAXIAL) ? 1 : 0;
       a.cubic = (FEAT & FEAT_CUBIC) ? 1 : 0;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(32 * SL, 24 / SL) llg_staged_kernel(const LLGA
       float* own = reinterpret_cast<float*>(buf + buf_bytes);
       const size_t a0 = (size_t)s0 * 32;
       fence_proxy_async();
-      mbar_arrive_expect_tx(&mbar[b], bytes + db + nb * (uint32_t)na + (uint32_t)a.stage_extra_tx);
+      mbar_arrive_expect_tx(&mbar[b], bytes + db + nb * (uint32_t)na + (uint32_t)a.wait_test);
       if (bytes) bulk_copy_g2s(buf, src, bytes, &mbar[b]);
       if (db) bulk_copy_g2s(sdict, a.cdict, db, &mbar[b]);
       bulk_copy_g2s(own, a.ax + a0, nb, &mbar[b]);
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(128, 6) llg_warp_kernel(const LLGArgs<float> a
       float* own = reinterpret_cast<float*>(buf + buf_bytes);
       const size_t a0 = (size_t)s0 * 32;
       fence_proxy_async();
-      mbar_arrive_expect_tx(&mb[b], bytes + 128u * (uint32_t)na + (uint32_t)a.stage_extra_tx);
+      mbar_arrive_expect_tx(&mb[b], bytes + 128u * (uint32_t)na + (uint32_t)a.wait_test);
       if (bytes) bulk_copy_g2s(buf, a.crec + o0, bytes, &mb[b]);
       bulk_copy_g2s(own, a.ax + a0, 128, &mb[b]);
       bulk_copy_g2s(own + 32, a.ay + a0, 128, &mb[b]);
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(32 * SL, 24 / SL) llg_window_kernel(const LLGA
       const uint32_t db = 16u * (uint32_t)(a.tab_scalar ? a.cdict_n : 2 * a.cdict_n);
       if (tid == 0) {
          fence_proxy_async();
-         mbar_arrive_expect_tx(&mbar, rb + db + 12u * (uint32_t)__ldg(a.wtile_w + t) + (uint32_t)a.stage_extra_tx);
+         mbar_arrive_expect_tx(&mbar, rb + db + 12u * (uint32_t)__ldg(a.wtile_w + t) + (uint32_t)a.wait_test);
          if (rb) bulk_copy_g2s(stage_smem, a.lrec + tile_off, rb, &mbar);
          bulk_copy_g2s(sdict, a.cdict, db, &mbar);
       }

@@ -513,7 +513,7 @@ LLGArgs<R> make_args(vgpu_ctx* h) {
    a.fx = (R*)S.f[0]; a.fy = (R*)S.f[1]; a.fz = (R*)S.f[2];
    a.ex = (R*)S.e[0]; a.ey = (R*)S.e[1]; a.ez = (R*)S.e[2];
    a.status = S.status;
-   a.stage_extra_tx = h->stage_wait_test ? 16 : 0;
+   a.wait_test = h->stage_wait_test ? 16 : 0;
    a.sys_off = S.sys_off;
    a.m_per_sys = S.m_per_sys;
    a.ramp_n = S.ramp_n;
@@ -748,7 +748,8 @@ static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
 template <typename R>
 static int run_resident(vgpu_ctx* h, uint64_t n, StepMode mode, int var) {
    SysDev& S = h->sys;
-   const LLGArgs<R> a = make_args<R>(h);
+   LLGArgs<R> a = make_args<R>(h);
+   a.wait_test = h->resident_wait_test;
    const cudaError_t e = mode == STEP_CLUSTER ? launch_llg_cluster<R>(a, S.fmt, var, (int)n, S.one, h->stream)
                                               : launch_llg_resident<R>(a, S.fmt, var, (int)n, S.res, S.nslices, h->stream);
    if (e != cudaSuccess) return cuda_err(h, e, "resident llg launch");
@@ -840,7 +841,8 @@ int vgpu_ctx::check_status() {
    rc = cuda_err(this, cudaMemsetAsync(sys.status, 0, sizeof(int), stream), "status reset");
    if (rc) return rc;
    if (st & 1) return set_err(this, VGPU_ERR_NAN, "non-finite or non-normalisable spin produced by the integrator");
-   if (st & 2) return set_err(this, VGPU_ERR_TIMEOUT, "a bond-record copy into shared memory did not complete in time");
+   if (st & 2) return set_err(this, VGPU_ERR_TIMEOUT, "a bounded wait on the device ran out (a copy of bond records into shared memory, or the "
+                                        "neighbours' spins of a resident launch, did not arrive in time)");
    return VGPU_OK;
 }
 namespace vgpu {
@@ -1183,6 +1185,9 @@ extern "C" int vgpu_set_option(vgpu_handle h, int option, int value) {
          return VGPU_OK;
       case VGPU_OPT_STAGE_WAIT_TEST:
          h->stage_wait_test = value != 0;
+         return VGPU_OK;
+      case VGPU_OPT_RESIDENT_WAIT_TEST:
+         h->resident_wait_test = value != 0;
          return VGPU_OK;
       case VGPU_OPT_DIPOLE_FFT:
          if (value < -1 || value > 1) return set_err(h, VGPU_ERR_ARG, "dipole FFT: -1, 0 or 1");

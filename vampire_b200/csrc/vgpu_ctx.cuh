@@ -129,6 +129,7 @@ struct vgpu_ctx {
    int staged = -1;          // VGPU_OPT_STAGED_RECORDS (-1 default)
    int stage_sl = -1, stage_nbuf = -1;  // -1: per record layout (tile_shape in vgpu_api.cu)
    bool stage_wait_test = false;  // VGPU_OPT_STAGE_WAIT_TEST
+   bool resident_wait_test = false;  // VGPU_OPT_RESIDENT_WAIT_TEST
    int dipole_fft = -1;      // VGPU_OPT_DIPOLE_FFT (-1 default: FFT far field on regular cell grids)
    int compact = -1;         // VGPU_OPT_COMPACT_RECORDS (-1 default: compact records when built)
    int window = -1;          // VGPU_OPT_WINDOW_STAGING (-1 default: off)

@@ -114,7 +114,8 @@ struct LLGArgs {
                              // dipole), written by the predictor and read back by the
                              // corrector, or nullptr (the corrector computes it)
    int* status;              // device status word (non-finite spin flag)
-   int stage_extra_tx;       // staged passes: extra bytes each tile expects (0; > 0 tests the bounded wait)
+   int wait_test;            // tests of the bounded waits (0: none): extra bytes each tile of a staged pass
+                             // expects, or first words of a resident launch marked late
 };
 
 // the sweep's fraction at a.step, with every change of the step

@@ -28,6 +28,7 @@ OPT_COMPACT_RECORDS = 7
 OPT_WINDOW_STAGING = 8
 OPT_PROFILE_EVERY = 9
 OPT_STAGE_WARPS = 10
+OPT_RESIDENT_WAIT_TEST = 11
 EXCHANGE_FORMATS = ("iso_tab", "iso_bond", "vec_tab", "vec_bond", "dmi_tab", "tensor_bond")
 RECORDS_NONE, RECORDS_WIDE, RECORDS_COMPACT, RECORDS_WINDOW = 0, 1, 2, 3
 PASS_PREDICTOR, PASS_CORRECTOR = 0, 1
@@ -263,7 +264,7 @@ class Simulation:
     def set_option(self, option: int, value: int) -> None:
         """vgpu_set_option: OPT_STORE_INCREMENT, OPT_STAGED_RECORDS, OPT_STAGE_SLICES,
         OPT_STAGE_BUFFERS, OPT_DIPOLE_FFT, OPT_STAGE_WAIT_TEST, OPT_COMPACT_RECORDS,
-        OPT_WINDOW_STAGING, OPT_PROFILE_EVERY."""
+        OPT_WINDOW_STAGING, OPT_PROFILE_EVERY, OPT_STAGE_WARPS, OPT_RESIDENT_WAIT_TEST."""
         self._check(lib().vgpu_set_option(self._h, int(option), int(value)))
 
     def record_layout(self) -> Tuple[int, int]:

@@ -422,7 +422,7 @@ __global__ void adj_clear_pads_kernel(const AdjPlanes<R> p, int stride) {
 
 // m_z after a step: block sums of mu s_z added into out[0]
 template <typename R>
-__global__ void mz_kernel(int n, const R* __restrict__ sz, const int* __restrict__ mat,
+__global__ void mz_kernel(int n, const R* sz, const int* __restrict__ mat,
                           const MatParams<R>* __restrict__ mp, double* out) {
    pdl_begin();  // launched by launch_pdl
    const int i = blockIdx.x * blockDim.x + threadIdx.x;

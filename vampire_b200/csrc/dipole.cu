@@ -85,9 +85,8 @@ static DipoleState* dip_of(vgpu_ctx* h) { return (DipoleState*)h->extras[2]; }
 template <typename R>
 __global__ void __launch_bounds__(256)
     cell_moment_kernel(int nc, int glog, const int* __restrict__ start, const int* __restrict__ atoms,
-                       const R* __restrict__ sx, const R* __restrict__ sy, const R* __restrict__ sz,
-                       const int* __restrict__ mat, const double* __restrict__ mus_SI, double* __restrict__ mag,
-                       float4* __restrict__ mom) {
+                       const R* sx, const R* sy, const R* sz, const int* __restrict__ mat,
+                       const double* __restrict__ mus_SI, double* __restrict__ mag, float4* __restrict__ mom) {
    pdl_begin();
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    const int G = 1 << glog, c = t >> glog, lane = t & (G - 1);

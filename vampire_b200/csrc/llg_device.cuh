@@ -79,10 +79,21 @@ __device__ __forceinline__ void dmi_bond<double>(double jx, double jy, double jz
    hz += jz * z + (dx * y - dy * x);
 }
 
-// exchange gather of atom i over its SELL row, sources (sx,sy,sz)
-template <typename R> __device__ __forceinline__ R ld_src(const R* p, int coherent) {
-   return coherent ? __ldcg(p) : __ldg(p);
+// How a gather reads the spins: through L2 (LOAD = 1: written earlier in the same
+// launch by other blocks), by ordinary loads (isotropic table bonds, and
+// biquadratic lists beside them), or by the read-only path.  A system of
+// isotropic table bonds has kernels on its stream that let the next one start
+// before they have written the spins (launch_pdl), and the read-only path is
+// good only for what does not change while a kernel is resident.
+enum SpinLoad : int { SPIN_PLAIN = 0, SPIN_L2 = 1, SPIN_READ_ONLY = 2 };
+template <int LOAD, int FMT> constexpr int spin_load() {
+   return LOAD ? SPIN_L2 : FMT == FMT_ISO_TAB ? SPIN_PLAIN : SPIN_READ_ONLY;
 }
+template <typename R> __device__ __forceinline__ R ld_src(const R* p, int how) {
+   return how == SPIN_L2 ? __ldcg(p) : how == SPIN_READ_ONLY ? __ldg(p) : *p;
+}
+
+// exchange gather of atom i over its SELL row, sources (sx,sy,sz)
 
 // The row is given by its first entry (base) and width (w); exchange_gather
 // below finds them from the slice offsets of atom i.
@@ -90,15 +101,15 @@ template <typename R> __device__ __forceinline__ R ld_src(const R* p, int cohere
 // blocks (persistent batched kernel) and are read through L2 (ld.global.cg)
 template <typename R, int FMT, int LOAD = 0>
 __device__ __forceinline__ void exchange_gather_row(const LLGArgs<R>& a, int base, int w, int mi,
-                                                    const R* __restrict__ sx, const R* __restrict__ sy,
-                                                    const R* __restrict__ sz, R& hx, R& hy, R& hz) {
+                                                    const R* sx, const R* sy,
+                                                    const R* sz, R& hx, R& hy, R& hz) {
    const R* __restrict__ tab = a.jtab;
 #pragma unroll 4
    for (int k = 0; k < w; ++k) {
       const int e = base + 32 * k;
       const int c = __ldg(a.col + e);
       const int j = c & a.idx_mask;
-      const R x = ld_src(sx + j, LOAD), y = ld_src(sy + j, LOAD), z = ld_src(sz + j, LOAD);
+      const R x = ld_src(sx + j, (spin_load<LOAD, FMT>())), y = ld_src(sy + j, (spin_load<LOAD, FMT>())), z = ld_src(sz + j, (spin_load<LOAD, FMT>()));
       if (FMT == FMT_ISO_TAB) {
          const int mj = a.mat_shift ? (c >> a.mat_shift) : 0;
          const R J = __ldg(tab + mi * a.M + mj);
@@ -130,8 +141,8 @@ __device__ __forceinline__ void exchange_gather_row(const LLGArgs<R>& a, int bas
 }
 
 template <typename R, int FMT, int LOAD = 0>
-__device__ __forceinline__ void exchange_gather(const LLGArgs<R>& a, int i, int mi, const R* __restrict__ sx,
-                                                const R* __restrict__ sy, const R* __restrict__ sz, R& hx,
+__device__ __forceinline__ void exchange_gather(const LLGArgs<R>& a, int i, int mi, const R* sx,
+                                                const R* sy, const R* sz, R& hx,
                                                 R& hy, R& hz) {
    const int sl = i >> 5;
    const int off = __ldg(a.slice_off + sl);
@@ -147,8 +158,8 @@ __device__ __forceinline__ void exchange_gather(const LLGArgs<R>& a, int i, int 
 // STAGED: the records of this row were bulk-copied to shared memory; srec
 // points at the thread's first record there (stride 32 records per bond).
 template <typename R, int FMT, int W, int LOAD, bool STAGED>
-__device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base, int mi, const R* __restrict__ sx,
-                                                  const R* __restrict__ sy, const R* __restrict__ sz, R& hx, R& hy,
+__device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base, int mi, const R* sx,
+                                                  const R* sy, const R* sz, R& hx, R& hy,
                                                   R& hz, const int4* srec) {
    const R* __restrict__ tab = a.jtab;
    if (FMT == FMT_DMI_TAB && STAGED) {
@@ -163,7 +174,7 @@ __device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base,
 #pragma unroll
       for (int k = 0; k < W; ++k) {
          const int j = c[k] & a.idx_mask;
-         x[k] = ld_src(sx + j, LOAD); y[k] = ld_src(sy + j, LOAD); z[k] = ld_src(sz + j, LOAD);
+         x[k] = ld_src(sx + j, (spin_load<LOAD, FMT>())); y[k] = ld_src(sy + j, (spin_load<LOAD, FMT>())); z[k] = ld_src(sz + j, (spin_load<LOAD, FMT>()));
       }
 #pragma unroll
       for (int k = 0; k < W; ++k) {
@@ -186,7 +197,7 @@ __device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base,
 #pragma unroll
       for (int k = 0; k < W; ++k) {
          const int j = rec[k].x & a.idx_mask;
-         x[k] = ld_src(sx + j, LOAD); y[k] = ld_src(sy + j, LOAD); z[k] = ld_src(sz + j, LOAD);
+         x[k] = ld_src(sx + j, (spin_load<LOAD, FMT>())); y[k] = ld_src(sy + j, (spin_load<LOAD, FMT>())); z[k] = ld_src(sz + j, (spin_load<LOAD, FMT>()));
       }
 #pragma unroll
       for (int k = 0; k < W; ++k) {
@@ -209,7 +220,7 @@ __device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base,
 #pragma unroll
       for (int k = 0; k < W; ++k) {
          const int j = c[k] & a.idx_mask;
-         x[k] = ld_src(sx + j, LOAD); y[k] = ld_src(sy + j, LOAD); z[k] = ld_src(sz + j, LOAD);
+         x[k] = ld_src(sx + j, (spin_load<LOAD, FMT>())); y[k] = ld_src(sy + j, (spin_load<LOAD, FMT>())); z[k] = ld_src(sz + j, (spin_load<LOAD, FMT>()));
       }
 #pragma unroll
       for (int k = 0; k < W; ++k) {
@@ -227,8 +238,8 @@ __device__ __forceinline__ void exchange_gather_w(const LLGArgs<R>& a, int base,
 // same coupling values, so the two record layouts give identical fields.
 // STAGED: sw points at the thread's first word in shared memory (stride 32).
 template <typename R, int W, int LOAD, bool STAGED>
-__device__ __forceinline__ void exchange_gather_c(const LLGArgs<R>& a, int base, const R* __restrict__ sx,
-                                                  const R* __restrict__ sy, const R* __restrict__ sz, R& hx, R& hy,
+__device__ __forceinline__ void exchange_gather_c(const LLGArgs<R>& a, int base, const R* sx,
+                                                  const R* sy, const R* sz, R& hx, R& hy,
                                                   R& hz, const uint32_t* sw, const float4* dict) {
    const uint32_t jmask = (1u << a.crec_shift) - 1u;
    uint32_t c[W];
@@ -238,7 +249,7 @@ __device__ __forceinline__ void exchange_gather_c(const LLGArgs<R>& a, int base,
 #pragma unroll
    for (int k = 0; k < W; ++k) {
       const int j = (int)(c[k] & jmask);
-      x[k] = ld_src(sx + j, LOAD); y[k] = ld_src(sy + j, LOAD); z[k] = ld_src(sz + j, LOAD);
+      x[k] = ld_src(sx + j, (spin_load<LOAD, FMT_DMI_TAB>())); y[k] = ld_src(sy + j, (spin_load<LOAD, FMT_DMI_TAB>())); z[k] = ld_src(sz + j, (spin_load<LOAD, FMT_DMI_TAB>()));
    }
 #pragma unroll
    for (int k = 0; k < W; ++k) {
@@ -302,8 +313,8 @@ __device__ __forceinline__ void exchange_gather_win(const LLGArgs<R>& a, int w_r
 // biquadratic exchange field of atom i at own spin S over its SELL-32 list:
 // sum_j 2 J_bq (S.s_j) s_j (src/exchange/biquadratic_fields.cpp:60-76)
 template <typename R, int LOAD = 0>
-__device__ __forceinline__ void biquadratic_field(const LLGArgs<R>& a, int i, const R* __restrict__ sx,
-                                                  const R* __restrict__ sy, const R* __restrict__ sz, const R S[3],
+__device__ __forceinline__ void biquadratic_field(const LLGArgs<R>& a, int i, const R* sx,
+                                                  const R* sy, const R* sz, const R S[3],
                                                   R& hx, R& hy, R& hz) {
    hx = hy = hz = 0;
    const int sl = i >> 5;
@@ -314,7 +325,7 @@ __device__ __forceinline__ void biquadratic_field(const LLGArgs<R>& a, int i, co
       const int e = base + 32 * k;
       const int j = __ldg(a.bq_col + e);
       const R twoJbq = (R)2 * __ldg(a.bq_j + e);
-      const R x = ld_src(sx + j, LOAD), y = ld_src(sy + j, LOAD), z = ld_src(sz + j, LOAD);
+      const R x = ld_src(sx + j, (spin_load<LOAD, FMT_ISO_TAB>())), y = ld_src(sy + j, (spin_load<LOAD, FMT_ISO_TAB>())), z = ld_src(sz + j, (spin_load<LOAD, FMT_ISO_TAB>()));
       const R d = S[0] * x + S[1] * y + S[2] * z;
       hx += twoJbq * x * d;
       hy += twoJbq * y * d;
@@ -348,8 +359,8 @@ __device__ __forceinline__ E biquadratic_energy(const LLGArgs<R>& a, int i, cons
 // REC: which FP32 DMI record layout the caller was compiled for (REC_ANY:
 // compact when a.crec is set, else 16-byte; the staged passes fix one).
 template <typename R, int FMT, int LOAD, bool STAGED = false, int REC = REC_ANY>
-__device__ __forceinline__ void exchange_field(const LLGArgs<R>& a, int i, int mi, const R* __restrict__ sx,
-                                               const R* __restrict__ sy, const R* __restrict__ sz, R& hx, R& hy,
+__device__ __forceinline__ void exchange_field(const LLGArgs<R>& a, int i, int mi, const R* sx,
+                                               const R* sy, const R* sz, R& hx, R& hy,
                                                R& hz, const int4* srec_tile = nullptr, int tile_off = 0,
                                                const float4* sdict = nullptr, const float* swin = nullptr,
                                                int wmax = 0) {

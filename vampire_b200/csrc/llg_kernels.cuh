@@ -202,20 +202,20 @@ template <typename R> __device__ __forceinline__ IsoRow iso_row(const LLGArgs<R>
 }
 
 template <typename R>
-__device__ __forceinline__ void iso_field(const LLGArgs<R>& a, const IsoRow& r, R J, const R* __restrict__ sx,
-                                          const R* __restrict__ sy, const R* __restrict__ sz, R& hx, R& hy, R& hz) {
+__device__ __forceinline__ void iso_field(const LLGArgs<R>& a, const IsoRow& r, R J, const R* sx, const R* sy,
+                                          const R* sz, R& hx, R& hy, R& hz) {
    auto add = [&](R x, R y, R z) { hx += J * x; hy += J * y; hz += J * z; };
    if (r.w == 6) {
       R x[6], y[6], z[6];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) { x[k] = __ldg(sx + r.j[k]); y[k] = __ldg(sy + r.j[k]); z[k] = __ldg(sz + r.j[k]); }
+      for (int k = 0; k < 6; ++k) { x[k] = sx[r.j[k]]; y[k] = sy[r.j[k]]; z[k] = sz[r.j[k]]; }
 #pragma unroll
       for (int k = 0; k < 6; ++k) add(x[k], y[k], z[k]);
    } else {
 #pragma unroll 4
       for (int k = 0; k < r.w; ++k) {
          const int j = __ldg(a.col + r.base + 32 * k) & a.idx_mask;
-         add(__ldg(sx + j), __ldg(sy + j), __ldg(sz + j));
+         add(sx[j], sy[j], sz[j]);
       }
    }
 }

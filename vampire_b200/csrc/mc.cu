@@ -217,6 +217,10 @@ __global__ void __launch_bounds__(kMCBlock, mc_row_blocks<R>(W))
       for (int k = 0; k <= W; ++k) c[k] = __ldcs(r + 32 * k);
    };
    if (t < end) load(t);
+   if (t < p.first) {  // another colour's row, whose neighbours move meanwhile: bonds to the zero spin
+#pragma unroll
+      for (int k = 0; k <= W; ++k) c[k] = a.n_alloc - 1;
+   }
    pdl_begin();
    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
    int rejected = 0;
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(kMCBlock, mc_row_blocks<R>(W))
 #pragma unroll
       for (int k = 0; k < W; ++k) {
          const int j = c[k + 1] & a.idx_mask;
-         x[k] = __ldg(a.ax + j); y[k] = __ldg(a.ay + j); z[k] = __ldg(a.az + j);
+         x[k] = a.ax[j]; y[k] = a.ay[j]; z[k] = a.az[j];
          J[k] = __ldg(a.jtab + mi * a.M + (c[k + 1] >> p.shift));
       }
       if (t + stride < end) load(t + stride);

@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256) stats_mag_small_kernel(const LLGArgs<R> a
       const float4* Z = reinterpret_cast<const float4*>(a.az);
 #pragma unroll 2
       for (int g = tid; g < ng; g += stride) {
-         const float4 x = __ldg(X + g), y = __ldg(Y + g), z = __ldg(Z + g);
+         const float4 x = X[g], y = Y[g], z = Z[g];
          const int4 m = a.mat ? __ldg(reinterpret_cast<const int4*>(a.mat) + g) : make_int4(0, 0, 0, 0);
          const int4 bn = NB == 1 ? make_int4(0, 0, 0, 0) : __ldg(reinterpret_cast<const int4*>(mask) + g);
          add(m.x, bn.x, x.x, y.x, z.x);

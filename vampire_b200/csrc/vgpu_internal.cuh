@@ -235,13 +235,24 @@ VGPU_EXTERN(double)
 extern template cudaError_t launch_thermal_noise<float>(const LLGArgs<float>&, cudaStream_t);
 extern template cudaError_t launch_thermal_noise<double>(const LLGArgs<double>&, cudaStream_t);
 
-// A kernel launched with programmatic stream serialisation: its blocks may be
-// scheduled while the previous kernel of the stream drains.  The kernel must
-// call pdl_begin() before it touches global memory: the previous kernel of the
-// stream is complete and its writes are visible after that.  (Letting the next
-// kernel's blocks in earlier, with griddepcontrol.launch_dependents after the
-// wait, was measured too: 0.97x - 1.03x, 2 - 3 % slower for passes of several
-// blocks per SM, whose slots the waiting blocks take.)
+// Programmatic stream serialisation.  A kernel launched by launch_pdl may have its
+// blocks scheduled while the previous kernel of the stream drains; pdl_begin()
+// returns when that kernel is complete and its writes are visible.
+//
+// Three kernels (llg_iso_pass_kernel, mc_rows_kernel, llg_cluster_kernel; all on
+// isotropic table bonds) also let the next kernel's blocks in early
+// (griddepcontrol.launch_dependents directly after their pdl_begin), so that
+// those read their rows of the neighbour list meanwhile.  Hence for every kernel
+// launched by launch_pdl:
+//  * before pdl_begin it reads only what the upload, a setup that ended with a
+//    synchronisation, or a copy on the stream has written, never what a kernel
+//    of the stream writes, and it writes nothing;
+//  * spins and predictor states it reads after pdl_begin come by ordinary loads,
+//    not by the read-only path (ld_src; no const __restrict__ kernel arguments):
+//    the kernel may have been resident before they were written.
+// (Letting the next kernel in early everywhere was measured too: 0.97x - 1.03x,
+// 2 - 3 % slower for passes of several blocks per SM, whose slots the waiting
+// blocks take.)
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... Args>

@@ -422,7 +422,10 @@ extern "C" int vgpu_mc_setup(vgpu_handle h, const int32_t* colour_in, int32_t* n
    if ((e = cudaMalloc(&s->atoms, sizeof(int) * order.size())) != cudaSuccess) return cuda_err(h, e, "mc atoms");
    if ((e = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, h->device)) != cudaSuccess)
       return cuda_err(h, e, "device");
-   if (S.fmt == FMT_ISO_TAB && S.zmax <= 12) {
+   // (a system without bonds has this format whatever its materials, also more of
+   // them than fit beside an atom's index in a word)
+   const bool words_fit = ((int64_t)(S.M - 1) << S.mat_shift) < ((int64_t)1 << 31);
+   if (S.fmt == FMT_ISO_TAB && S.zmax <= 12 && words_fit) {
       s->width = S.zmax <= 6 ? 6 : S.zmax <= 8 ? 8 : 12;
       if (cudaMalloc(&s->rows, sizeof(int) * 32 * (size_t)(s->width + 1) * ((nu + 31) / 32 + 1)) != cudaSuccess) {
          (void)cudaGetLastError();  // no room: the sweeps read the neighbour list

@@ -238,14 +238,17 @@ static int plan_resident(vgpu_ctx* h) {
          (void)cudaGetLastError();
          return VGPU_OK;
       }
+      // one-sided bonds: no plan.  The check's answer goes into the first word (0 else)
       int bad = 0;
       int rc = cuda_err(h, cudaMemsetAsync(p.spins, 0, bytes, h->stream), "resident plan");
-      if (!rc) rc = cuda_err(h, launch_resident_check<R>(a, S.status, h->stream), "resident plan");
+      if (!rc) rc = cuda_err(h, launch_resident_check<R>(a, (int*)p.spins, h->stream), "resident plan");
       if (!rc)
-         rc = cuda_err(h, cudaMemcpyAsync(&bad, S.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "resident plan");
+         rc = cuda_err(h, cudaMemcpyAsync(&bad, p.spins, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "resident plan");
       if (!rc) rc = cuda_err(h, cudaStreamSynchronize(h->stream), "resident plan");
-      if (!rc && bad) return cuda_err(h, cudaMemsetAsync(S.status, 0, sizeof(int), h->stream), "status");
-      if (rc) return rc;
+      if (rc || bad) {
+         h->release(p.spins);
+         return rc;
+      }
       S.res = p;
       return VGPU_OK;
    }

@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -733,10 +734,36 @@ int forward_step(vgpu_ctx* h, LLGArgs<R> a, R* x, R* pb, R* eb, int stride) {
 
 // steps of the backward run whose states and fields are held at once
 constexpr int kAdjRun = 64;
-// workspace that a handle keeps between calls (allocating and freeing it took 5
-// to 15 ms of a 15 ms gradient): 1 GiB of the 180, the states of 2,500 steps of
-// 32,768 spins
-constexpr size_t kAdjKeepBytes = (size_t)1 << 30;
+// Workspaces that handles keep between calls (allocating and freeing one took 5
+// to 15 ms of a 15 ms gradient): at most 1 GiB of a GPU's 180 for all handles of
+// the process together, the states of 2,500 steps of 32,768 spins.  A handle
+// that finds no room in it gives its workspace back at the end of each call; a
+// kept one goes with the system, and when an allocation of its handle fails
+// (vgpu_ctx::alloc).
+constexpr int64_t kAdjKeepBytes = (int64_t)1 << 30;
+std::atomic<int64_t> g_adj_kept[64];  // by device; none is kept on a device beyond
+
+// bytes that this handle's workspace may have and still be kept
+int64_t keep_room(const vgpu_ctx* h) {
+   if (h->device >= 64) return 0;
+   return kAdjKeepBytes - (g_adj_kept[h->device].load() - (int64_t)h->sys.adj_ws_kept);
+}
+
+// keeps the workspace after a call if there is room for it, else frees it
+void keep_or_drop(vgpu_ctx* h) {
+   SysDev& S = h->sys;
+   if (!S.adj_ws || S.adj_ws_kept) return;
+   const int64_t bytes = (int64_t)S.adj_ws_bytes;
+   if (h->device < 64) {
+      if (g_adj_kept[h->device].fetch_add(bytes) + bytes <= kAdjKeepBytes) {
+         S.adj_ws_kept = S.adj_ws_bytes;
+         return;
+      }
+      g_adj_kept[h->device].fetch_sub(bytes);
+   }
+   cudaStreamSynchronize(h->stream);
+   adjoint_drop(h);
+}
 
 // whether the sweeps (and, given its kernel, the backward run) can run resident
 template <typename R>
@@ -896,12 +923,12 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
          take(ws.rows, resident ? (size_t)kAdjRun * S.res.grid * (kResBlock / 32) : 0);
       };
       layout(nullptr);
-      if (all && bytes > kAdjKeepBytes) {
+      if (all && (int64_t)bytes > keep_room(h)) {
          all = false;
          continue;
       }
       if (S.adj_ws_bytes < bytes) {
-         h->release(S.adj_ws);
+         adjoint_drop(h);
          S.adj_ws = h->alloc(bytes);
          S.adj_ws_bytes = S.adj_ws ? bytes : 0;
       }
@@ -914,16 +941,10 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
       else if (resident) resident = false;
       else return set_err(h, VGPU_ERR_OOM, "cudaMalloc failed for the adjoint buffers (%zu bytes)", bytes);
    }
-   struct Release {  // a workspace beyond the limit goes back when the call is done
+   struct Done {
       vgpu_ctx* h;
-      ~Release() {
-         if (h->sys.adj_ws_bytes <= kAdjKeepBytes) return;
-         cudaStreamSynchronize(h->stream);
-         h->release(h->sys.adj_ws);
-         h->sys.adj_ws = nullptr;
-         h->sys.adj_ws_bytes = 0;
-      }
-   } release{h};
+      ~Done() { keep_or_drop(h); }
+   } done{h};
    // gathered: the states, s', and without resident threads also Hb0 and Hb1 (in
    // work; resident ones skip the padding)
    cudaError_t e = clear_pads<R>({{ws.seg, ws.pb, ws.held, ws.work},
@@ -1045,6 +1066,16 @@ int adjoint_typed(vgpu_handle h, uint64_t n_steps, const double* target, double 
 }
 
 }  // namespace
+
+bool vgpu::adjoint_drop(vgpu_ctx* h) {
+   SysDev& S = h->sys;
+   if (!S.adj_ws) return false;
+   h->release(S.adj_ws);
+   if (S.adj_ws_kept) g_adj_kept[h->device].fetch_sub((int64_t)S.adj_ws_kept);
+   S.adj_ws = nullptr;
+   S.adj_ws_bytes = S.adj_ws_kept = 0;
+   return true;
+}
 
 extern "C" int vgpu_mz_trajectory(vgpu_handle h, uint64_t n_steps, double* mz_out) {
    int rc = check_adjoint_ok(h);

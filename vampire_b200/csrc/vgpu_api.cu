@@ -63,6 +63,8 @@ void* vgpu_ctx::alloc(size_t bytes) {
    cudaError_t e = cudaMalloc(&p, bytes);
    if (e != cudaSuccess) {
       cudaGetLastError();
+      // what is only kept for the next gradient makes room
+      if (e == cudaErrorMemoryAllocation && vgpu::adjoint_drop(this)) return alloc(bytes);
       return nullptr;
    }
    allocs.push_back(p);
@@ -81,6 +83,7 @@ void vgpu_ctx::release(void* p) {
 }
 
 void vgpu_ctx::free_system() {
+   vgpu::adjoint_drop(this);
    for (void* p : allocs) cudaFree(p);
    allocs.clear();
    sys = SysDev();

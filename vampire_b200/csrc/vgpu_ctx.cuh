@@ -64,8 +64,9 @@ struct SysDev {
    double* mus_SI = nullptr;     // [M] moments in J/T
    void* hd_atom = nullptr;
    void* hm_atom = nullptr;  // per-atom mu0 Hd field for the magnetostatic energy
-   void* adj_ws = nullptr;   // adjoint workspace, kept between calls up to kAdjKeepBytes (adjoint.cu)
+   void* adj_ws = nullptr;   // adjoint workspace (adjoint.cu)
    size_t adj_ws_bytes = 0;
+   size_t adj_ws_kept = 0;   // its bytes in the sum of kept workspaces (0: it goes with the call)
    int* adj_bad = nullptr;   // result of the reciprocity check
    void* mc_tab = nullptr;   // Monte Carlo per-material tables
    std::vector<unsigned char> mc_tab_host;  // last contents copied to mc_tab
@@ -105,6 +106,7 @@ void mc_destroy(vgpu_ctx* h);
 void dipole_destroy(vgpu_ctx* h);
 void batch_destroy(vgpu_ctx* h);
 void torque_destroy(vgpu_ctx* h);
+bool adjoint_drop(vgpu_ctx* h);  // frees the adjoint workspace; whether there was one
 void cmc_destroy(vgpu_ctx* h);
 int torque_reset(vgpu_ctx* h);
 const double* batch_ramp(vgpu_ctx* h);

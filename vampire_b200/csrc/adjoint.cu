@@ -769,8 +769,10 @@ void keep_or_drop(vgpu_ctx* h) {
 template <typename R>
 int adjoint_resident(vgpu_ctx* h, const LLGArgs<R>& a, BackwardFn<R> back, bool* use) {
    *use = false;
+   if (passes_asked(h)) return VGPU_OK;
+   if (int rc = plan_resident<R>(h)) return rc;
    const ResidentPlan& p = h->sys.res;
-   if (p.K != 1 || passes_asked(h)) return VGPU_OK;
+   if (p.K != 1) return VGPU_OK;
    bool fits = false;
    cudaError_t e = path_fits<R>(a, h->sys.fmt, p, h->device, &fits);
    if (e == cudaSuccess && fits && back) e = one_atom_fits<R>(back, a, h->sys.fmt, p, h->device, &fits);

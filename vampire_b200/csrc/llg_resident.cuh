@@ -782,6 +782,13 @@ __global__ void res_mutual_kernel(const LLGArgs<R> a, int* bad) {
    }
 }
 
+// dynamic shared memory beyond what every kernel may take (few kernels' static
+// kilobyte counts against it: asked for from 40 KB)
+template <typename F> inline cudaError_t allow_smem(F* f, int smem) {
+   if (smem <= 40 * 1024) return cudaSuccess;
+   return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+}
+
 template <typename R> using ResidentFn = void (*)(LLGArgs<R>, int, char*, char*, uint32_t, uint32_t, int, int);
 
 // the kernel of a format, variant, number of atoms per thread and feature set
@@ -898,7 +905,7 @@ cudaError_t cluster_capacity(const LLGArgs<R>& a, int fmt, int var, const Cluste
    for (int feat : feats) {
       f = cluster_fn<R>(fmt, var, feat);
       if (c.size > 8) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+      if (e == cudaSuccess) e = allow_smem(f, (int)cfg.dynamicSmemBytes);
       int n = 0;
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, f, &cfg);
       if (e != cudaSuccess) return e;
@@ -944,7 +951,7 @@ cudaError_t resident_capacity(const LLGArgs<R>& a, int fmt, int var, const Resid
    int least = 1 << 30;
    for (int feat : feats) {
       const ResidentFn<R> f = resident_fn<R>(fmt, var, p.K, feat);
-      cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+      cudaError_t e = allow_smem(f, smem);
       int per_sm = 0;
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kResBlock, smem);
       if (e != cudaSuccess) return e;
@@ -978,7 +985,7 @@ inline cudaError_t one_atom_fits(F* f, const LLGArgs<R>& a, int fmt, const Resid
    const int smem = resident_smem<R>(a, fmt, p);
    int sms = 0, per_sm = 0;
    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemLimit);
+   if (e == cudaSuccess) e = allow_smem(f, smem);
    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kResBlock, smem);
    *fits = per_sm * sms >= p.grid;
    return e;

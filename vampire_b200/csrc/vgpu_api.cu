@@ -191,32 +191,36 @@ static int validate(vgpu_ctx* h, const vgpu_system_desc* d) {
    return VGPU_OK;
 }
 
+// Plan of the steps on one cluster, where the system runs so (S.one).
+template <typename R>
+static int plan_cluster(vgpu_ctx* h) {
+   SysDev& S = h->sys;
+   if (S.n > kClusterAtoms) return VGPU_OK;
+   // a block up to 128 atoms, else up to 16 blocks of at least 64 (us a step,
+   // simple cubic: 125 atoms 1.02 in one block, 1.22 in two; 990 atoms 1.45 in 16
+   // blocks, 1.50 in 8, 1.97 in 2)
+   ClusterShape c;
+   c.size = 1;
+   while (c.size < 16 && (c.size == 1 ? 128 : 64) * c.size < S.n) c.size *= 2;
+   c.threads = std::max(64, ((S.n + c.size - 1) / c.size + 31) / 32 * 32);
+   c.zmax = S.zmax;
+   if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, VAR_HEUN, c, &c.cap), "cluster plan")) return rc;
+   c.cap_var = VAR_HEUN;
+   if (c.cap > 0) S.one = c;
+   return VGPU_OK;
+}
+
 // Plan of the resident steps: the fewest atoms per thread at which the Heun
 // kernel's blocks are resident together (none: larger systems, and systems with
-// one-sided bonds, run one launch per pass).
+// one-sided bonds, run one launch per pass).  Made at the upload, but for a system
+// that steps on one cluster (its first gradient makes it) and while an option asks
+// for the passes (the records in use, and so the shared memory, may be others).
 template <typename R>
-static int plan_resident(vgpu_ctx* h) {
+int plan_resident(vgpu_ctx* h) {
    SysDev& S = h->sys;
-   S.res = ResidentPlan();
-   S.one = ClusterShape();
-   S.zmax = 0;
-   for (int s = 0; s < S.nslices; ++s) S.zmax = std::max(S.zmax, (S.off_host[s + 1] - S.off_host[s]) / 32);
+   if (S.res_planned) return VGPU_OK;
+   S.res_planned = true;
    if (S.fmt == FMT_DMI_TAB && sizeof(R) == 4 && !S.crec) return VGPU_OK;  // the kernel reads compact records
-   {
-      // one cluster: a block up to 128 atoms, else up to 16 blocks of at least 64
-      // (us a step, simple cubic: 125 atoms 1.02 in one block, 1.22 in two; 990
-      // atoms 1.45 in 16 blocks, 1.50 in 8, 1.97 in 2)
-      ClusterShape c;
-      c.size = 1;
-      while (c.size < 16 && (c.size == 1 ? 128 : 64) * c.size < S.n) c.size *= 2;
-      c.threads = std::max(64, ((S.n + c.size - 1) / c.size + 31) / 32 * 32);
-      c.zmax = S.zmax;
-      if (S.n <= kClusterAtoms) {
-         if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, VAR_HEUN, c, &c.cap), "cluster plan")) return rc;
-         c.cap_var = VAR_HEUN;
-         if (c.cap > 0) S.one = c;
-      }
-   }
    int sms = 0;
    if (int rc = cuda_err(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device), "device")) return rc;
    const LLGArgs<R> a = make_args<R>(h);
@@ -257,6 +261,9 @@ static int plan_resident(vgpu_ctx* h) {
    }
    return VGPU_OK;
 }
+
+template int plan_resident<float>(vgpu_ctx*);
+template int plan_resident<double>(vgpu_ctx*);
 
 template <typename R>
 static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
@@ -402,7 +409,9 @@ static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
    S.off_host = std::move(off);
    S.uploaded = true;
    if ((rc = h->refresh_materials())) return rc;
-   return plan_resident<R>(h);
+   for (int s = 0; s < S.nslices; ++s) S.zmax = std::max(S.zmax, (S.off_host[s + 1] - S.off_host[s]) / 32);
+   if ((rc = plan_cluster<R>(h))) return rc;
+   return S.one.size || passes_asked(h) ? VGPU_OK : plan_resident<R>(h);
 }
 
 template <typename R>
@@ -736,6 +745,7 @@ static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
          return VGPU_OK;
       }
    }
+   if (int rc = plan_resident<R>(h)) return rc;
    if (!S.res.K) return VGPU_OK;
    if (S.res.cap_var != *var) {
       int sms = 0;

@@ -31,7 +31,8 @@ struct SysDev {
    std::vector<uint32_t> crec_host;  // host copy of crec (window planning)
    std::vector<int> off_host;        // host copy of slice_off
    ResidentPlan res;                 // resident steps (systems that fit the GPU's resident threads)
-   ClusterShape one;                 // the system on one cluster (systems of at most 16 x 1,024 atoms)
+   bool res_planned = false;         // plan_resident has run
+   ClusterShape one;                 // the system on one cluster (FP32 isotropic, at most kClusterAtoms)
    int zmax = 0;                     // bonds of the widest row
    // window plan of the window-staged passes (built on first use for the tile
    // shape and owned-atom count it was made for)
@@ -167,6 +168,7 @@ struct vgpu_ctx {
 
 namespace vgpu {
 template <typename R> LLGArgs<R> make_args(vgpu_ctx* h);
+template <typename R> int plan_resident(vgpu_ctx* h);
 }
 
 namespace vgpu {

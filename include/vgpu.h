@@ -697,10 +697,10 @@ int vgpu_batch_system_range(vgpu_handle h, int32_t k, int32_t* first_atom, int32
  *   grad[1] = dL/dKu_SI (ku2 = Ku/mu_s), grad[2..4] = dL/dH_applied [1/T],
  * by the adjoint of the step with checkpoints every `every` steps (0: every
  * state is kept where the kept workspaces have room for them, else checkpoints
- * every ceil(sqrt(n_steps))).  The workspace stays allocated for the next call
- * while the kept ones of all handles of the process on that GPU are at most
- * 1 GiB together; it goes with the system (a new upload, vgpu_destroy), and
- * when another allocation of the handle finds no memory.  Every exchange format (isotropic, vectorial,
+ * every ceil(sqrt(n_steps))).  A workspace of at most 1 GiB stays allocated for the
+ * next call while the kept ones of all handles of the process on that GPU are
+ * at most 8 GiB together; it goes with the system (a new upload, vgpu_destroy),
+ * and when another allocation of the handle finds no memory.  Every exchange format (isotropic, vectorial,
  * diagonal + DMI, full tensor) and any number of materials, provided the
  * couplings are reciprocal in SI units (mu_s,j J_ji = (mu_s,i J_ij)^T, as a
  * symmetric exchange matrix and the three-site DMI give; checked on the

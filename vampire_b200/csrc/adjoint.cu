@@ -735,18 +735,18 @@ int forward_step(vgpu_ctx* h, LLGArgs<R> a, R* x, R* pb, R* eb, int stride) {
 // steps of the backward run whose states and fields are held at once
 constexpr int kAdjRun = 64;
 // Workspaces that handles keep between calls (allocating and freeing one took 5
-// to 15 ms of a 15 ms gradient): at most 1 GiB of a GPU's 180 for all handles of
-// the process together, the states of 2,500 steps of 32,768 spins.  A handle
-// that finds no room in it gives its workspace back at the end of each call; a
-// kept one goes with the system, and when an allocation of its handle fails
-// (vgpu_ctx::alloc).
-constexpr int64_t kAdjKeepBytes = (int64_t)1 << 30;
+// to 15 ms of a 15 ms gradient): at most 1 GiB each, the states of 2,500 steps of
+// 32,768 spins, and 8 GiB of a GPU's 180 for all handles of the process together
+// (a program that fits a few systems in turn keeps them all).  A handle that
+// finds no room gives its workspace back at the end of each call; a kept one goes
+// with the system, and when an allocation of its handle fails (vgpu_ctx::alloc).
+constexpr int64_t kAdjKeepBytes = (int64_t)1 << 30, kAdjKeepAll = (int64_t)8 << 30;
 std::atomic<int64_t> g_adj_kept[64];  // by device; none is kept on a device beyond
 
 // bytes that this handle's workspace may have and still be kept
 int64_t keep_room(const vgpu_ctx* h) {
    if (h->device >= 64) return 0;
-   return kAdjKeepBytes - (g_adj_kept[h->device].load() - (int64_t)h->sys.adj_ws_kept);
+   return std::min(kAdjKeepBytes, kAdjKeepAll - (g_adj_kept[h->device].load() - (int64_t)h->sys.adj_ws_kept));
 }
 
 // keeps the workspace after a call if there is room for it, else frees it
@@ -754,8 +754,8 @@ void keep_or_drop(vgpu_ctx* h) {
    SysDev& S = h->sys;
    if (!S.adj_ws || S.adj_ws_kept) return;
    const int64_t bytes = (int64_t)S.adj_ws_bytes;
-   if (h->device < 64) {
-      if (g_adj_kept[h->device].fetch_add(bytes) + bytes <= kAdjKeepBytes) {
+   if (h->device < 64 && bytes <= kAdjKeepBytes) {
+      if (g_adj_kept[h->device].fetch_add(bytes) + bytes <= kAdjKeepAll) {
          S.adj_ws_kept = S.adj_ws_bytes;
          return;
       }

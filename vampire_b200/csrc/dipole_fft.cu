@@ -439,13 +439,12 @@ cudaError_t z_prepare(int logn) {
 template <typename C>
 cudaError_t field_apply(FFTField* f, const double* mag, double* field, cudaStream_t st, int* launches) {
    using R = typename RealOf<C>::type;
-   const int px = f->p[0], py = f->p[1];
+   const int py = f->p[1];
    const int gx = f->g[0], gy = f->g[1], gz = f->g[2], hx = f->hx;
    C* grid = static_cast<C*>(f->grid);
    const C* tw[3] = {static_cast<const C*>(f->tw[0]), static_cast<const C*>(f->tw[1]), static_cast<const C*>(f->tw[2])};
    const size_t cs = (size_t)gz * py * hx;
    const size_t plane = (size_t)py * hx;
-   (void)px;
    cudaError_t e = x_forward<C>(MomentRows{f->box_cell, mag, f->nc, gx}, grid, cs, f->logp[0], 3, gy * gz, gy, py,
                                 tw[0], st);
    if (e == cudaSuccess) e = strided<C, false>(grid, cs, f->logp[1], 3, gz * hx, hx, plane, hx, tw[1], gy, py, st);

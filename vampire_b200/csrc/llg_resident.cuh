@@ -548,224 +548,6 @@ __global__ void __launch_bounds__(kResBlock, (res_min_blocks<R, FMT, VAR_HEUN_EX
       for (int c = 0; c < 3; ++c) x[(size_t)c * stride + i] = S0[c];
 }
 
-// ---------------------------------------------------------------------------
-// FP32 systems of isotropic bonds with at most 2,048 atoms: the system on one
-// thread-block cluster, the states in its distributed shared memory.
-//
-// A small system lives on a few SMs of one GPC, so its spins need not travel
-// through L2: each block keeps its atoms' spins and predictor states in shared
-// memory, neighbours are read from the block that has them, and the half-steps
-// are separated by the cluster's hardware barrier (arrive after the store, the
-// next noise drawn, then wait).  Microseconds a step against the tagged spins in
-// L2 above: 125 atoms 1.05 and 1.51, 990 atoms 1.49 and 2.02, 2,016 atoms 1.83
-// and 2.03; from 4,096 atoms the reads between SMs cost more than L2 (2.24 and
-// 1.97; 8,000 atoms 3.41 and 2.15), and FP64 gains nothing (990 atoms 3.4 and
-// 2.8), so those run above.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned res_cluster_rank() {
-   unsigned r;
-   asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
-   return r;
-}
-__device__ __forceinline__ void res_cluster_arrive() {
-   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void res_cluster_wait() {
-   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// a spin in shared memory, padded to a power of two
-template <typename R> struct alignas(4 * sizeof(R)) ResVec {
-   R x, y, z, pad;
-};
-
-// address of `slot` of the spin array at shared address `arr` in block `rank`
-// of the cluster, and the spin at such an address
-template <typename R>
-__device__ __forceinline__ uint32_t res_address(uint32_t arr, uint32_t rank, uint32_t slot) {
-   uint32_t p;
-   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(arr), "r"(rank));
-   return p + (uint32_t)sizeof(ResVec<R>) * slot;
-}
-__device__ __forceinline__ void res_remote(uint32_t p, float& x, float& y, float& z) {
-   float pad;
-   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(pad) : "r"(p));
-}
-__device__ __forceinline__ void res_remote(uint32_t p, double& x, double& y, double& z) {
-   asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(p));
-   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(z) : "r"(p + 16u));
-}
-
-// the spin at p, in this block's own shared memory (`own`: a plain shared-memory
-// address) or in another block's.  The path between SMs is the narrow one, and
-// own neighbours are most.
-__device__ __forceinline__ void res_near(uint32_t p, bool own, float& x, float& y, float& z) {
-   float pad;
-   asm volatile(
-       "{\n .reg .pred o;\n setp.ne.u32 o, %5, 0;\n"
-       " @o ld.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];\n"
-       " @!o ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
-       : "=f"(x), "=f"(y), "=f"(z), "=f"(pad)
-       : "r"(p), "r"((uint32_t)own));
-}
-__device__ __forceinline__ void res_near(uint32_t p, bool own, double& x, double& y, double& z) {
-   asm volatile(
-       "{\n .reg .pred o;\n setp.ne.u32 o, %4, 0;\n"
-       " @o ld.shared::cta.v2.f64 {%0, %1}, [%3];\n @o ld.shared::cta.f64 %2, [%3 + 16];\n"
-       " @!o ld.shared::cluster.v2.f64 {%0, %1}, [%3];\n @!o ld.shared::cluster.f64 %2, [%3 + 16];\n}"
-       : "=d"(x), "=d"(y), "=d"(z)
-       : "r"(p), "r"((uint32_t)own));
-}
-
-// bond words of the cluster kernel: block << 12 | slot (the slot after the last
-// thread's: the zero spin that padded bonds read), coupling index or material << 16
-constexpr int kClusterBlock = kClusterAtoms / 16;
-constexpr uint32_t kResSlotBits = 12;
-
-template <typename R>
-__host__ __device__ inline ResLayout res_cluster_layout(int threads, int zmax, int M, int dict_bytes) {
-   ResLayout l;
-   const int vec = (threads + 1) * (int)sizeof(ResVec<R>);
-   l.mats = 2 * vec;
-   l.dict = (l.mats + (M <= kResMaxMat ? M * (int)sizeof(MatParams<R>) : 0) + 15) & ~15;
-   l.words = l.dict + dict_bytes;
-   l.bytes = l.words + 4 * threads * zmax;
-   return l;
-}
-
-// nsteps steps of all atoms, one per thread, in order over the blocks of one
-// cluster.  zmax: bonds of the widest row.
-template <typename R, int FMT, int VAR, int RF>
-__global__ void __launch_bounds__(kClusterBlock) llg_cluster_kernel(const LLGArgs<R> in, int nsteps, int zmax) {
-   static_assert(res_words<R, FMT>(), "formats whose bonds are one word");
-   LLGArgs<R> a = fold_iso<R, RF>(in);
-   extern __shared__ __align__(32) unsigned char res_smem[];
-   const int T = blockDim.x, tid = threadIdx.x;
-   const int dict_bytes = FMT == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
-   const ResLayout lay = res_cluster_layout<R>(T, zmax, a.M, dict_bytes);
-   ResVec<R>* sA = reinterpret_cast<ResVec<R>*>(res_smem);
-   ResVec<R>* sB = sA + T + 1;
-   MatParams<R>* s_mat = reinterpret_cast<MatParams<R>*>(res_smem + lay.mats);
-   float4* s_dict = reinterpret_cast<float4*>(res_smem + lay.dict);
-   uint32_t* s_words = reinterpret_cast<uint32_t*>(res_smem + lay.words);
-   const uint32_t rank = res_cluster_rank();
-   const int i = (int)rank * T + tid;
-   const bool on = i < a.n_upd;
-   const bool one_j = (RF & ISO_FIXED) != 0 || a.M == 1 || (a.sys_off && a.m_per_sys == 1);
-   ResRow<R> row{0, 0, nullptr, 0, one_j, (R)0, s_dict};
-   R S0[3] = {0, 0, 0}, P[3] = {0, 0, 0}, E[3] = {0, 0, 0};
-   const uint32_t zero_word = (rank << kResSlotBits) | (uint32_t)T;
-   if (on) {
-      const int off = __ldg(a.slice_off + (i >> 5));
-      row.base = off + (i & 31);
-      row.w = (__ldg(a.slice_off + (i >> 5) + 1) - off) >> 5;
-      row.mi = a.mat ? __ldg(a.mat + i) : 0;
-      if (FMT == FMT_ISO_TAB) row.j0 = __ldg(a.jtab + row.mi * a.M + row.mi);
-      for (int k = 0; k < row.w; ++k) {
-         const int e = row.base + 32 * k;
-         const uint32_t c = FMT == FMT_ISO_TAB ? (uint32_t)__ldg(a.col + e) : __ldg(a.crec + e);
-         const int j = (int)(c & (FMT == FMT_ISO_TAB ? (uint32_t)a.idx_mask : (1u << a.crec_shift) - 1u));
-         const uint32_t q = one_j && FMT == FMT_ISO_TAB ? 0u : res_coupling<R, FMT>(a, c);
-         uint32_t wd = zero_word;
-         if (j < a.n) wd = ((uint32_t)(j / T) << kResSlotBits) | (uint32_t)(j % T);
-         s_words[k * T + tid] = wd | (q << 16);
-      }
-   }
-   if (tid == 0) sA[T] = sB[T] = ResVec<R>{(R)0, (R)0, (R)0, (R)0};
-   for (int q = tid; q < dict_bytes / 16; q += T) s_dict[q] = __ldg(a.cdict + q);
-   if (a.M <= kResMaxMat) {
-      const int nw = a.M * (int)(sizeof(MatParams<R>) / 4);
-      for (int q = tid; q < nw; q += T)
-         reinterpret_cast<uint32_t*>(s_mat)[q] = __ldg(reinterpret_cast<const uint32_t*>(a.mp) + q);
-   }
-   const uint32_t arrA = (uint32_t)__cvta_generic_to_shared(sA), dB = (uint32_t)((T + 1) * (int)sizeof(ResVec<R>));
-   __syncthreads();  // materials and dictionary in place
-   const MatParams<R> m = a.M <= kResMaxMat ? s_mat[row.mi] : a.mp[row.mi];
-   if (a.sys_off && on) {
-      // the stream and atom numbering of this system (thermal_xi), once
-      const int k = row.mi / a.m_per_sys;
-      const uint64_t seed = (((uint64_t)a.seed_hi << 32) | a.seed_lo) + (uint64_t)k;
-      a.noise_base = 0u - (uint32_t)__ldg(a.sys_off + k);
-      a.seed_lo = (uint32_t)seed;
-      a.seed_hi = (uint32_t)(seed >> 32);
-   }
-   a.sys_off = nullptr;
-   // ISO_FIXED: the addresses of the six neighbours (rows of fewer: the zero slot)
-   constexpr uint32_t kSlot = (1u << kResSlotBits) - 1u;
-   uint32_t nb[6], own = 0;
-   if constexpr ((RF & ISO_FIXED) != 0) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-         const uint32_t c = k < row.w ? s_words[k * T + tid] : zero_word;
-         const uint32_t r = (c >> kResSlotBits) & 15u;
-         if (r == rank) own |= 1u << k;
-         nb[k] = r == rank ? arrA + (uint32_t)sizeof(ResVec<R>) * (c & kSlot) : res_address<R>(arrA, r, c & kSlot);
-      }
-   }
-   // everything above is as the upload or a copy on the stream left it; the spins
-   // and the dipole field are the previous kernel's
-   pdl_begin();
-   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-   if (on) { S0[0] = a.ax[i]; S0[1] = a.ay[i]; S0[2] = a.az[i]; }
-   sA[tid] = ResVec<R>{S0[0], S0[1], S0[2], (R)0};
-   res_cluster_arrive();
-   const uint64_t step0 = a.step;
-   // d: 0 for the spins, dB for the predictor states
-   auto field = [&](uint32_t d, const R S[3], R H[3]) {
-      R hx = 0, hy = 0, hz = 0;
-      if constexpr ((RF & ISO_FIXED) != 0) {
-         R x[6], y[6], z[6];
-#pragma unroll
-         for (int k = 0; k < 6; ++k) res_near(nb[k] + d, (own >> k) & 1u, x[k], y[k], z[k]);
-#pragma unroll
-         for (int k = 0; k < 6; ++k) { hx += row.j0 * x[k]; hy += row.j0 * y[k]; hz += row.j0 * z[k]; }
-      } else {
-         constexpr int W = sizeof(R) == 8 ? 4 : 6;  // loads in flight
-         for (int k0 = 0; k0 < row.w; k0 += W) {
-            uint32_t c[W];
-            R x[W], y[W], z[W];
-#pragma unroll
-            for (int k = 0; k < W; ++k) c[k] = k0 + k < row.w ? s_words[(k0 + k) * T + tid] : zero_word;
-#pragma unroll
-            for (int k = 0; k < W; ++k)
-               res_remote(res_address<R>(arrA, (c[k] >> kResSlotBits) & 15u, c[k] & kSlot) + d, x[k], y[k], z[k]);
-#pragma unroll
-            for (int k = 0; k < W; ++k)
-               if (k0 + k < row.w) res_bond<R, FMT>(a, row, k0 + k, c[k] >> 16, x[k], y[k], z[k], hx, hy, hz);
-         }
-      }
-      site_field<R, 0, VAR != VAR_HEUN>(a, i, m, nullptr, nullptr, nullptr, S, hx, hy, hz, H);
-      H[0] += E[0]; H[1] += E[1]; H[2] += E[2];
-   };
-   for (int s = 0; s < nsteps; ++s) {
-      a.step = step0 + (uint64_t)s;
-      set_ramp(a);
-      if (on) external_field<R>(a, i, m, true, E);
-      res_cluster_wait();  // every block's spins of this step in place
-      if (on) {
-         R H[3];
-         field(0, S0, H);
-         first_half<R, VAR>(a, i, m, S0, H, P);
-         sB[tid] = ResVec<R>{P[0], P[1], P[2], (R)0};
-      }
-      res_cluster_arrive();
-      res_cluster_wait();  // every predictor state in place, every read of the spins done
-      if (on) {
-         R H[3], o[3];
-         field(dB, P, H);
-         second_half<R, VAR>(a, i, m, S0, P, H, o);
-         S0[0] = o[0]; S0[1] = o[1]; S0[2] = o[2];
-         sA[tid] = ResVec<R>{o[0], o[1], o[2], (R)0};
-      }
-      res_cluster_arrive();
-   }
-   if (on) {
-      a.ax[i] = S0[0]; a.ay[i] = S0[1]; a.az[i] = S0[2];
-      a.bx[i] = P[0]; a.by[i] = P[1]; a.bz[i] = P[2];
-   }
-   res_cluster_wait();  // no block leaves while its shared memory is read
-}
-
 // every bond i -> j has a bond j -> i (*bad set otherwise)
 template <typename R>
 __global__ void res_mutual_kernel(const LLGArgs<R> a, int* bad) {
@@ -839,92 +621,6 @@ inline ResidentFn<R> resident_fn(int fmt, int var, int K, int feat) {
       case FMT_DMI_TAB: return resident_fmt<R, FMT_DMI_TAB>(var, K, feat);
       default: return resident_fmt<R, FMT_TENSOR_BOND>(var, K, feat);
    }
-}
-
-// the cluster kernel of a variant and feature set (nullptr: none)
-template <typename R> using ClusterFn = void (*)(LLGArgs<R>, int, int);
-
-template <typename R>
-inline ClusterFn<R> cluster_fn(int fmt, int var, int feat) {
-   if constexpr (sizeof(R) == 4) {
-      if (fmt != FMT_ISO_TAB) return nullptr;
-      switch (feat) {
-#define VGPU_F(k) \
-   case k: return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN, k>;
-         VGPU_ISO_FEATURES(VGPU_F)
-#undef VGPU_F
-      }
-      if (var == VAR_HEUN) return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN, 0>;
-      if (var == VAR_HEUN_EXT) return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_HEUN_EXT, 0>;
-      return llg_cluster_kernel<R, FMT_ISO_TAB, VAR_MIDPOINT, 0>;
-   }
-   return nullptr;
-}
-
-template <typename R>
-cudaError_t cluster_config(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, cudaLaunchConfig_t* cfg,
-                           cudaLaunchAttribute* attr, ClusterFn<R>* f) {
-   *f = cluster_fn<R>(fmt, var, c.zmax <= 6 ? iso_features<R>(a, fmt, var) : 0);
-   if (!*f) return cudaErrorInvalidValue;
-   const int dict = fmt == FMT_DMI_TAB ? 16 * (a.tab_scalar ? a.cdict_n : 2 * a.cdict_n) : 0;
-   *cfg = cudaLaunchConfig_t{};
-   cfg->gridDim = dim3(c.size);
-   cfg->blockDim = dim3(c.threads);
-   cfg->dynamicSmemBytes = (size_t)res_cluster_layout<R>(c.threads, c.zmax, a.M, dict).bytes;
-   attr[0].id = cudaLaunchAttributeClusterDimension;
-   attr[0].val.clusterDim.x = c.size;
-   attr[0].val.clusterDim.y = 1;
-   attr[0].val.clusterDim.z = 1;
-   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-   attr[1].val.programmaticStreamSerializationAllowed = 1;
-   cfg->attrs = attr;
-   cfg->numAttrs = 2;
-   return cudaSuccess;
-}
-
-// clusters of a shape that the GPU holds at once, whatever the parameters turn
-// out to be (0: it cannot run): the least over the generic kernel and the
-// compiled features
-template <typename R>
-cudaError_t cluster_capacity(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, int* clusters) {
-   *clusters = 0;
-   if (!cluster_fn<R>(fmt, var, 0)) return cudaSuccess;
-   cudaLaunchConfig_t cfg;
-   cudaLaunchAttribute attr[2];
-   ClusterFn<R> f;
-   cudaError_t e = cluster_config<R>(a, fmt, var, c, &cfg, attr, &f);
-   if (e != cudaSuccess) return e;
-   if (cfg.dynamicSmemBytes > kStageSmemLimit) return cudaSuccess;
-   std::vector<int> feats{0};
-   if (fmt == FMT_ISO_TAB && var == VAR_HEUN && c.zmax <= 6) {
-#define VGPU_F(k) feats.push_back(k);
-      VGPU_ISO_FEATURES(VGPU_F)
-#undef VGPU_F
-   }
-   int least = 1 << 30;
-   for (int feat : feats) {
-      f = cluster_fn<R>(fmt, var, feat);
-      if (c.size > 8) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess) e = allow_smem(f, (int)cfg.dynamicSmemBytes);
-      int n = 0;
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, f, &cfg);
-      if (e != cudaSuccess) return e;
-      least = std::min(least, n);
-   }
-   *clusters = least;
-   return cudaSuccess;
-}
-
-template <typename R>
-cudaError_t launch_llg_cluster(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ClusterShape& c,
-                               cudaStream_t st) {
-   cudaLaunchConfig_t cfg;
-   cudaLaunchAttribute attr[2];
-   ClusterFn<R> f;
-   cudaError_t e = cluster_config<R>(a, fmt, var, c, &cfg, attr, &f);
-   if (e != cudaSuccess) return e;
-   cfg.stream = st;
-   return cudaLaunchKernelEx(&cfg, f, a, nsteps, c.zmax);
 }
 
 // dynamic shared memory of a plan

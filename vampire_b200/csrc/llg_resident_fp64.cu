@@ -6,8 +6,6 @@ namespace vgpu {
 template cudaError_t resident_capacity<double>(const LLGArgs<double>&, int, int, const ResidentPlan&, int, int*);
 template cudaError_t launch_resident_check<double>(const LLGArgs<double>&, int*, cudaStream_t);
 template cudaError_t launch_llg_resident<double>(const LLGArgs<double>&, int, int, int, const ResidentPlan&, int, cudaStream_t);
-template cudaError_t cluster_capacity<double>(const LLGArgs<double>&, int, int, const ClusterShape&, int*);
-template cudaError_t launch_llg_cluster<double>(const LLGArgs<double>&, int, int, int, const ClusterShape&, cudaStream_t);
 template cudaError_t path_fits<double>(const LLGArgs<double>&, int, const ResidentPlan&, int, bool*);
 template cudaError_t launch_llg_path<double>(const LLGArgs<double>&, int, int, const ResidentPlan&, int, double*, double*, int, double*, double*, cudaStream_t);
 }  // namespace vgpu

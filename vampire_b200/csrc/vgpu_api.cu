@@ -191,11 +191,11 @@ static int validate(vgpu_ctx* h, const vgpu_system_desc* d) {
    return VGPU_OK;
 }
 
-// Plan of the steps on one cluster, where the system runs so (S.one).
-template <typename R>
+// Plan of the steps on one cluster, where the system runs so (S.one): FP32 and
+// isotropic table bonds.
 static int plan_cluster(vgpu_ctx* h) {
    SysDev& S = h->sys;
-   if (S.n > kClusterAtoms) return VGPU_OK;
+   if (S.n > kClusterAtoms || S.fmt != FMT_ISO_TAB || h->prec != VGPU_PREC_FP32) return VGPU_OK;
    // a block up to 128 atoms, else up to 16 blocks of at least 64 (us a step,
    // simple cubic: 125 atoms 1.02 in one block, 1.22 in two; 990 atoms 1.45 in 16
    // blocks, 1.50 in 8, 1.97 in 2)
@@ -204,7 +204,7 @@ static int plan_cluster(vgpu_ctx* h) {
    while (c.size < 16 && (c.size == 1 ? 128 : 64) * c.size < S.n) c.size *= 2;
    c.threads = std::max(64, ((S.n + c.size - 1) / c.size + 31) / 32 * 32);
    c.zmax = S.zmax;
-   if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, VAR_HEUN, c, &c.cap), "cluster plan")) return rc;
+   if (int rc = cuda_err(h, cluster_capacity(make_args<float>(h), VAR_HEUN, c, &c.cap), "cluster plan")) return rc;
    c.cap_var = VAR_HEUN;
    if (c.cap > 0) S.one = c;
    return VGPU_OK;
@@ -410,7 +410,7 @@ static int upload_typed(vgpu_ctx* h, const vgpu_system_desc* d) {
    S.uploaded = true;
    if ((rc = h->refresh_materials())) return rc;
    for (int s = 0; s < S.nslices; ++s) S.zmax = std::max(S.zmax, (S.off_host[s + 1] - S.off_host[s]) / 32);
-   if ((rc = plan_cluster<R>(h))) return rc;
+   if ((rc = plan_cluster(h))) return rc;
    return S.one.size || passes_asked(h) ? VGPU_OK : plan_resident<R>(h);
 }
 
@@ -736,8 +736,7 @@ static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
    *var = integrator == INTEG_MIDPOINT ? VAR_MIDPOINT : S.aniso_ext ? VAR_HEUN_EXT : VAR_HEUN;
    if (S.one.size) {
       if (S.one.cap_var != *var) {
-         if (int rc = cuda_err(h, cluster_capacity<R>(make_args<R>(h), S.fmt, *var, S.one, &S.one.cap), "cluster plan"))
-            return rc;
+         if (int rc = cuda_err(h, cluster_capacity(make_args<float>(h), *var, S.one, &S.one.cap), "cluster plan")) return rc;
          S.one.cap_var = *var;
       }
       if (S.one.cap > 0) {
@@ -764,10 +763,14 @@ static int step_mode(vgpu_ctx* h, int integrator, StepMode* mode, int* var) {
 template <typename R>
 static int run_resident(vgpu_ctx* h, uint64_t n, StepMode mode, int var) {
    SysDev& S = h->sys;
-   LLGArgs<R> a = make_args<R>(h);
-   a.wait_test = h->resident_wait_test;
-   const cudaError_t e = mode == STEP_CLUSTER ? launch_llg_cluster<R>(a, S.fmt, var, (int)n, S.one, h->stream)
-                                              : launch_llg_resident<R>(a, S.fmt, var, (int)n, S.res, S.nslices, h->stream);
+   cudaError_t e;
+   if (mode == STEP_CLUSTER) {
+      e = launch_llg_cluster(make_args<float>(h), var, (int)n, S.one, h->stream);
+   } else {
+      LLGArgs<R> a = make_args<R>(h);
+      a.wait_test = h->resident_wait_test;
+      e = launch_llg_resident<R>(a, S.fmt, var, (int)n, S.res, S.nslices, h->stream);
+   }
    if (e != cudaSuccess) return cuda_err(h, e, "resident llg launch");
    h->kernel_launches += 1;
    // past every number of this launch: its last spins are not the next one's first

@@ -176,7 +176,8 @@ struct ResidentPlan {
    uint32_t epoch = 1;        // number of the next half-step (0: what the cleared buffer holds)
    int cap_var = -1, cap_blocks = 0;  // blocks of a variant's kernel that the GPU holds at once
 };
-// The system on one cluster, one atom per thread (llg_resident.cuh).
+// An FP32 system of isotropic bonds on one cluster, one atom per thread
+// (llg_cluster.cu).
 constexpr int kClusterAtoms = 2048;
 constexpr int kClusterSteps = 5;  // steps of one launch
 struct ClusterShape {
@@ -185,11 +186,8 @@ struct ClusterShape {
    int zmax = 0;              // bonds of the widest row
    int cap_var = -1, cap = 0; // clusters of a variant's kernel that the GPU holds at once
 };
-template <typename R>
-cudaError_t cluster_capacity(const LLGArgs<R>& a, int fmt, int var, const ClusterShape& c, int* clusters);
-template <typename R>
-cudaError_t launch_llg_cluster(const LLGArgs<R>& a, int fmt, int var, int nsteps, const ClusterShape& c,
-                               cudaStream_t st);
+cudaError_t cluster_capacity(const LLGArgs<float>& a, int var, const ClusterShape& c, int* clusters);
+cudaError_t launch_llg_cluster(const LLGArgs<float>& a, int var, int nsteps, const ClusterShape& c, cudaStream_t st);
 
 // blocks of the variant's kernel that are resident together (0: no such kernel)
 template <typename R>
@@ -223,9 +221,6 @@ extern template cudaError_t launch_llg_pass<double>(const LLGArgs<double>&, int,
    extern template cudaError_t launch_resident_check<R>(const LLGArgs<R>&, int*, cudaStream_t);                \
    extern template cudaError_t launch_llg_resident<R>(const LLGArgs<R>&, int, int, int, const ResidentPlan&, int, \
                                                       cudaStream_t);                                          \
-   extern template cudaError_t cluster_capacity<R>(const LLGArgs<R>&, int, int, const ClusterShape&, int*);    \
-   extern template cudaError_t launch_llg_cluster<R>(const LLGArgs<R>&, int, int, int, const ClusterShape&,    \
-                                                     cudaStream_t);                                           \
    extern template cudaError_t path_fits<R>(const LLGArgs<R>&, int, const ResidentPlan&, int, bool*);          \
    extern template cudaError_t launch_llg_path<R>(const LLGArgs<R>&, int, int, const ResidentPlan&, int, R*, R*, int, \
                                                   R*, double*, cudaStream_t);

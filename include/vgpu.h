@@ -227,9 +227,10 @@ int vgpu_set_noise_replay(vgpu_handle h, const double* xi);
 #define VGPU_OPT_STAGE_SLICES 3
 #define VGPU_OPT_STAGE_BUFFERS 4
 /* VGPU_OPT_DIPOLE_FFT (read by vgpu_dipole_setup): 1 or -1 (default) = the
- * far-field cell sum by FP64 FFT convolution when every occupied cell centre
- * lies on one regular grid (falls back to the direct sum otherwise), 0 =
- * always the direct all-pairs sum. */
+ * far-field cell sum by FFT convolution when every occupied cell centre lies on
+ * one regular grid (falls back to the direct sum otherwise; in the handle's
+ * precision, but in FP64 on grids of at most 8 cells per axis), 0 = always the
+ * direct all-pairs sum. */
 #define VGPU_OPT_DIPOLE_FFT 5
 /* VGPU_OPT_STAGE_WAIT_TEST: 1 = staged passes wait for 16 bytes more than each
  * tile's copy delivers, so their bounded wait (1 s) runs out and the step

@@ -36,9 +36,9 @@
 //
 // Precision follows the handle: in the FP64 build every step is FP64, so the
 // result equals the direct FP64 sum to rounding (~1e-15 of the field); the
-// FP32 production handles transform FP32 grids (the tensor spectra computed
-// in FP64 once and rounded, twiddles rounded from FP64, moments and fields
-// FP64 at the ends), a few 1e-7 of the field.  Cost O(P^3 log P) instead of
+// FP32 production handles transform FP32 grids where an axis has more than 8
+// cells (the tensor spectra computed in FP64 once and rounded, twiddles rounded
+// from FP64, moments and fields FP64 at the ends), a few 1e-7 of the field.  Cost O(P^3 log P) instead of
 // O(Nc^2).
 #include "dipole_fft.cuh"
 
@@ -551,6 +551,13 @@ FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double
    }
    f->np = np;
    f->hx = f->p[0] / 2 + 1;
+   // Grids of at most 8 cells per axis stay in FP64: with so few passes the two
+   // roundings of packing real lines in pairs weigh more than the passes they
+   // save (2-norm error of B against FP64 on FP32 handles: 4^3 cells 1.76e-7 with
+   // complex radix-2 lines, 1.81e-7 with packed FP32 lines; 8^3 2.24e-7 and
+   // 2.35e-7; from 9 cells on packed lines are the more exact, 10^3 2.50e-7 and
+   // 2.21e-7), and such a grid costs its launches whatever its type.
+   fp32 = fp32 && std::max(f->p[0], std::max(f->p[1], f->p[2])) > 16;
    f->fp32 = fp32;
    // cell at each point of the G-box; two cells on one grid point are not a grid
    const size_t nbox = (size_t)f->g[0] * f->g[1] * f->g[2];

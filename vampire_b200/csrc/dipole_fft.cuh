@@ -13,7 +13,8 @@ struct FFTField;
 // small enough; otherwise returns nullptr with the reason in *why (and
 // *err == cudaSuccess).  cpos holds x, y, z, w per cell (Angstrom); cells with
 // natoms <= 0 are empty.  fp32: the transforms of every update in FP32 (the
-// spectra computed in FP64 and rounded), else FP64.  Work is queued on `st`.
+// spectra computed in FP64 and rounded) where an axis has more than 8 cells, else
+// FP64.  Work is queued on `st`.
 FFTField* fft_field_create(int nc, const double* cpos, const int* natoms, double size, bool fp32, cudaStream_t st,
                            cudaError_t* err, std::string* why);
 

@@ -516,8 +516,8 @@ int vgpu_mc_counters(vgpu_handle h, double* moves, double* rejects);
  * (angle move of one spin, the second spin of the pair keeping the moment
  * perpendicular to the constraint, acceptance exp(-dE/kT) (Mz'/Mz)^2
  * |s2z/s2z'| with Mz' > 0): the pairs of a phase are atoms of one colour, so
- * their energy changes are independent and one warp accepts them in order
- * with the running total moment, the reference's rule.  The pairs differ from
+ * their energy changes are independent and they are accepted in order with
+ * the running total moment, the reference's rule.  The pairs differ from
  * the reference's random choice: the chains agree in distribution.
  * vgpu_cmc_pairs runs one phase on given pairs (2*num_pairs atoms, all of one
  * colour, each once) with given random numbers rnd[4*num_pairs] (the
@@ -764,11 +764,15 @@ int vgpu_magnetization_noalloc(const float* sx, const float* sy, const float* sz
 int vgpu_get_stream(vgpu_handle h, void** stream);
 
 /* Wait for the handle's stream; reports VGPU_ERR_NAN if a pass flagged a
- * non-finite spin since the last check. */
+ * non-finite spin, and VGPU_ERR_TIMEOUT if a bounded wait on the device ran
+ * out, since the last check. */
 int vgpu_synchronize(vgpu_handle h);
 
 /* enable != 0: time every launch with CUDA events on the handle's stream
- * (resets the accumulators and the kernel-launch counter). */
+ * (resets the accumulators and the kernel-launch counter).  Steps then run one
+ * launch per pass at every size, so a system that would otherwise run several
+ * steps in one launch is timed on other kernels than it runs unprofiled (with
+ * the same results). */
 int vgpu_profile(vgpu_handle h, int enable);
 
 /* Accumulated device milliseconds and launch counts per kind

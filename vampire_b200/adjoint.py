@@ -5,11 +5,12 @@ L = sum_{t=1..N} dt_SI (m_z(t) - target_t)^2, m_z the moment-weighted mean of
 s_z after step t, and its gradient with respect to the exchange constant J
 (every coupling scaled together), the uniaxial constant Ku and the applied
 field (Hx, Hy, Hz) comes from the hand-written adjoint kernels of
-libvgpu.so (vgpu_adjoint_llg, sqrt(N)-step checkpointing with recomputation),
-wrapped as a torch.autograd.Function for fitting.  The adjoint runs in FP32
-(FP64 sums for m_z, the loss and the gradients) unless the FP64 debug build
-is asked for; both agree with central differences of the FP64 forward loss
-to about 1e-5 on the benchmark problem.  For systems of several
+libvgpu.so (vgpu_adjoint_llg: every state kept where the workspace has room,
+else sqrt(N)-step checkpoints with recomputation), wrapped as a
+torch.autograd.Function for fitting.  The adjoint runs in FP32 (FP64 sums for
+m_z, the loss and the gradients) unless the FP64 debug build is asked for; both
+agree with central differences of the FP64 forward loss to about 1e-5 on the
+benchmark problem.  For systems of several
 materials, and tensor or DMI couplings, loss_and_grad_materials adds the
 gradients with respect to each material pair's exchange constant and the
 DMI strength (vgpu_adjoint_llg_materials).

@@ -141,8 +141,8 @@ __device__ __forceinline__ void second_half(const LLGArgs<R>& a, int i, const Ma
 // no host dipole field, no field per material -- with the thermal term, a batch
 // (field ramp, temperature and noise stream per system) and the macrocell field
 // given by the other bits.  The branches on those facts and the parameter loads
-// behind them are gone: the resident step went from 741 to 374 warp
-// instructions per 32 atoms with them and the bond addresses in registers.
+// behind them are gone (406 warp instructions per 32 atoms in the predictor of a
+// thermal batch).
 constexpr int kIsoBlock = 256;
 enum IsoFeat : int { ISO_FIXED = 1, ISO_THERMAL = 2, ISO_BATCH = 4, ISO_CELL = 8 };
 #define VGPU_ISO_FEATURES(F) F(1) F(3) F(5) F(7) F(9) F(11)

@@ -17,8 +17,11 @@
 // release/acquire fences a half-step took 2.9 us, no better than a launch.)
 // Microseconds a step of a long launch, simple cubic, 300 K: 2.15 at 8,000 and
 // 1.98 at 32,768 atoms (5.0 in two launches), FP64 2.95 and 3.08; 151,951 atoms
-// 5.5 (11.0), where the issue of about 560 instructions per 32 atoms is the
-// bound; a 37,044-atom FCC alloy with DMI 5.0 (8.6).
+// 5.5 (11.0); a 37,044-atom FCC alloy with DMI 5.0 (8.6).  What bounds it is the
+// wait for the words, the largest share of the cycles between two instructions of
+// a warp at every size, with 14 % of the issue slots in use at 8,000 atoms, 49 %
+// (566 instructions per 32 atoms and step, polls included) and half of the L1
+// data pipe at 151,951.
 //
 // The two states keep apart what a reader may still need: an atom overwrites
 // its spin of the last step only after reading every neighbour's predictor

@@ -193,8 +193,8 @@ __device__ __forceinline__ bool mc_trial(const MCArgs<R>& p, int i, int mi, R h[
 // meanwhile; the first row is read, and the next colour's launch begun, before
 // the previous colour is done (the rows are written at the setup only).
 // PLAIN: no term beyond exchange, the applied field and the uniaxial
-// anisotropy, and no replayed numbers (a trial is 409 instructions a warp
-// with all the tests, and their issue is what remains).
+// anisotropy, and no replayed numbers (331 warp instructions a trial, 409 with
+// all the tests; 58 % of the issue slots, the gather's latency the largest wait).
 // A colour of simple cubic 50^3 x 31 temperatures (1.94 million trials): 65 us
 // on the neighbour list, 37 on trial rows, 32 PLAIN; with 6 or 10 blocks of
 // 128 per SM in place of 8 (64 registers) 32.5 and 33.
@@ -823,7 +823,8 @@ __global__ void __launch_bounds__(128) cmc_propose_kernel(const CMCArgs<R> p) {
 // z, the thread decides its pairs in order, and this repeats until no decision
 // changed.  After round r the first r threads hold the chain's decisions
 // whatever they held before, so the loop ends after at most kCmcThreads + 1
-// rounds with the one solution there is, the sequential one; two to four
+// rounds with the one solution there is, the sequential one (the running moment
+// as a prefix sum, so rounded in another order than pair by pair); two to four
 // rounds are usual.  (A one-warp walk of the chain, 32 pairs' data passed
 // through shuffles, was bound by its latency: 742 us for 3,456 pairs.  A step
 // of 13,824 spins at 400 K, four phases each, took 2.68 ms with it and takes
@@ -1016,7 +1017,7 @@ uint64_t gcd64(uint64_t a, uint64_t b) {
 }
 
 // one phase: K pairs (explicit, or the affine pairing of colour c), proposals
-// in parallel, acceptance by one warp
+// in parallel, then their acceptance in order
 template <typename R>
 int cmc_phase(vgpu_handle h, const R* tab, const int* list, int count, const int* given, int K, const double* rnd,
               uint32_t phase, const double* P, double* Mdev) {

@@ -165,8 +165,13 @@ cudaError_t launch_llg_staged(const LLGArgs<float>& a, int mode, int nslices, co
 // Resident steps (llg_resident.cuh): many steps in one cooperative launch,
 // K atoms per thread.
 constexpr int kResidentBlock = 128;  // threads per block
-// steps of one launch.  A cooperative launch keeps its threads on the SMs until
-// it ends, and programs hold small systems by the dozen: those take turns.
+// Steps of one launch (beside kClusterSteps below).  Longer runs of the small
+// systems are faster for one handle and for many alike -- us a step for runs of
+// 5 / 10 steps (cluster / grid), of 20, and uncut: 1,000 atoms 1.90, 1.62, 1.54,
+// 32 such handles 24.4, 8.4, 4.8; 8,000 atoms 2.58, 2.40, 2.21, 32 handles 13.3,
+// 11.5, 7.9; 256 particles as a handle each 116, 52, 28 -- but with 20 the last
+// would be less than the 5 times behind the batch (14.9) that the batch is
+// tested for.
 constexpr int kGridSmallAtoms = 16384, kGridSmallSteps = 10, kGridSteps = 4096;
 struct ResidentPlan {
    int K = 0;                 // atoms per thread (0: no plan)
